@@ -21,6 +21,7 @@
 #include "bands_kernels.cuh"
 #include "stats_kernels.cuh"
 #include "xmarch.cuh"
+#include "colsolve.cuh"
 
 using namespace cfd;
 
@@ -83,6 +84,12 @@ struct cfd_ctx {
     int JC = 16;
     int SNT = 64;           // threads per CTA of the column sweeps (k_solve_uvw, k_solve_p)
     int nch = 1;
+    // warp-per-column solves (k_col_solve): rows per lane (0: the column is too tall, the
+    // thread-per-column sweeps run), columns of a group and the coefficient table
+    int colM = 0, colC = 4;
+    int nsm = 1;            // SMs of the device (CTAs of the persistent kernels)
+    double* coltab = nullptr;
+    cfd::ColMaps colmap, colmap_p;  // of the solves and of cfd_solve_p
     double* scal = nullptr;
     double* mf_work = nullptr;
     double2* stage0 = nullptr;
@@ -336,8 +343,7 @@ int ilog2(int b) {
 //   CFD_ZLINES_LOG2  log2 of the lines per CTA of the two-step z kernels (2..4)
 //   CFD_XLINE_STOCKHAM 1: nonlinear through the Stockham x-line kernel and per-slot z pass
 //   CFD_XLINE_PATH   3: packed two-step x-line kernel (1.5 inverse lines per row)
-//   CFD_SOLVE_WARP   1: Helmholtz solves one warp per column on precomputed LU factors
-//   CFD_SOLVE_COLS   columns (warps) per CTA of the warp-per-column solve (1..8)
+//   CFD_SOLVE_GROUP  columns of a group of the warp-per-column solves (4 or 8)
 //   CFD_RHS_CHUNK    y-planes per thread of the right-hand-side kernel (2..64)
 int env_int(const char* name, int dflt, int lo, int hi) {
     const char* v = std::getenv(name);
@@ -828,6 +834,65 @@ int ib_all(cfd_ctx* c) {
     return ib_grid<T2>(c, c->ibu, c->d.ju0, 2, c->du1, c->u1, c->du3, c->u3, c->Hib, c->phys, 0, c->d.nyu);
 }
 
+// The warp-per-column solves: mode 7 = u, v, w, the pressure and v_corr (the substep's), 1 =
+// u, v, w (cfd_solve_uvw), 2 = the pressure with psi and the divergence (cfd_solve_p).
+int col_solve(cfd_ctx* c, int mode, int krk, const char* name) {
+    const double ab = kRKa[krk - 1] + kRKb[krk - 1];
+    ColArgs a;
+    a.tab = c->coltab;
+    a.beta = kRKb[krk - 1] * c->dt / c->re;
+    a.dtirk = (1.0 / c->dt) / ab;
+    a.dtrk = c->dt * ab;
+    a.mean_diag = c->mean_diag;
+    a.err = c->scal + 3;
+    a.ahead = col_ahead(c->colC, c->d.ncol);
+    prof_mark(c);
+    col_launch(mode, c->colM, c->colC, c->nsm, c->stream, c->d, c->g, mode == 2 ? c->colmap_p : c->colmap, a);
+    return launched(c, name);
+}
+
+// Coefficients of k_col_solve, tab[(i*kColTabs + k)*32 + lane] for row r = lane*m + i: k 0..2
+// and 3..5 dyu2i and dyv2i of the interior velocity rows, the sum of the three in place of the
+// middle one (the surplus of the diagonal), 6 dthdyu of the centre of p row r, 7
+// dthdyv of the interior face above it (the factors of D.G, LU_buildP,
+// tridLU_3D_IB.f90:417-491); 0 where there is none.
+int col_table(cfd_ctx* c, const cfd_config* cfg) {
+    const Dims& d = c->d;
+    c->colM = c->mb ? 0 : col_rows_per_lane(d.nyu);
+    const int m = c->colM;
+    if (!m) return CFD_OK;
+    c->colC = env_int("CFD_SOLVE_GROUP", col_cols(m, d.ncol), 4, 8) == 8 && m <= 15 ? 8 : 4;
+    std::vector<double> h((size_t)32 * m * kColTabs, 0.0);
+    for (int r = 0; r < 32 * m; ++r) {
+        double* e = &h[(size_t)(r % m) * kColTabs * 32 + r / m];
+        auto put = [&](int k, double v) { e[(size_t)k * 32] = v; };
+        for (int f = 0; f < 2; ++f) {
+            const double* w = (f ? cfg->dyv2i : cfg->dyu2i) + 3 * r;
+            if (r <= 0 || r >= (f ? d.nyv : d.nyu) - 1) continue;
+            put(3 * f, w[0]);
+            put(3 * f + 1, (w[0] + w[2]) + w[1]);
+            put(3 * f + 2, w[2]);
+        }
+        // p row r: centre r + 1 of the u grid, between faces r and r + 1 of the v grid
+        if (r < d.nyp) put(6, cfg->dthdyu[r + 1]);
+        if (r < d.nyp - 1) put(7, cfg->dthdyv[r + 1]);
+    }
+    AL(c->coltab, double, h.size());
+    CK(cudaMemcpy(c->coltab, h.data(), sizeof(double) * h.size(), cudaMemcpyHostToDevice));
+    CK(col_prepare(m));
+    ColMaps &a = c->colmap, &b = c->colmap_p;
+    const int nu = d.nyu, nv = d.nyv, np = d.nyp;
+    const struct { CUtensorMap* map; const void* f; int n; } all[] = {
+        {&a.src[0], c->du1, nu}, {&a.src[1], c->du3, nu}, {&a.src[2], c->du2, nv}, {&a.dst[0], c->u1, nu},
+        {&a.dst[1], c->u3, nu},  {&a.dst[2], c->u2, nv},  {&a.p, c->p, np},        {&b.src[0], c->u1, nu},
+        {&b.src[1], c->u3, nu},  {&b.src[2], c->u2, nv},  {&b.dst[0], c->psi, np}, {&b.dst[1], c->div, np},
+        {&b.p, c->p, np}};
+    for (const auto& x : all)
+        if (!col_map(x.map, x.f, d.ncol, x.n, m, c->colC)) { c->colM = 0; break; }
+    b.dst[2] = b.dst[1];
+    return CFD_OK;
+}
+
 // One launch of the Helmholtz solves on stream st: the systems part0 .. part0 + nsys - 1
 // (0 = u/w, 1 = v).
 int launch_solve(cfd_ctx* c, cudaStream_t st, double beta, int part0, int nsys) {
@@ -836,20 +901,6 @@ int launch_solve(cfd_ctx* c, cudaStream_t st, double beta, int part0, int nsys) 
     k_solve_uvw<<<gb, c->SNT, 0, st>>>(d, c->g, beta, c->u1, c->u2, c->u3, c->du1, c->du2, c->du3, c->cs, c->cs_v,
                                        part0);
     return launched(c, "k_solve_uvw");
-}
-
-int solve_kernel(cfd_ctx* c, int krk);
-
-// The IB round trips (u/w and v grids on two streams inside ib_all), then one solve launch
-// over both systems.  Measured at re550: running the v solve beside the u/w round trip as
-// a second graph branch split the solve into two launches of half the CTAs and lost 4.5 %
-// (FP32-mixed) and 3.8 % (FP64) of the step rate.
-template <typename T2>
-int ib_solve_all(cfd_ctx* c, int krk) {
-    int s = ib_all<T2>(c);
-    if (s != CFD_OK) return s;
-    c->hx_valid = false;  // the solve changes u, v, w
-    return solve_kernel(c, krk);
 }
 
 int solve_kernel(cfd_ctx* c, int krk) {
@@ -863,14 +914,15 @@ int solve_kernel(cfd_ctx* c, int krk) {
         LK("k_mb_solve_uvw");
         return CFD_OK;
     }
+    if (c->colM) return col_solve(c, 1, krk, "k_col_solve_uvw");
     return launch_solve(c, c->stream, beta, 0, 2);
 }
 
-int meanflow_kernel(cfd_ctx* c, int krk) {
+int meanflow_kernel(cfd_ctx* c, int krk, bool ghosts = false) {
     const double beta = kRKb[krk - 1] * c->dt / c->re;
     const double bdt = -kRKd[krk - 1] * c->dt;
     prof_mark(c);
-    k_meanflow<<<1, 32, 0, c->stream>>>(c->d, c->g, beta, bdt, c->qxt, c->ctpress, c->u1, c->scal, c->mf_work);
+    k_meanflow<<<1, 32, 0, c->stream>>>(c->d, c->g, beta, bdt, c->qxt, c->ctpress, c->u1, c->scal, c->mf_work, ghosts);
     LK("k_meanflow");
     return CFD_OK;
 }
@@ -886,6 +938,7 @@ int solvep_kernel(cfd_ctx* c, int krk, bool with_div) {
         LK("k_mb_solve_p");
         return CFD_OK;
     }
+    if (c->colM) return col_solve(c, 2, krk, "k_col_solve_p");
     const dim3 gp((d.ncol + c->SNT - 1) / c->SNT);
     k_solve_p<false><<<gp, c->SNT, 0, c->stream>>>(d, c->g, dtirk, c->u1, c->u2, c->u3, c->p, c->psi,
                                                    with_div ? c->div : nullptr, c->cs, c->mean_diag, 0.0);
@@ -919,7 +972,15 @@ int substep(cfd_ctx* c, int krk) {
     int s;
     if ((s = nl_transforms<T2>(c)) != CFD_OK) return s;
     if ((s = rhs_kernel<T2, 7>(c, krk)) != CFD_OK) return s;
-    if ((s = ib_solve_all<T2>(c, krk)) != CFD_OK) return s;
+    if ((s = ib_all<T2>(c)) != CFD_OK) return s;
+    c->hx_valid = false;  // the solve changes u, v, w
+    if (c->colM) {
+        // the mean mode has no part in the pressure or its correction (kx = kz = 0), so
+        // meanflow_ctU may follow them; it then extrapolates its column's ghost rows itself
+        if ((s = col_solve(c, 7, krk, "k_col_solve")) != CFD_OK) return s;
+        return c->ctpress == 0 ? meanflow_kernel(c, krk, true) : CFD_OK;
+    }
+    if ((s = solve_kernel(c, krk)) != CFD_OK) return s;
     if (c->ctpress == 0 && (s = meanflow_kernel(c, krk)) != CFD_OK) return s;
     // solveP + v_corr in one column sweep (psi is not stored on this path)
     const Dims& d = c->d;
@@ -1080,6 +1141,7 @@ int create_impl(const cfd_config* cfg, const cfd_ib_list* ibu, const cfd_ib_list
     if (cfg->ny < 4 || cfg->dsty < 0) return fail(c, CFD_ERR_SIZE, "ny must be >= 4 and dsty >= 0");
     c->device = device;
     CK(cudaSetDevice(device));
+    CK(cudaDeviceGetAttribute(&c->nsm, cudaDevAttrMultiProcessorCount, device));
     CK(cudaStreamCreateWithFlags(&c->own_stream, cudaStreamNonBlocking));
     c->stream = c->own_stream;
     c->fx = fx;
@@ -1364,8 +1426,11 @@ int create_impl(const cfd_config* cfg, const cfd_ib_list* ibu, const cfd_ib_list
         const size_t hxs = (size_t)(2 * nyu + nyv) * d.ngal2 * d.nkx;
         if (mixed) AL(c->Hx, float2, hxs); else AL(c->Hx, double2, hxs);
     }
-    AL(c->cs, double, nc * nyu);
-    AL(c->cs_v, double, nc * nyv);
+    if ((s = col_table(c, cfg)) != CFD_OK) return s;
+    if (!c->colM) {  // the sweeps' scaled upper diagonals
+        AL(c->cs, double, nc * nyu);
+        AL(c->cs_v, double, nc * nyv);
+    }
     c->JC = tune_int(&cfd_tuning::rhs_chunk, "CFD_RHS_CHUNK", 4, 2, 64);
     c->SNT = 1 << ilog2(tune_int(&cfd_tuning::solve_cols, "CFD_SOLVE_THREADS", 64, 32, 256));
     c->nch = (d.nyu - 2 + c->JC - 1) / c->JC;
@@ -1910,6 +1975,7 @@ int cfd_get_scalars(cfd_ctx* c, double* mpgx, double* qx, double* dgx) {
     if (mpgx) *mpgx = h[0];
     if (qx) *qx = h[1];
     if (dgx) *dgx = h[2];
+    if (h[3] != 0.0) return fail(c, CFD_ERR_CUDA, "a transfer of the column solves did not complete");
     if (!std::isfinite(h[0]) || !std::isfinite(h[1]) || !std::isfinite(h[2]))
         return fail(c, CFD_ERR_NONFINITE, "non-finite mean-flow scalars (mpgx %g, Qx %g)", h[0], h[1]);
     return CFD_OK;
