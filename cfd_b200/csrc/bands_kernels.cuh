@@ -9,8 +9,10 @@
 // products of a plane that does not carry a column read as zero, as the reference's module
 // arrays do (allocated to zero, start.f90:613, and never transposed there).
 //
-// One thread per column walks its segments in turn; the one-band contexts keep the tuned
-// kernels of channel_kernels.cuh and never launch these.
+// One thread per column walks its segments in turn (the right-hand sides in chunks of planes:
+// 558 -> 54 us a substep at 128 x 97(+56) x 128 with a 64 x 64 middle band); the implicit solves
+// are the segment rows of k_col_solve (colsolve.cuh), and the sweeps here only take columns too
+// tall for it.  One-band contexts never launch these.
 #pragma once
 
 #include "channel_kernels.cuh"
@@ -24,9 +26,6 @@ struct MBSeg {
     double gwb, gwt;
 };
 
-__device__ __forceinline__ bool mb_long(const Dims& d, int i, int q) {
-    return i <= d.n1m / 2 && (q < d.n2m / 2 || q >= d.n2 - d.n2m / 2);
-}
 __device__ __forceinline__ MBSeg mb_seg(const Dims& d, const Geo& g, bool lng, int s) {
     const int m = d.ny - 2 - d.jb;  // N(3,2) = N(4,2)
     if (lng) return MBSeg{d.ju0, d.ju1, d.jv0, d.jv1, d.jp0, d.jp1, g.gwb, g.gwt};
@@ -48,9 +47,11 @@ __global__ void __launch_bounds__(256) k_mb_rhs(Dims d, Geo g, RKCoef c, const d
                                                 double2* __restrict__ du1, double2* __restrict__ du2,
                                                 double2* __restrict__ du3, const T2* __restrict__ S0,
                                                 const T2* __restrict__ S1, const T2* __restrict__ S2,
-                                                const T2* __restrict__ S3) {
+                                                const T2* __restrict__ S3, int JC) {
+    // one thread = one column and a chunk of JC planes (blockIdx.y), as k_rhs
     const int col = blockIdx.x * blockDim.x + threadIdx.x;
     if (col >= d.ncol) return;
+    const int c0 = d.ju0 + 1 + blockIdx.y * JC, c1 = c0 + JC - 1;
     const int i = col % d.nkx, q = col / d.nkx;
     const double kxv = g.kx[i], kzv = g.kz[q];
     const double k2 = (-kxv * kxv) + (-kzv * kzv);
@@ -61,7 +62,7 @@ __global__ void __launch_bounds__(256) k_mb_rhs(Dims d, Geo g, RKCoef c, const d
     constexpr bool RHS0 = (MODE & 1) != 0, NL = (MODE & 2) != 0, PRO = (MODE & 4) != 0;
     for (int s = 0; s < (lng ? 1 : 2); ++s) {
         const MBSeg S = mb_seg(d, g, lng, s);
-        for (int j = S.u0 + 1; j <= S.u1 - 1; ++j) {
+        for (int j = max(S.u0 + 1, c0); j <= min(S.u1 - 1, c1); ++j) {
             const size_t ju = (size_t)(j - d.ju0);
             const double2 a_m = u1[(ju - 1) * nc + col], a_0 = u1[ju * nc + col], a_p = u1[(ju + 1) * nc + col];
             const double2 w_m = u3[(ju - 1) * nc + col], w_0 = u3[ju * nc + col], w_p = u3[(ju + 1) * nc + col];
@@ -101,7 +102,7 @@ __global__ void __launch_bounds__(256) k_mb_rhs(Dims d, Geo g, RKCoef c, const d
             du1[ju * nc + col] = r1;
             du3[ju * nc + col] = r3;
         }
-        for (int j = S.v0 + 1; j <= S.v1 - 1; ++j) {
+        for (int j = max(S.v0 + 1, c0); j <= min(S.v1 - 1, c1); ++j) {
             const size_t jv = (size_t)(j - d.jv0);
             const double2 v_m = u2[(jv - 1) * nc + col], v_0 = u2[jv * nc + col], v_p = u2[(jv + 1) * nc + col];
             double2 r2;
@@ -128,7 +129,7 @@ __global__ void __launch_bounds__(256) k_mb_rhs(Dims d, Geo g, RKCoef c, const d
             if (PRO) r2 = dadd(v_0, dscl(c.dt, r2));
             du2[jv * nc + col] = r2;
         }
-        if (PRO) {
+        if (PRO && blockIdx.y == 0) {
             du1[(size_t)(S.u0 - d.ju0) * nc + col] = dc(0, 0);
             du3[(size_t)(S.u0 - d.ju0) * nc + col] = dc(0, 0);
             du1[(size_t)(S.u1 - d.ju0) * nc + col] = dc(0, 0);

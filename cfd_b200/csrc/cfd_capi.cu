@@ -690,16 +690,16 @@ template <typename T2, int MODE>
 int rhs_kernel(cfd_ctx* c, int krk) {
     const Dims& d = c->d;
     dim3 gb((d.ncol + 255) / 256);
+    gb.y = c->nch;
     prof_mark(c);
     if (c->mb) {
         k_mb_rhs<T2, MODE><<<gb, 256, 0, c->stream>>>(d, c->g, coef(c, krk), c->scal, c->u1, c->u2, c->u3, c->p,
                                                       (T2*)c->Nu1, (T2*)c->Nu2, (T2*)c->Nu3, c->du1, c->du2, c->du3,
                                                       (const T2*)c->S[0], (const T2*)c->S[1], (const T2*)c->S[2],
-                                                      (const T2*)c->S[3]);
+                                                      (const T2*)c->S[3], c->JC);
         LK("k_mb_rhs");
         return CFD_OK;
     }
-    gb.y = c->nch;
     k_rhs<T2, MODE><<<gb, 256, 0, c->stream>>>(d, c->g, coef(c, krk), c->scal, c->u1, c->u2, c->u3, c->p, (T2*)c->Nu1,
                                                (T2*)c->Nu2, (T2*)c->Nu3, c->du1, c->du2, c->du3, (const T2*)c->S[0],
                                                (const T2*)c->S[1], (const T2*)c->S[2], (const T2*)c->S[3], c->JC);
@@ -847,7 +847,7 @@ int col_solve(cfd_ctx* c, int mode, int krk, const char* name) {
     a.err = c->scal + 3;
     a.ahead = col_ahead(c->colC, c->d.ncol);
     prof_mark(c);
-    col_launch(mode, c->colM, c->colC, c->nsm, c->stream, c->d, c->g, mode == 2 ? c->colmap_p : c->colmap, a);
+    col_launch(mode, c->colM, c->colC, c->mb, c->nsm, c->stream, c->d, c->g, mode == 2 ? c->colmap_p : c->colmap, a);
     return launched(c, name);
 }
 
@@ -858,10 +858,10 @@ int col_solve(cfd_ctx* c, int mode, int krk, const char* name) {
 // tridLU_3D_IB.f90:417-491); 0 where there is none.
 int col_table(cfd_ctx* c, const cfd_config* cfg) {
     const Dims& d = c->d;
-    c->colM = c->mb ? 0 : col_rows_per_lane(d.nyu);
+    c->colM = col_rows_per_lane(d.nyu);
     const int m = c->colM;
     if (!m) return CFD_OK;
-    c->colC = env_int("CFD_SOLVE_GROUP", col_cols(m, d.ncol), 4, 8) == 8 && m <= 15 ? 8 : 4;
+    c->colC = env_int("CFD_SOLVE_GROUP", col_cols(m, d.ncol), 4, 8) == 8 && m <= 15 && !c->mb ? 8 : 4;
     std::vector<double> h((size_t)32 * m * kColTabs, 0.0);
     for (int r = 0; r < 32 * m; ++r) {
         double* e = &h[(size_t)(r % m) * kColTabs * 32 + r / m];
@@ -879,7 +879,7 @@ int col_table(cfd_ctx* c, const cfd_config* cfg) {
     }
     AL(c->coltab, double, h.size());
     CK(cudaMemcpy(c->coltab, h.data(), sizeof(double) * h.size(), cudaMemcpyHostToDevice));
-    CK(col_prepare(m));
+    CK(col_prepare(m, c->mb));
     ColMaps &a = c->colmap, &b = c->colmap_p;
     const int nu = d.nyu, nv = d.nyv, np = d.nyp;
     const struct { CUtensorMap* map; const void* f; int n; } all[] = {
@@ -906,6 +906,7 @@ int launch_solve(cfd_ctx* c, cudaStream_t st, double beta, int part0, int nsys) 
 int solve_kernel(cfd_ctx* c, int krk) {
     const Dims& d = c->d;
     const double beta = kRKb[krk - 1] * c->dt / c->re;
+    if (c->colM) return col_solve(c, 1, krk, "k_col_solve_uvw");
     prof_mark(c);
     if (c->mb) {
         dim3 gb((d.ncol + 255) / 256);
@@ -914,7 +915,6 @@ int solve_kernel(cfd_ctx* c, int krk) {
         LK("k_mb_solve_uvw");
         return CFD_OK;
     }
-    if (c->colM) return col_solve(c, 1, krk, "k_col_solve_uvw");
     return launch_solve(c, c->stream, beta, 0, 2);
 }
 
@@ -931,6 +931,7 @@ int solvep_kernel(cfd_ctx* c, int krk, bool with_div) {
     const Dims& d = c->d;
     const double dtirk = (1.0 / c->dt) / (kRKa[krk - 1] + kRKb[krk - 1]);
     dim3 gb((d.ncol + 255) / 256);
+    if (c->colM) return col_solve(c, 2, krk, "k_col_solve_p");
     prof_mark(c);
     if (c->mb) {
         k_mb_solve_p<false><<<gb, 256, 0, c->stream>>>(d, c->g, dtirk, c->u1, c->u2, c->u3, c->p, c->psi,
@@ -938,7 +939,6 @@ int solvep_kernel(cfd_ctx* c, int krk, bool with_div) {
         LK("k_mb_solve_p");
         return CFD_OK;
     }
-    if (c->colM) return col_solve(c, 2, krk, "k_col_solve_p");
     const dim3 gp((d.ncol + c->SNT - 1) / c->SNT);
     k_solve_p<false><<<gp, c->SNT, 0, c->stream>>>(d, c->g, dtirk, c->u1, c->u2, c->u3, c->p, c->psi,
                                                    with_div ? c->div : nullptr, c->cs, c->mean_diag, 0.0);

@@ -49,6 +49,11 @@ struct Geo {
     double gw1t, gw3b;  // three bands: gridweighting(1,2) and gridweighting(3,1)
 };
 
+// three bands: the column's mode exists in the middle band too
+__device__ __forceinline__ bool mb_long(const Dims& d, int i, int q) {
+    return i <= d.n1m / 2 && (q < d.n2m / 2 || q >= d.n2 - d.n2m / 2);
+}
+
 __device__ __forceinline__ int row_of(const Dims& d, int q) { return q < d.n2 / 2 ? q : q + (d.ngal2 - d.n2); }
 
 __device__ __forceinline__ double2 dc(double a, double b) { double2 r; r.x = a; r.y = b; return r; }

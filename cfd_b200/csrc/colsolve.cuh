@@ -214,10 +214,14 @@ struct ColArgs {
     bool ahead;         // prefetch the next columns into L2 while these are solved
 };
 
+// MB: a three-band channel.  A short column (a mode of the wall bands only) is two independent
+// segments, u rows 0..bu and tu..nyu-1 with v and p rows to match; the rows between are identity
+// rows with zero right-hand sides, and the segments' inner ends the band-interface rows.
+//
 // MODE bits: 1 = the Helmholtz solves of u, v, w; 2 = solveP on the velocities, p += psi; 4 =
 // v_corr.  7 is the substep's, 1 and 2 are the stage entry points' (2 stores psi and the
 // divergence).
-template <int M, int C, int MODE>
+template <int M, int C, int MODE, bool MB>
 __global__ void __launch_bounds__(32 * C * col_groups(M, C))
     k_col_solve(Dims d, Geo g, const __grid_constant__ ColMaps maps, ColArgs A) {
     constexpr int G = col_groups(M, C), NB = col_boxes(M), BR = 32 * M / NB, RB = col_region(M, C), PB = 16 * C;
@@ -273,12 +277,16 @@ __global__ void __launch_bounds__(32 * C * col_groups(M, C))
     auto row = [&](int f, int r) -> double2& { return *reinterpret_cast<double2*>(reg + f * RB + r * PB + swz(r)); };
     const bool top = lane == 31;  // its row M would be the region's end: never part of a column
 
+    const int bu = d.jb + 2 - d.ju0, tu = d.ny - 2 - d.jb - d.ju0;
     unsigned phase = 0;
     bool ok = true;
     for (; q < nq; q += stride, phase ^= 1) {
         const int col = min(q * C + wc, d.ncol - 1);
         const double kxv = g.kx[col % d.nkx], kzv = g.kz[col / d.nkx];
         const double k2 = -kxv * kxv - kzv * kzv;
+        const bool sh = MB && !mb_long(d, col % d.nkx, col / d.nkx);  // a short column
+        // the weight of the face above p row r (0 at the ends of the column or segment)
+        auto face = [&](int i, int r) { return MB && sh && r >= bu - 2 && r < tu ? 0.0 : T(i, 7); };
         ok = mbar_wait(bar, phase);
         if (!ok) break;
         if (lead) {
@@ -299,6 +307,7 @@ __global__ void __launch_bounds__(32 * C * col_groups(M, C))
                     a = A.beta * T(i, 3);
                     c = A.beta * T(i, 5);
                     s = 1.0 - A.beta * (T(i, 4) + (r > 0 && r < n - 1 ? k2 : 0.0));
+                    if (MB && sh && r >= bu - 1 && r <= tu) { a = c = 0.0; s = 1.0; }
                 });
 #pragma unroll
                 for (int i = 0; i < M; ++i) R(2, i) = y[0][i];
@@ -310,6 +319,11 @@ __global__ void __launch_bounds__(32 * C * col_groups(M, C))
                 a = r == n - 1 ? -g.gwt : A.beta * T(i, 0);
                 c = r == 0 ? -g.gwb : A.beta * T(i, 2);
                 s = r > 0 && r < n - 1 ? 1.0 - A.beta * (T(i, 1) + k2) : 1.0 - (a + c);
+                if (MB && sh && r >= bu && r <= tu) {
+                    a = r == bu ? -g.gw1t : 0.0;
+                    c = r == tu ? -g.gw3b : 0.0;
+                    s = 1.0 - (a + c);
+                }
             };
             if constexpr (M <= 15) {
                 double2 y[2][M];
@@ -351,19 +365,20 @@ __global__ void __launch_bounds__(32 * C * col_groups(M, C))
                 const bool in = i < M - 1 || !top;
                 const double2 va = in ? R(2, i + 1) : vb;
                 if (!(UVW && M <= 15)) ps[0][i] = in ? dadd(dik(kxv, R(0, i + 1)), dik(kzv, R(1, i + 1))) : dc(0, 0);
-                const double2 v = dadd(ps[0][i], dscl(T(i, 6), dsub(va, vb)));
+                double2 v = dadd(ps[0][i], dscl(T(i, 6), dsub(va, vb)));
+                if (MB && sh && r > bu - 2 && r < tu) v = dc(0, 0);
                 vb = va;
                 if (MODE == 2) dv[i] = v;
                 ps[0][i] = (r < n && !(mean && r == 0)) ? dscl(-A.dtirk, v) : dc(0, 0);
             }
             // D.G: the off-diagonals are dthdyu of the centre times dthdyv of the faces (0 at walls)
-            const double dlow = __shfl_up_sync(0xffffffffu, T(M - 1, 7), 1);
+            const double dlow = __shfl_up_sync(0xffffffffu, face(M - 1, row0 + M - 1), 1);
             warp_tridiag<M, 1>(ps, [&](int i, double& a, double& c, double& s) {
                 const int r = row0 + i;
                 const double dt = T(i, 6);
-                a = dt * (i > 0 ? T(i > 0 ? i - 1 : 0, 7) : (lane ? dlow : 0.0));
-                c = dt * T(i, 7);
-                s = r < n ? -k2 : 1.0;
+                a = dt * (i > 0 ? face(i > 0 ? i - 1 : 0, r - 1) : (lane ? dlow : 0.0));
+                c = dt * face(i, r);
+                s = r < n && !(MB && sh && r > bu - 2 && r < tu) ? -k2 : 1.0;
                 if (mean && r == 0) { s = A.mean_diag; c = 0.0; }
             });
             __syncwarp();
@@ -387,7 +402,7 @@ __global__ void __launch_bounds__(32 * C * col_groups(M, C))
                 for (int i = 0; i < M; ++i) {
                     if (i == M - 1 && top) break;
                     if (f < 2) R(f, i + 1) = dsub(x[i], dik(A.dtrk * (f ? kzv : kxv), ps[0][i]));
-                    else R(f, i + 1) = dsub(x[i], dscl(A.dtrk * T(i, 7), dsub(i < M - 1 ? ps[0][i < M - 1 ? i + 1 : 0] : pn, ps[0][i])));
+                    else R(f, i + 1) = dsub(x[i], dscl(A.dtrk * face(i, row0 + i), dsub(i < M - 1 ? ps[0][i < M - 1 ? i + 1 : 0] : pn, ps[0][i])));
                 }
             }
             __syncwarp();
@@ -434,11 +449,15 @@ __global__ void __launch_bounds__(32 * C * col_groups(M, C))
     if (lead) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
 }
 
-// Host side (colsolve.cu)
-cudaError_t col_prepare(int m);  // raises the shared-memory limit of the kernels
-// tensor map of a field of n planes for columns of m rows per lane; false if it cannot be made
+// Host side (colsolve.cu; the _mb forms in colsolve_mb.cu): m rows per lane, cols columns a group
+// (4 in three bands), mb three bands
+cudaError_t col_prepare(int m, bool mb);  // raises the shared-memory limit of the kernels
+cudaError_t col_prepare_mb(int m);
+// tensor map of a field of n planes; false if it cannot be made
 bool col_map(CUtensorMap* map, const void* field, int ncol, int n, int m, int cols);
-void col_launch(int mode, int m, int cols, int nsm, cudaStream_t st, const Dims& d, const Geo& g, const ColMaps& maps,
-                const ColArgs& a);
+void col_launch(int mode, int m, int cols, bool mb, int nsm, cudaStream_t st, const Dims& d, const Geo& g,
+                const ColMaps& maps, const ColArgs& a);
+void col_launch_mb(int mode, int m, int nsm, cudaStream_t st, const Dims& d, const Geo& g, const ColMaps& maps,
+                   const ColArgs& a);
 
 }  // namespace cfd
