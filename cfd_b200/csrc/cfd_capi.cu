@@ -801,7 +801,8 @@ int ib_grid(cfd_ctx* c, const IBDev& ib, int j0, int nb, double2* rhs_a, double2
         dim3 g5((d.nkx + CH - 1) / CH, ib.npl, nb);
         FFT_SWITCH(d.ngal2, {
             k_ib_zfwd<T2, NF><<<g5, 256, zsmem(d.ngal2, CH, e), c->stream>>>(d, (const T2*)Hib, ib.npl, dst, j0,
-                                                                            ib.planes, c->fz, twz<T2>(c), CH, ilog2(CH));
+                                                                            ib.planes,
+                                                                            c->RWIX2 ? ib.rowflag : nullptr, c->fz, twz<T2>(c), CH, ilog2(CH));
         });
         LK("k_ib_zfwd");
     }

@@ -1311,7 +1311,8 @@ __global__ void __launch_bounds__(256) k_ib_xfwd(Dims d, T2* __restrict__ Hib, i
 // (planes_to_modes_dU/dV).  grid: x = kx chunk, y = plane, z = batch fb
 template <typename T2, int NF>
 __global__ void __launch_bounds__(256) k_ib_zfwd(Dims d, const T2* __restrict__ Hib, int npl, IBDst dst, int j0,
-                                                 const int* __restrict__ planes, FFTDesc fz, const T2* __restrict__ twz,
+                                                 const int* __restrict__ planes,
+                                                 const unsigned char* __restrict__ rowflag, FFTDesc fz, const T2* __restrict__ twz,
                                                  int CH, int bshift) {
     using R = decltype(T2::x);
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -1324,7 +1325,10 @@ __global__ void __launch_bounds__(256) k_ib_zfwd(Dims d, const T2* __restrict__ 
     const T2* H = Hib + ((size_t)(2 * fb) * npl + p) * (size_t)n * d.nkx;
     for (int t = threadIdx.x; t < (n << bshift); t += blockDim.x) {
         const int b = t & (CH - 1), z = t >> bshift, i = kx0 + b;
-        buf0[swz(z, b, bshift)] = i < d.nkx ? H[(size_t)z * d.nkx + i] : cx<T2>((R)0, (R)0);
+        T2 v = i < d.nkx ? H[(size_t)z * d.nkx + i] : cx<T2>((R)0, (R)0);
+        // rows left out of the x round trip lose Im of kx = 0 all the same (k_ib_zfwd2)
+        if (rowflag && i == 0 && !rowflag[z]) v.y = (R)0;
+        buf0[swz(z, b, bshift)] = v;
     }
     __syncthreads();
     T2* res = fft_batch<T2, NF, -1>(buf0, buf1, CH, bshift, fz, tw);
