@@ -5,7 +5,7 @@ import os
 import subprocess
 
 HERE = os.path.dirname(os.path.abspath(__file__))
-SRCS = [os.path.join(HERE, "csrc", f) for f in ("cfd_capi.cu", "colsolve.cu", "colsolve_mb.cu", "cfd_noalloc.cu")]
+SRCS = [os.path.join(HERE, "csrc", f) for f in sorted(os.listdir(os.path.join(HERE, "csrc"))) if f.endswith(".cu")]
 DEPS = SRCS + [os.path.join(HERE, "csrc", f) for f in sorted(os.listdir(os.path.join(HERE, "csrc")))
                if f.endswith(".cuh")] + [os.path.join(os.path.dirname(HERE), "include", "cfd_b200.h")]
 OUT = os.path.join(HERE, "_lib", "libcfdb200.so")

@@ -18,6 +18,7 @@
 
 #include "../../include/cfd_b200.h"
 #include "channel_kernels.cuh"
+#include "lines.cuh"
 #include "bands_kernels.cuh"
 #include "stats_kernels.cuh"
 #include "xmarch.cuh"
@@ -292,17 +293,14 @@ int ilog2(int b) {
         default: { constexpr int NF = 0; __VA_ARGS__; } break;    \
     }
 
-// Run BODY with (TN1, TN2) = the two-step split of n; sets ok = false if n has none.
-#define TWO_SWITCH(n, ok, ...)                                               \
-    switch (n) {                                                             \
-        case 64: { constexpr int TN1 = 8, TN2 = 8; __VA_ARGS__; } break;     \
-        case 96: { constexpr int TN1 = 8, TN2 = 12; __VA_ARGS__; } break;    \
-        case 128: { constexpr int TN1 = 8, TN2 = 16; __VA_ARGS__; } break;   \
-        case 192: { constexpr int TN1 = 16, TN2 = 12; __VA_ARGS__; } break;  \
-        case 384: { constexpr int TN1 = 16, TN2 = 24; __VA_ARGS__; } break;  \
-        case 768: { constexpr int TN1 = 32, TN2 = 24; __VA_ARGS__; } break;  \
-        default: ok = false; break;                                          \
-    }
+// the two-step split of a length, 0 x 0 if it has none; alt: the transposed one of a named length
+void line_split(int n, int& n1, int& n2, bool alt = false) {
+    const auto* k = line_kernels<float2>(n, alt);
+    n1 = k ? k->n1 : 0;
+    n2 = k ? k->n2 : 0;
+}
+// lengths a z plane of a three-band channel can have
+bool band_length(int n) { return n == 64 || n == 96 || n == 128 || n == 192 || n == 384 || n == 768; }
 
 // Splits of the marching x-line kernel (x-line path 6): its second step holds N2 = 8 or 16
 // points per lane, so that the unpack partners kb and N2 - kb share a warp
@@ -315,27 +313,6 @@ int ilog2(int b) {
         case 384: { constexpr int TN1 = 24, TN2 = 16; __VA_ARGS__; } break;  \
         default: ok = false; break;                                          \
     }
-
-// The transposed splits (the other radix order), selected by cfd_tuning.xsplit/zsplit = 2
-// for the x-line kernel and the nonlinear pass's z kernels.
-#define TWO_SWITCH_ALT(n, ok, ...)                                           \
-    switch (n) {                                                             \
-        case 64: { constexpr int TN1 = 16, TN2 = 4; __VA_ARGS__; } break;    \
-        case 96: { constexpr int TN1 = 12, TN2 = 8; __VA_ARGS__; } break;    \
-        case 128: { constexpr int TN1 = 16, TN2 = 8; __VA_ARGS__; } break;   \
-        case 192: { constexpr int TN1 = 12, TN2 = 16; __VA_ARGS__; } break;  \
-        case 384: { constexpr int TN1 = 24, TN2 = 16; __VA_ARGS__; } break;  \
-        case 768: { constexpr int TN1 = 24, TN2 = 32; __VA_ARGS__; } break;  \
-        default: ok = false; break;                                          \
-    }
-#define TWO_SWITCH_SEL(alt, n, ok, ...)          \
-    do {                                         \
-        if (alt) {                               \
-            TWO_SWITCH_ALT(n, ok, __VA_ARGS__);  \
-        } else {                                 \
-            TWO_SWITCH(n, ok, __VA_ARGS__);      \
-        }                                        \
-    } while (0)
 
 // shared memory of k_xline2 (elements): B*LX + N
 // Launch-shape overrides (unset: the built-in choice; a cfd_tuning field takes precedence).
@@ -388,75 +365,40 @@ int set_smem_attrs(cfd_ctx* c) {
         if (e == cudaSuccess) e = cudaFuncSetAttribute(k_ib_xinv<T2, NF>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)si);
         if (e == cudaSuccess) e = cudaFuncSetAttribute(k_ib_xfwd<T2, NF>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sf);
     });
+    auto set = [&](auto* f, size_t n) {
+        if (f && e == cudaSuccess) e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)n);
+    };
     if (c->LZ2 >= 0) {
-        bool ok = true;
-        TWO_SWITCH(n2, ok, {
-            if (e == cudaSuccess)
-                e = cudaFuncSetAttribute(k_zinv2<T2, TN1, TN2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)c->SMZ2);
-        });
-        TWO_SWITCH_SEL(c->ZALT, n2, ok, {
-            if (e == cudaSuccess)
-                e = cudaFuncSetAttribute(k_zinv2s<T2, TN1, TN2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)c->SMZN);
-            if (e == cudaSuccess)
-                e = cudaFuncSetAttribute(k_zfwd2<T2, TN1, TN2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)c->SMZN);
-            if constexpr (std::is_same<T2, double2>::value) {
-                if (e == cudaSuccess && c->ZR)
-                    e = cudaFuncSetAttribute(k_zinv2sd<TN1, TN2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)c->SMZN);
-                if (e == cudaSuccess && c->ZR)
-                    e = cudaFuncSetAttribute(k_zfwd2d<TN1, TN2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)c->SMZN);
-            }
-        });
-    }
-    if (c->LZ2 >= 0) {
-        bool ok = true;
-        TWO_SWITCH(n2, ok, {
-            if (e == cudaSuccess)
-                e = cudaFuncSetAttribute(k_ib_zinv2<T2, TN1, TN2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)c->SMZ2);
-            if (e == cudaSuccess)
-                e = cudaFuncSetAttribute(k_ib_zfwd2<T2, TN1, TN2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)c->SMZ2);
-        });
+        const auto* k = line_kernels<T2>(n2);
+        const auto* kn = line_kernels<T2>(n2, c->ZALT);
+        set(k->zinv2, c->SMZ2);
+        set(k->ib_zinv, c->SMZ2);
+        set(k->ib_zfwd, c->SMZ2);
+        set(kn->zinv2s, c->SMZN);
+        set(kn->zfwd2, c->SMZN);
+        set(kn->zinv2s_r, c->SMZN);
+        set(kn->zfwd2_r, c->SMZN);
     }
     if (c->RWIX2) {
-        bool ok = true;
-        TWO_SWITCH(n1, ok, {
-            if (e == cudaSuccess)
-                e = cudaFuncSetAttribute(k_ib_xinv2<T2, TN1, TN2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)c->SMIX2);
-            if (e == cudaSuccess)
-                e = cudaFuncSetAttribute(k_ib_xfwd2<T2, TN1, TN2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)c->SMFX2);
-        });
+        set(line_kernels<T2>(n1)->ib_xinv, c->SMIX2);
+        set(line_kernels<T2>(n1)->ib_xfwd, c->SMFX2);
     }
     if (c->RW2) {
-        bool ok = true;
-        TWO_SWITCH_SEL(c->XALT, n1, ok, {
-            if (e == cudaSuccess)
-                e = cudaFuncSetAttribute(k_xline2<T2, TN1, TN2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)c->SM2);
-            if constexpr (std::is_same<T2, float2>::value)
-                if (e == cudaSuccess && c->XR64)
-                    e = cudaFuncSetAttribute(k_xline2r<TN1, TN2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)c->SM2);
-        });
+        set(line_kernels<T2>(n1, c->XALT)->xline2, c->SM2);
+        if (c->XR64) set(line_kernels<T2>(n1, c->XALT)->xline2_r, c->SM2);
+        if (c->XL3) set(line_kernels<T2>(n1)->xline3, c->SM3);
+        if (c->RW4) set(line_kernels<T2>(n1)->xline4, c->SM4);
         if constexpr (std::is_same<T2, float2>::value)
             if (c->XMRW) {
-                MARCH_SWITCH(n1, ok, {
-                    if (e == cudaSuccess)
-                        e = cudaFuncSetAttribute(k_xmarch<float2, TN1, TN2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                 (int)c->SMXM);
-                });
+                bool ok = true;
+                MARCH_SWITCH(n1, ok, set(k_xmarch<float2, TN1, TN2>, c->SMXM););
             }
-        TWO_SWITCH(n1, ok, {
-            if (e == cudaSuccess && c->XL3)
-                e = cudaFuncSetAttribute(k_xline3<T2, TN1, TN2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)c->SM3);
-            if constexpr (std::is_same<T2, float2>::value)
-                if (e == cudaSuccess && c->RW4)
-                    e = cudaFuncSetAttribute(k_xline4<TN1, TN2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)c->SM4);
-        });
     }
     if (c->mb && c->LZ2 >= 0) {
-        bool ok = true;
-        const int smz = (int)std::max(c->SMZ2, c->SMZm);
-        TWO_SWITCH(c->dM.ngal2, ok, {
-            if (e == cudaSuccess) e = cudaFuncSetAttribute(k_zinv2<T2, TN1, TN2>, cudaFuncAttributeMaxDynamicSharedMemorySize, smz);
-            if (e == cudaSuccess) e = cudaFuncSetAttribute(k_zfwd2<T2, TN1, TN2>, cudaFuncAttributeMaxDynamicSharedMemorySize, smz);
-        });
+        const auto* k = line_kernels<T2>(c->dM.ngal2);
+        const size_t smz = std::max(c->SMZ2, c->SMZm);
+        set(k->zinv2, smz);
+        set(k->zfwd2, smz);
         FFT_SWITCH(c->dM.ngal1, {
             if (e == cudaSuccess) e = cudaFuncSetAttribute(k_xline<T2, NF>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sx);
         });
@@ -506,12 +448,9 @@ int nl_transforms_mb(cfd_ctx* c) {
         const Dims& d = *bp;
         const bool mid = bp == &c->dM;
         dim3 gz2((std::max(d.nsu, d.nsv) * d.nkx + CH2 - 1) / CH2, 3, 2);
-        bool ok = true;
-        TWO_SWITCH(d.ngal2, ok, {
-            k_zinv2<T2, TN1, TN2><<<gz2, mid ? c->NTZm : c->NTZ2, mid ? c->SMZm : c->SMZ2, c->stream>>>(
-                d, c->g, c->u1, c->u2, c->u3, (T2*)c->H[0], (T2*)c->H[1], (T2*)c->H[2], twz_b(mid), c->LZ2);
-        });
-        if (!ok) return fail(c, CFD_ERR_SIZE, "no two-step split for Ngal2=%d", d.ngal2);
+        const auto* k = line_kernels<T2>(d.ngal2);
+        k->zinv2<<<gz2, mid ? c->NTZm : c->NTZ2, mid ? c->SMZm : c->SMZ2, c->stream>>>(
+            d, c->g, c->u1, c->u2, c->u3, (T2*)c->H[0], (T2*)c->H[1], (T2*)c->H[2], twz_b(mid), c->LZ2);
     }
     LK("k_zinv2");
     prof_mark(c);
@@ -531,12 +470,9 @@ int nl_transforms_mb(cfd_ctx* c) {
         const Dims& d = *bp;
         const bool mid = bp == &c->dM;
         dim3 gf2((std::max(d.nsu, d.nsv) * d.nkx + CH2 - 1) / CH2, 4, 2);
-        bool ok = true;
-        TWO_SWITCH(d.ngal2, ok, {
-            k_zfwd2<T2, TN1, TN2><<<gf2, mid ? c->NTZm : c->NTZ2, mid ? c->SMZm : c->SMZ2, c->stream>>>(
-                d, (T2*)c->H[0], (T2*)c->H[1], (T2*)c->H[2], (T2*)c->H[3], (T2*)c->S[0], (T2*)c->S[1], (T2*)c->S[2],
-                (T2*)c->S[3], twz_b(mid), c->LZ2);
-        });
+        line_kernels<T2>(d.ngal2)->zfwd2<<<gf2, mid ? c->NTZm : c->NTZ2, mid ? c->SMZm : c->SMZ2, c->stream>>>(
+            d, (T2*)c->H[0], (T2*)c->H[1], (T2*)c->H[2], (T2*)c->H[3], (T2*)c->S[0], (T2*)c->S[1], (T2*)c->S[2],
+            (T2*)c->S[3], twz_b(mid), c->LZ2);
     }
     LK("k_zfwd2");
     return CFD_OK;
@@ -553,30 +489,16 @@ int nl_transforms(cfd_ctx* c) {
         // each field transformed once on its own planes; the x-line kernel interpolates in y
         const int CH2 = 1 << c->LZ2;
         dim3 gz2((std::max(d.nyu, d.nyv) * d.nkx + CH2 - 1) / CH2, 3);
-        bool ok = true;
-        TWO_SWITCH_SEL(c->ZALT, d.ngal2, ok, {
-            bool capped = false;
-            if constexpr (std::is_same<T2, double2>::value) {
-                if (c->ZR) {
-                    k_zinv2sd<TN1, TN2><<<gz2, c->NTZN, c->SMZN, c->stream>>>(d, c->u1, c->u2, c->u3, (double2*)c->Hx,
-                                                                            twz<double2>(c), c->LZ2);
-                    capped = true;
-                }
-            }
-            if (!capped)
-                k_zinv2s<T2, TN1, TN2><<<gz2, c->NTZN, c->SMZN, c->stream>>>(d, c->u1, c->u2, c->u3, (T2*)c->Hx,
-                                                                          twz<T2>(c), c->LZ2);
-        });
+        const auto* k = line_kernels<T2>(d.ngal2, c->ZALT);
+        (c->ZR ? k->zinv2s_r : k->zinv2s)<<<gz2, c->NTZN, c->SMZN, c->stream>>>(d, c->u1, c->u2, c->u3, (T2*)c->Hx,
+                                                                              twz<T2>(c), c->LZ2);
         LK("k_zinv2s");
         c->hx_valid = true;
     } else if (c->LZ2 >= 0) {
         const int CH2 = 1 << c->LZ2;
         dim3 gz2((std::max(d.nyu, d.nyv) * d.nkx + CH2 - 1) / CH2, 3, 2);
-        bool ok = true;
-        TWO_SWITCH(d.ngal2, ok, {
-            k_zinv2<T2, TN1, TN2><<<gz2, c->NTZ2, c->SMZ2, c->stream>>>(d, c->g, c->u1, c->u2, c->u3, (T2*)c->H[0],
-                                                                     (T2*)c->H[1], (T2*)c->H[2], twz<T2>(c), c->LZ2);
-        });
+        line_kernels<T2>(d.ngal2)->zinv2<<<gz2, c->NTZ2, c->SMZ2, c->stream>>>(
+            d, c->g, c->u1, c->u2, c->u3, (T2*)c->H[0], (T2*)c->H[1], (T2*)c->H[2], twz<T2>(c), c->LZ2);
         LK("k_zinv2");
     } else {
         dim3 gz((d.nkx + CH - 1) / CH, d.nslot, 3);
@@ -589,18 +511,13 @@ int nl_transforms(cfd_ctx* c) {
     }
     prof_mark(c);
     bool xdone = false;
-    if constexpr (std::is_same<T2, float2>::value) {
-        if (c->RW4) {
-            dim3 gx4(d.ngal2 / c->RW4, d.nslot);
-            bool ok = true;
-            TWO_SWITCH(d.ngal1, ok, {
-                k_xline4<TN1, TN2><<<gx4, c->NT4, c->SM4, c->stream>>>(d, c->g, (const float2*)c->Hx, (float2*)c->H[0],
-                                                                     (float2*)c->H[1], (float2*)c->H[2],
-                                                                     (float2*)c->H[3], twx<float2>(c), c->RW4);
-            });
-            LK("k_xline4");
-            xdone = true;
-        }
+    const auto* kx = c->RW2 ? line_kernels<T2>(d.ngal1, c->XALT) : nullptr;
+    if (c->RW4) {
+        dim3 gx4(d.ngal2 / c->RW4, d.nslot);
+        kx->xline4<<<gx4, c->NT4, c->SM4, c->stream>>>(d, c->g, (const T2*)c->Hx, (T2*)c->H[0], (T2*)c->H[1],
+                                                     (T2*)c->H[2], (T2*)c->H[3], twx<T2>(c), c->RW4);
+        LK("k_xline4");
+        xdone = true;
     }
     if constexpr (std::is_same<T2, float2>::value) {
         if (!xdone && c->XMRW) {
@@ -618,31 +535,14 @@ int nl_transforms(cfd_ctx* c) {
     if (xdone) {
     } else if (c->RW2 && c->XL3) {
         dim3 gx3(d.ngal2 / c->RW2, d.nslot);
-        bool ok = true;
-        TWO_SWITCH(d.ngal1, ok, {
-            k_xline3<T2, TN1, TN2><<<gx3, c->NT2, c->SM3, c->stream>>>(d, c->g, (const T2*)c->Hx, (T2*)c->H[0],
-                                                                    (T2*)c->H[1], (T2*)c->H[2], (T2*)c->H[3],
-                                                                    twx<T2>(c), c->RW2);
-        });
+        kx->xline3<<<gx3, c->NT2, c->SM3, c->stream>>>(d, c->g, (const T2*)c->Hx, (T2*)c->H[0], (T2*)c->H[1],
+                                                     (T2*)c->H[2], (T2*)c->H[3], twx<T2>(c), c->RW2);
         LK("k_xline3");
     } else if (c->RW2) {
-        dim3 gx2(d.ngal2 / c->RW2, d.nslot);
-        bool ok = true;
-        TWO_SWITCH_SEL(c->XALT, d.ngal1, ok, {
-            bool capped = false;
-            if constexpr (std::is_same<T2, float2>::value) {
-                if (c->XR64) {
-                    k_xline2r<TN1, TN2><<<gx2, c->NT2, c->SM2, c->stream>>>(
-                        d, c->g, (const float2*)c->Hx, (float2*)c->H[0], (float2*)c->H[1], (float2*)c->H[2],
-                        (float2*)c->H[3], twx<float2>(c), c->RW2, ilog2(c->RW2));
-                    capped = true;
-                }
-            }
-            if (!capped)
-                k_xline2<T2, TN1, TN2><<<gx2, c->NT2, c->SM2, c->stream>>>(d, c->g, (const T2*)c->Hx, (T2*)c->H[0],
-                                                                        (T2*)c->H[1], (T2*)c->H[2], (T2*)c->H[3],
-                                                                        twx<T2>(c), c->RW2, ilog2(c->RW2));
-        });
+        dim3 gx2((d.ngal2 + c->RW2 - 1) / c->RW2, d.nslot);
+        (c->XR64 ? kx->xline2_r : kx->xline2)<<<gx2, c->NT2, c->SM2, c->stream>>>(
+            d, c->g, (const T2*)c->Hx, (T2*)c->H[0], (T2*)c->H[1], (T2*)c->H[2], (T2*)c->H[3], twx<T2>(c), c->RW2,
+            ilog2(c->RW2));
         LK("k_xline2");
     } else {
         dim3 gx(d.ngal2 / c->RWx, d.nslot);
@@ -656,23 +556,10 @@ int nl_transforms(cfd_ctx* c) {
     if (c->LZ2 >= 0) {
         const int CH2 = 1 << c->LZ2;
         dim3 gf2((std::max(d.nyu, d.nyv) * d.nkx + CH2 - 1) / CH2, 4, 2);
-        bool ok = true;
-        TWO_SWITCH_SEL(c->ZALT, d.ngal2, ok, {
-            bool capped = false;
-            if constexpr (std::is_same<T2, double2>::value) {
-                if (c->ZR) {
-                    k_zfwd2d<TN1, TN2><<<gf2, c->NTZN, c->SMZN, c->stream>>>(
-                        d, (double2*)c->H[0], (double2*)c->H[1], (double2*)c->H[2], (double2*)c->H[3],
-                        (double2*)c->S[0], (double2*)c->S[1], (double2*)c->S[2], (double2*)c->S[3], twz<double2>(c),
-                        c->LZ2);
-                    capped = true;
-                }
-            }
-            if (!capped)
-                k_zfwd2<T2, TN1, TN2><<<gf2, c->NTZN, c->SMZN, c->stream>>>(
-                    d, (T2*)c->H[0], (T2*)c->H[1], (T2*)c->H[2], (T2*)c->H[3], (T2*)c->S[0], (T2*)c->S[1],
-                    (T2*)c->S[2], (T2*)c->S[3], twz<T2>(c), c->LZ2);
-        });
+        const auto* k = line_kernels<T2>(d.ngal2, c->ZALT);
+        (c->ZR ? k->zfwd2_r : k->zfwd2)<<<gf2, c->NTZN, c->SMZN, c->stream>>>(
+            d, (T2*)c->H[0], (T2*)c->H[1], (T2*)c->H[2], (T2*)c->H[3], (T2*)c->S[0], (T2*)c->S[1], (T2*)c->S[2],
+            (T2*)c->S[3], twz<T2>(c), c->LZ2);
         LK("k_zfwd2");
     } else {
         dim3 gf((d.nkx + CH - 1) / CH, d.nslot, 4);
@@ -727,11 +614,8 @@ int ib_grid(cfd_ctx* c, const IBDev& ib, int j0, int nb, double2* rhs_a, double2
     if (c->LZ2 >= 0) {
         const int CH2 = 1 << c->LZ2;
         dim3 g1((ib.npl * d.nkx + CH2 - 1) / CH2, 1, vel.H ? nb : 2 * nb);
-        bool ok = true;
-        TWO_SWITCH(d.ngal2, ok, {
-            k_ib_zinv2<T2, TN1, TN2><<<g1, c->NTZ2, c->SMZ2, c->stream>>>(d, src, j0, ib.planes, ib.npl, (T2*)Hib,
-                                                                        twz<T2>(c), c->LZ2, vel.H ? 2 : 1);
-        });
+        line_kernels<T2>(d.ngal2)->ib_zinv<<<g1, c->NTZ2, c->SMZ2, c->stream>>>(
+            d, src, j0, ib.planes, ib.npl, (T2*)Hib, twz<T2>(c), c->LZ2, vel.H ? 2 : 1);
         LK("k_ib_zinv2");
     } else {
         dim3 g1((d.nkx + CH - 1) / CH, ib.npl, 2 * nb);
@@ -744,13 +628,9 @@ int ib_grid(cfd_ctx* c, const IBDev& ib, int j0, int nb, double2* rhs_a, double2
     prof_mark(c);
     if (c->RWIX2) {
         dim3 g2((ib.nact + c->RWIX2 - 1) / c->RWIX2, ib.npl, nb);
-        bool ok = true;
         if (ib.nact > 0) {
-            TWO_SWITCH(d.ngal1, ok, {
-                k_ib_xinv2<T2, TN1, TN2><<<g2, c->NTIX2, c->SMIX2, c->stream>>>(d, (T2*)Hib, ib.npl, (R*)phys,
-                                                                              ib.arow, ib.nact, twx<T2>(c), c->RWIX2,
-                                                                              vel);
-            });
+            line_kernels<T2>(d.ngal1)->ib_xinv<<<g2, c->NTIX2, c->SMIX2, c->stream>>>(
+                d, (T2*)Hib, ib.npl, (R*)phys, ib.arow, ib.nact, twx<T2>(c), c->RWIX2, vel);
             LK("k_ib_xinv2");
         }
     } else {
@@ -770,12 +650,9 @@ int ib_grid(cfd_ctx* c, const IBDev& ib, int j0, int nb, double2* rhs_a, double2
     prof_mark(c);
     if (c->RWIX2) {
         dim3 g4((ib.nact + c->RWFX2 - 1) / c->RWFX2, ib.npl, nb);
-        bool ok = true;
         if (ib.nact > 0) {
-            TWO_SWITCH(d.ngal1, ok, {
-                k_ib_xfwd2<T2, TN1, TN2><<<g4, c->NTFX2, c->SMFX2, c->stream>>>(
-                    d, (T2*)Hib, ib.npl, (const R*)phys, ib.arow, ib.nact, twx<T2>(c), c->RWFX2);
-            });
+            line_kernels<T2>(d.ngal1)->ib_xfwd<<<g4, c->NTFX2, c->SMFX2, c->stream>>>(
+                d, (T2*)Hib, ib.npl, (const R*)phys, ib.arow, ib.nact, twx<T2>(c), c->RWFX2);
             LK("k_ib_xfwd2");
         }
     } else {
@@ -790,12 +667,8 @@ int ib_grid(cfd_ctx* c, const IBDev& ib, int j0, int nb, double2* rhs_a, double2
     if (c->LZ2 >= 0) {
         const int CH2 = 1 << c->LZ2;
         dim3 g5((ib.npl * d.nkx + CH2 - 1) / CH2, 1, nb);
-        bool ok = true;
-        TWO_SWITCH(d.ngal2, ok, {
-            k_ib_zfwd2<T2, TN1, TN2><<<g5, c->NTZ2, c->SMZ2, c->stream>>>(d, (const T2*)Hib, ib.npl, dst, j0,
-                                                                        ib.planes, c->RWIX2 ? ib.rowflag : nullptr,
-                                                                        twz<T2>(c), c->LZ2);
-        });
+        line_kernels<T2>(d.ngal2)->ib_zfwd<<<g5, c->NTZ2, c->SMZ2, c->stream>>>(
+            d, (const T2*)Hib, ib.npl, dst, j0, ib.planes, c->RWIX2 ? ib.rowflag : nullptr, twz<T2>(c), c->LZ2);
         LK("k_ib_zfwd2");
     } else {
         dim3 g5((d.nkx + CH - 1) / CH, ib.npl, nb);
@@ -1266,26 +1139,27 @@ int create_impl(const cfd_config* cfg, const cfd_ib_list* ibu, const cfd_ib_list
     if (d.ngal2 % c->RWibf) return fail(c, CFD_ERR_SIZE, "Ngal2 must be even");
     // the transposed split of the x-line transform (tuning xsplit = 2) is for path 1 only
     const int xpath = g_tuning && g_tuning->xline_path ? g_tuning->xline_path : env_int("CFD_XLINE_PATH", (mixed && d.ngal1 == 384) ? 6 : 1, 1, 6);
-    const bool xalt = (xpath == 1 || xpath == 5) && tune_int(&cfd_tuning::xsplit, "CFD_XSPLIT", 1, 1, 2) == 2;
+    // (the tuning variants exist for the six named lengths; the others run path 1)
+    const bool named = line_kernels_named<float2>(d.ngal1) != nullptr;
+    const bool xalt = named && (xpath == 1 || xpath == 5) && tune_int(&cfd_tuning::xsplit, "CFD_XSPLIT", 1, 1, 2) == 2;
     {
-        bool ok = true;
         int n1s = 0, n2s = 0;
-        TWO_SWITCH_SEL(xalt, d.ngal1, ok, { n1s = TN1; n2s = TN2; });
-        if (ok) {
+        line_split(d.ngal1, n1s, n2s, xalt);
+        if (n1s) {
             int rw = tune_int(&cfd_tuning::xline_rows, "CFD_XLINE_ROWS", 4, 2, 8);
             rw = 1 << (31 - __builtin_clz(rw));  // a power of two
-            while (rw >= 2 && ((d.ngal2 % rw) || xline2_smem(n1s, n2s, rw, esz) > budget)) rw /= 2;
-            if (rw >= 2 && d.ngal2 % rw == 0 && (2 * rw * n1s) % 32 == 0) {
+            while (rw >= 2 && ((named && d.ngal2 % rw) || xline2_smem(n1s, n2s, rw, esz) > budget)) rw /= 2;
+            if (rw >= 2) {
                 c->RW2 = rw;
-                c->NT2 = 2 * rw * std::max(n1s, n2s);
+                c->NT2 = (2 * rw * std::max(n1s, n2s) + 31) / 32 * 32;
                 c->SM2 = xline2_smem(n1s, n2s, rw, esz);
                 // packed lines (k_xline3): twiddles, exchange of 2*rw lines, physical rows /
                 // forward spectra
                 const size_t N = (size_t)n1s * n2s, LX = (size_t)((n1s * (n2s + 1)) | 1);
                 c->SM3 = (N + 2 * rw * LX + std::max((size_t)3 * (rw / 2) * N, (size_t)2 * rw * (N + 1))) * esz;
                 const int xp = xpath;
-                c->XL3 = xp == 3 && c->SM3 <= 220 * 1024;
-                if (xp == 4 && mixed) {
+                c->XL3 = named && xp == 3 && c->SM3 <= 220 * 1024;
+                if (named && xp == 4 && mixed) {
                     // line pairs: rows per CTA from the same tuning field, up to 8 (the
                     // kernel's launch bound, 8*max(N1,N2) threads)
                     int r4 = tune_int(&cfd_tuning::xline_rows, "CFD_XLINE_ROWS", 8, 2, 8);
@@ -1309,10 +1183,9 @@ int create_impl(const cfd_config* cfg, const cfd_ib_list* ibu, const cfd_ib_list
          env_int("CFD_XLINE_STOCKHAM", 0, 0, 1)))
         c->RW2 = 0;
     {
-        bool ok = true;
         int n1s = 0, n2s = 0;
-        TWO_SWITCH(d.ngal2, ok, { n1s = TN1; n2s = TN2; });
-        if (ok) {
+        line_split(d.ngal2, n1s, n2s);
+        if (n1s) {
             const int zl = g_tuning && (g_tuning->zlines == 4 || g_tuning->zlines == 8 || g_tuning->zlines == 16) ? g_tuning->zlines : 0;
             const int lb = zl ? ilog2(zl) : env_int("CFD_ZLINES_LOG2", mixed ? 4 : 3, 2, 4);
             c->LZ2 = lb;
@@ -1325,7 +1198,7 @@ int create_impl(const cfd_config* cfg, const cfd_ib_list* ibu, const cfd_ib_list
     if (c->LZ2 < 0) c->RW2 = 0;  // the two-step x-line kernels read the output of k_zinv2s
     if (!c->RW2) c->RW4 = 0;
     c->XALT = c->RW2 && xalt;  // (xalt implies path 1: neither k_xline3 nor k_xline4)
-    c->XR64 = c->RW2 && !c->XL3 && !c->RW4 && mixed && xpath == 5;
+    c->XR64 = c->RW2 && !c->XL3 && !c->RW4 && mixed && named && xpath == 5;
     // the x-line pass marching in y (FP32-mixed, one band; the default for 384-point x lines,
     // where it measured 0.607 against 0.811 ms per launch; at 64 and 192 points the per-slot
     // kernels were faster; FP64 contexts and lengths without its split run path 1): rows per
@@ -1357,28 +1230,26 @@ int create_impl(const cfd_config* cfg, const cfd_ib_list* ibu, const cfd_ib_list
     // 0.34 / 0.61 ms per launch at re550; the 768-point split spills at that cap
     c->ZR = c->RW2 && c->precision == CFD_PREC_FP64 && d.ngal2 <= 384 && env_int("CFD_Z_R112", 1, 0, 1);
     if (c->RW2 && c->LZ2 >= 0 && tune_int(&cfd_tuning::zsplit, "CFD_ZSPLIT", 1, 1, 2) == 2) {
-        bool ok = true;
         int n1s = 0, n2s = 0;
-        TWO_SWITCH_ALT(d.ngal2, ok, { n1s = TN1; n2s = TN2; });
-        if (ok) {
+        line_split(d.ngal2, n1s, n2s, true);
+        if (n1s) {
             c->ZALT = true;
             c->NTZN = (1 << c->LZ2) * std::max(n1s, n2s);
             c->SMZN = ((size_t)(1 << c->LZ2) * ((n1s * (n2s + 1)) | 1) + (size_t)n1s * n2s) * esz;
         }
     }
     {
-        bool ok = true;
         int n1s = 0, n2s = 0;
-        TWO_SWITCH(d.ngal1, ok, { n1s = TN1; n2s = TN2; });
-        if (ok) {
+        line_split(d.ngal1, n1s, n2s);
+        if (n1s) {
             const int N = n1s * n2s, L1 = (n1s * (n2s + 1)) | 1, mx = std::max(n1s, n2s);
             for (int rw = 8; rw >= 1; rw /= 2) {
                 const size_t sm = ((size_t)N + (size_t)rw * L1) * esz;
-                if (d.ngal2 % rw == 0 && sm <= budget && rw * mx <= 1024) { c->RWIX2 = rw; c->SMIX2 = sm; c->NTIX2 = rw * mx; break; }
+                if (sm <= budget && rw * mx <= 1024) { c->RWIX2 = rw; c->SMIX2 = sm; c->NTIX2 = rw * mx; break; }
             }
             for (int rw = 16; rw >= 2; rw /= 2) {
                 const size_t sm = ((size_t)N + (size_t)(rw / 2) * (N + 1) + (size_t)(rw / 2) * L1) * esz;
-                if (d.ngal2 % rw == 0 && sm <= budget && (rw / 2) * mx <= 1024) { c->RWFX2 = rw; c->SMFX2 = sm; c->NTFX2 = (rw / 2) * mx; break; }
+                if (sm <= budget && (rw / 2) * mx <= 1024) { c->RWFX2 = rw; c->SMFX2 = sm; c->NTFX2 = (rw / 2) * mx; break; }
             }
             if (!c->RWIX2 || !c->RWFX2) c->RWIX2 = c->RWFX2 = 0;
         }
@@ -1387,10 +1258,9 @@ int create_impl(const cfd_config* cfg, const cfd_ib_list* ibu, const cfd_ib_list
         // three bands: the per-slot interpolating z pass, the Stockham x-line kernel and the
         // two-step forward z pass, launched once per band; thread-per-column solves
         c->RW2 = 0; c->XL3 = false; c->RW4 = 0; c->XALT = c->ZALT = false; c->XR64 = false; c->ZR = false;
-        bool ok = true;
         int n1s = 0, n2s = 0;
-        TWO_SWITCH(cfg->ngal2_mid, ok, { n1s = TN1; n2s = TN2; });
-        if (c->LZ2 < 0 || !ok)
+        line_split(cfg->ngal2_mid, n1s, n2s);
+        if (!band_length(cfg->ngal2) || !band_length(cfg->ngal2_mid))
             return fail(c, CFD_ERR_SIZE, "three bands need two-step z lengths (64, 96, 128, 192, 384, 768) in both");
         c->NTZm = (1 << c->LZ2) * std::max(n1s, n2s);
         c->SMZm = ((size_t)(1 << c->LZ2) * ((n1s * (n2s + 1)) | 1) + (size_t)n1s * n2s) * esz;

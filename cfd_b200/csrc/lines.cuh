@@ -1,0 +1,97 @@
+// lines.cuh - the two-step transform kernels of every length, as a table of kernels per length.
+//
+// A length N = N1*N2 has its kernels where both factors fit a thread's registers: every even
+// 2^a 3^b from 12 to 768.  They are instantiated in lines_*.cu, a few lengths each, so that the
+// units compile side by side.  Against the radix-by-radix kernels that lengths other than the
+// named six (64, 96, 128, 192, 384, 768) ran before, microseconds a launch on B200 (z inverse, x,
+// z forward): 256 x 129 x 256 FP64 232, 602, 249 -> 46, 233, 85, FP32 177, 459, 152 -> 38, 147,
+// 49; 144 x 131 x 108 FP32 70, 146, 55 -> 8, 38, 13; 24 x 17(+6) x 18 FP64 4.1, 6.1, 3.9 -> 2.2,
+// 3.1, 2.3.  The shared-memory passes of those kernels, and a slot's z transform for each field
+// and slot instead of one a plane, were what they spent their time on.
+#pragma once
+
+#include "transform_kernels.cuh"
+
+namespace cfd {
+
+template <typename T2>
+struct LineKernels {
+    using R = decltype(T2::x);
+    int n1, n2;
+    void (*zinv2)(Dims, Geo, const double2*, const double2*, const double2*, T2*, T2*, T2*, const T2*, int);
+    void (*zinv2s)(Dims, const double2*, const double2*, const double2*, T2*, const T2*, int);
+    void (*zfwd2)(Dims, const T2*, const T2*, const T2*, const T2*, T2*, T2*, T2*, T2*, const T2*, int);
+    // the FP64 z kernels at 112 registers (null for FP32 and above 384 points)
+    void (*zinv2s_r)(Dims, const double2*, const double2*, const double2*, T2*, const T2*, int);
+    void (*zfwd2_r)(Dims, const T2*, const T2*, const T2*, const T2*, T2*, T2*, T2*, T2*, const T2*, int);
+    void (*xline2)(Dims, Geo, const T2*, T2*, T2*, T2*, T2*, const T2*, int, int);
+    // tuning variants of the six named lengths: 64 registers (FP32), packed rows, line pairs (FP32)
+    void (*xline2_r)(Dims, Geo, const T2*, T2*, T2*, T2*, T2*, const T2*, int, int);
+    void (*xline3)(Dims, Geo, const T2*, T2*, T2*, T2*, T2*, const T2*, int);
+    void (*xline4)(Dims, Geo, const T2*, T2*, T2*, T2*, T2*, const T2*, int);
+    void (*ib_zinv)(Dims, IBSrc, int, const int*, int, T2*, const T2*, int, int);
+    void (*ib_xinv)(Dims, const T2*, int, R*, const int*, int, const T2*, int, IBVel);
+    void (*ib_xfwd)(Dims, T2*, int, const R*, const int*, int, const T2*, int);
+    void (*ib_zfwd)(Dims, const T2*, int, IBDst, int, const int*, const unsigned char*, const T2*, int);
+};
+
+// The kernels of length n, null where it has none; alt: the transposed split of the six named
+// lengths (only zinv2s, zfwd2, xline2 and their variants).
+template <typename T2> const LineKernels<T2>* line_kernels(int n, bool alt = false);
+
+// what each unit holds (null for the lengths it does not)
+template <typename T2> const LineKernels<T2>* line_kernels_named(int n);
+template <typename T2> const LineKernels<T2>* line_kernels_alt(int n);
+template <typename T2> const LineKernels<T2>* line_kernels_small(int n);
+template <typename T2> const LineKernels<T2>* line_kernels_mid(int n);
+template <typename T2> const LineKernels<T2>* line_kernels_large(int n);
+template <typename T2> const LineKernels<T2>* line_kernels_large2(int n);
+template <> const LineKernels<float2>* line_kernels_named<float2>(int n);
+template <> const LineKernels<double2>* line_kernels_named<double2>(int n);
+template <> const LineKernels<float2>* line_kernels_alt<float2>(int n);
+template <> const LineKernels<double2>* line_kernels_alt<double2>(int n);
+template <> const LineKernels<float2>* line_kernels_small<float2>(int n);
+template <> const LineKernels<double2>* line_kernels_small<double2>(int n);
+template <> const LineKernels<float2>* line_kernels_mid<float2>(int n);
+template <> const LineKernels<double2>* line_kernels_mid<double2>(int n);
+template <> const LineKernels<float2>* line_kernels_large<float2>(int n);
+template <> const LineKernels<double2>* line_kernels_large<double2>(int n);
+template <> const LineKernels<float2>* line_kernels_large2<float2>(int n);
+template <> const LineKernels<double2>* line_kernels_large2<double2>(int n);
+template <> const LineKernels<float2>* line_kernels<float2>(int n, bool alt);
+template <> const LineKernels<double2>* line_kernels<double2>(int n, bool alt);
+
+enum { kLinesAll, kLinesNamed, kLinesAlt };
+
+template <typename T2, int N1, int N2, int WHAT>
+const LineKernels<T2>* line_table() {
+    constexpr bool F32 = sizeof(T2) == 8;
+    static const LineKernels<T2> k = [] {
+        LineKernels<T2> t{};
+        t.n1 = N1;
+        t.n2 = N2;
+        t.zinv2s = k_zinv2s<T2, N1, N2>;
+        t.zfwd2 = k_zfwd2<T2, N1, N2>;
+        t.xline2 = k_xline2<T2, N1, N2>;
+        if constexpr (!F32 && N1 * N2 <= 384) {
+            t.zinv2s_r = k_zinv2sd<N1, N2>;
+            t.zfwd2_r = k_zfwd2d<N1, N2>;
+        }
+        if constexpr (F32 && WHAT != kLinesAll) t.xline2_r = k_xline2r<N1, N2>;
+        if constexpr (WHAT == kLinesNamed) {
+            t.xline3 = k_xline3<T2, N1, N2>;
+            if constexpr (F32) t.xline4 = k_xline4<N1, N2>;
+        }
+        if constexpr (WHAT != kLinesAlt) {
+            t.zinv2 = k_zinv2<T2, N1, N2>;
+            t.ib_zinv = k_ib_zinv2<T2, N1, N2>;
+            t.ib_xinv = k_ib_xinv2<T2, N1, N2>;
+            t.ib_xfwd = k_ib_xfwd2<T2, N1, N2>;
+            t.ib_zfwd = k_ib_zfwd2<T2, N1, N2>;
+        }
+        return t;
+    }();
+    return &k;
+}
+
+}  // namespace cfd

@@ -1,0 +1,15 @@
+// lines_large2_f64.cu - two-step kernels of the lengths below (lines.cuh).
+#include "lines.cuh"
+
+namespace cfd {
+
+template <>
+const LineKernels<double2>* line_kernels_large2<double2>(int n) {
+    switch (n) {
+        case 576: return line_table<double2, 24, 24, kLinesAll>();
+        case 648: return line_table<double2, 24, 27, kLinesAll>();
+        default: return nullptr;
+    }
+}
+
+}  // namespace cfd

@@ -1,0 +1,19 @@
+// lines_mid_f32.cu - two-step kernels of the lengths below (lines.cuh).
+#include "lines.cuh"
+
+namespace cfd {
+
+template <>
+const LineKernels<float2>* line_kernels_mid<float2>(int n) {
+    switch (n) {
+        case 144: return line_table<float2, 12, 12, kLinesAll>();
+        case 162: return line_table<float2, 18, 9, kLinesAll>();
+        case 216: return line_table<float2, 12, 18, kLinesAll>();
+        case 256: return line_table<float2, 16, 16, kLinesAll>();
+        case 288: return line_table<float2, 16, 18, kLinesAll>();
+        case 324: return line_table<float2, 18, 18, kLinesAll>();
+        default: return nullptr;
+    }
+}
+
+}  // namespace cfd

@@ -1,0 +1,19 @@
+// lines_named_f64.cu - two-step kernels of the lengths below (lines.cuh).
+#include "lines.cuh"
+
+namespace cfd {
+
+template <>
+const LineKernels<double2>* line_kernels_named<double2>(int n) {
+    switch (n) {
+        case 64: return line_table<double2, 8, 8, kLinesNamed>();
+        case 96: return line_table<double2, 8, 12, kLinesNamed>();
+        case 128: return line_table<double2, 8, 16, kLinesNamed>();
+        case 192: return line_table<double2, 16, 12, kLinesNamed>();
+        case 384: return line_table<double2, 16, 24, kLinesNamed>();
+        case 768: return line_table<double2, 32, 24, kLinesNamed>();
+        default: return nullptr;
+    }
+}
+
+}  // namespace cfd
