@@ -11,6 +11,7 @@
 #include <cmath>
 #include <cstdarg>
 #include <cstdio>
+#include <cstdint>
 #include <cstdlib>
 #include <cstring>
 #include <string>
@@ -182,6 +183,12 @@ struct cfd_ctx {
         double* part = nullptr;   // [cp][ns][8] partial plane sums
         int nseg = 1;             // segments of tile rows of the conditional sums
         double* cpart = nullptr;  // [cp][2][nseg][6][dnx*dnz] their partial sums (nseg > 1)
+        // lengths with two-step transforms (k_st_z, k_st_x): planes of a chunk, and of a chunk
+        // with conditional sums; z-transformed fields, partial sums, folded rows
+        int lcp = 0, lcpc = 0, nrow = 0;
+        double2* hs = nullptr;
+        double* lpart = nullptr;
+        double* fold = nullptr;
         // spectra (spectra.f90): [plane][column] each; null when not configured
         double *spu = nullptr, *spv = nullptr, *spw = nullptr, *spuv = nullptr, *spp = nullptr;
     } st;
@@ -1348,6 +1355,16 @@ int strided_cft(cfd_ctx* c, double* dptr, int n, int ise, int isa, int m, long l
     if (!fft_plan(n, fd)) return fail(c, CFD_ERR_SIZE, "length %d not 2^a*3^b", n);
     const double2* tw = n == c->d.ngal2 ? c->twz_d : (n == c->d.ngal1 ? c->twx_d : nullptr);
     if (!tw) return fail(c, CFD_ERR_SIZE, "cft length must be Ngal2 or Ngal1");
+    if (const auto* k = line_kernels<double2>(n)) {
+        const bool a2 = ((uintptr_t)dptr & 15) == 0 && !((ise | isa | bstride) & 1);
+        auto* f = k->pl_cft[iopt < 0][a2];
+        const int lsm = (int)(((size_t)8 * ((k->n1 * (k->n2 + 1)) | 1) + n) * sizeof(double2));
+        CK(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, lsm));
+        prof_mark(c);
+        f<<<dim3((m + 7) / 8, nb), 8 * std::max(k->n1, k->n2), lsm, c->stream>>>(dptr, ise, isa, m, bstride, tw, 3);
+        LK("k_pl_cft");
+        return CFD_OK;
+    }
     const int CH = 8;
     const int sm = fft_generic_smem(n, CH);
     CK(cudaFuncSetAttribute(k_cft_strided, cudaFuncAttributeMaxDynamicSharedMemorySize, sm));
@@ -1363,6 +1380,23 @@ int strided_rft(cfd_ctx* c, double* dptr, int n, int isa, int m, long long bstri
     if (!fft_plan(n, fd) || (n & 1)) return fail(c, CFD_ERR_SIZE, "length %d not even 2^a*3^b", n);
     const double2* tw = n == c->d.ngal1 ? c->twx_d : (n == c->d.ngal2 ? c->twz_d : nullptr);
     if (!tw) return fail(c, CFD_ERR_SIZE, "rft length must be Ngal1 or Ngal2");
+    if (const auto* k = line_kernels<double2>(n)) {
+        // two lines a transform; as many transforms a CTA as keep two or more CTAs on an SM
+        const bool a2 = ((uintptr_t)dptr & 15) == 0 && !((isa | bstride) & 1);
+        auto* f = k->pl_rft[iopt <= 0][a2];
+        auto lsm = [&](int nl) {
+            return (int)((nl * (size_t)(((k->n1 * (k->n2 + 1)) | 1) + (iopt <= 0 ? n + 1 : 0)) + n) * sizeof(double2));
+        };
+        int nl = 8;
+        while (nl > 1 && lsm(nl) > 72 * 1024) nl /= 2;
+        CK(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, lsm(nl)));
+        const int pairs = (m + 1) / 2;
+        prof_mark(c);
+        f<<<dim3((pairs + nl - 1) / nl, nb), (nl * std::max(k->n1, k->n2) + 31) / 32 * 32, lsm(nl), c->stream>>>(
+            dptr, isa, m, bstride, tw, nl);
+        LK("k_pl_rft");
+        return CFD_OK;
+    }
     const int CH = 8;
     const int sm = fft_generic_smem(n, CH);
     CK(cudaFuncSetAttribute(k_rft_strided, cudaFuncAttributeMaxDynamicSharedMemorySize, sm));
@@ -1384,8 +1418,20 @@ void dfree(cfd_ctx* c, void* p) {
 
 // Plane scratch and maxima of the statistics pass (also used by the CFL query alone).
 int stats_scratch(cfd_ctx* c) {
-    if (c->st.planes) return CFD_OK;
+    if (c->st.planes || c->st.hs) return CFD_OK;
     const Dims& d = c->d;
+    if (line_kernels<double2>(d.ngal1) && line_kernels<double2>(d.ngal2)) {
+        // chunks of planes whose five transformed fields take about 64 MB, half the L2
+        const auto* kx = line_kernels<double2>(d.ngal1);
+        const size_t pb = (size_t)d.ngal2 * d.nkx * sizeof(double2);
+        c->st.lcp = (int)std::min<size_t>(d.nyu, std::max<size_t>(4, ((size_t)64 << 20) / (5 * pb)));
+        const int rw = st_x_lines(kx->n1, kx->n2) / 4;
+        c->st.nrow = (d.ngal2 + rw - 1) / rw;
+        AL(c->st.hs, double2, (size_t)(5 * c->st.lcp + 4) * d.ngal2 * d.nkx);
+        AL(c->st.lpart, double, (size_t)d.nyu * c->st.nrow * 32);
+        AL(c->st.mx, double, (size_t)3 * d.nyu);
+        return CFD_OK;
+    }
     AL(c->st.planes, double, (size_t)3 * c->st.cp * (d.ngal1 + 2) * d.ngal2);
     AL(c->st.mx, double, (size_t)3 * d.nyu);
     AL(c->st.part, double, (size_t)c->st.cp * c->st.ns * 8);
@@ -1442,10 +1488,49 @@ int stats_scratch(cfd_ctx* c) {
     return CFD_OK;
 }
 
-// One pass over the u, v and p planes in chunks of cp planes per field: build the planes
+// One pass over the planes in chunks: the maxima, and with acc the sums (stats_pass_lines where both
+// lengths have two-step transforms).  Otherwise, in chunks of cp planes per field: build the planes
 // of the chunk from the spectral state, transform them to physical space (FP64), reduce.
 // acc = false computes only the CFL maxima (u, w on u planes, v on v planes).
+int stats_pass_lines(cfd_ctx* c, bool acc) {
+    const Dims& d = c->d;
+    auto& st = c->st;
+    const auto *kz = line_kernels<double2>(d.ngal2), *kx = line_kernels<double2>(d.ngal1);
+    const bool cond = acc && st.dnx > 0;
+    const int cp = cond ? st.lcpc : st.lcp, nlr = acc ? 4 : 2, rw = st_x_lines(kx->n1, kx->n2) / nlr;
+    const int nrow = (d.ngal2 + rw - 1) / rw, nf = acc ? 5 : 3;
+    const size_t smz = ((size_t)8 * ((kz->n1 * (kz->n2 + 1)) | 1) + d.ngal2) * sizeof(double2);
+    const size_t smx = ((size_t)nlr * rw * st_x_row(kx->n1, kx->n2) + d.ngal1) * sizeof(double2);
+    const int ntx = (nlr * rw * std::max(kx->n1, kx->n2) + 31) / 32 * 32;
+    CK(cudaFuncSetAttribute(kz->st_z, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smz));
+    CK(cudaFuncSetAttribute(kx->st_x[acc], cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smx));
+    for (int j0 = 0; j0 < d.nyu; j0 += cp) {
+        const int n = std::min(cp, d.nyu - j0);
+        StChunk s{j0, n, {0, cp, 2 * cp + 1, 3 * cp + 4, 4 * cp + 4}, {j0, j0, j0 - 2, j0, j0}, {n, n + 1, n + 3, n, n}};
+        prof_mark(c);
+        kz->st_z<<<dim3(((n + 3) * d.nkx + 7) / 8, nf), 8 * std::max(kz->n1, kz->n2), smz, c->stream>>>(
+            d, c->g, s, c->u1, c->u2, c->u3, c->p, st.hs, c->twz_d, 3);
+        LK("k_st_z");
+        prof_mark(c);
+        kx->st_x[acc]<<<dim3(nrow, n), ntx, smx, c->stream>>>(d, c->g, s, st.hs, c->twx_d, rw, ilog2(rw), st.lpart,
+                                                             cond ? st.fold : nullptr, st.dnx, st.nbu, st.nbv, st.nbp);
+        LK("k_st_x");
+        const int nb = std::max(st.nbu, std::max(st.nbv, st.nbp));
+        if (cond && (j0 < nb || j0 + n > d.nyp - nb)) {
+            prof_mark(c);
+            k_st_fold<<<dim3((kStQ * st.dnx * st.dnz + 255) / 256, n), 256, 0, c->stream>>>(
+                d, st.fold, j0, st.dnx, st.dnz, st.nbu, st.nbv, st.nbp, st.cu, st.cv, st.cp_);
+            LK("k_st_fold");
+        }
+    }
+    prof_mark(c);
+    k_st_fin_lines<<<d.nyu, 256, 0, c->stream>>>(d, c->g, st.lpart, nrow, nlr, st.su, st.sv, st.sp, st.mx);
+    LK("k_st_fin_lines");
+    return CFD_OK;
+}
+
 int stats_pass(cfd_ctx* c, bool acc) {
+    if (c->st.hs) return stats_pass_lines(c, acc);
     const Dims& d = c->d;
     const Geo& g = c->g;
     auto& st = c->st;
@@ -1890,9 +1975,9 @@ int cfd_stats_configure(cfd_ctx* c, const cfd_stats_config* sc) {
             return fail(c, CFD_ERR_ARG, "tile %d x %d must divide Ngal1 x Ngal2", sc->dnx, sc->dnz);
         if (sc->jband + 1 > d.ju1) return fail(c, CFD_ERR_ARG, "jband %d above the channel", sc->jband);
     }
-    for (double* p : {st.su, st.sv, st.sp, st.cu, st.cv, st.cp_, st.spu, st.spv, st.spw, st.spuv, st.spp, st.cpart})
+    for (double* p : {st.su, st.sv, st.sp, st.cu, st.cv, st.cp_, st.spu, st.spv, st.spw, st.spuv, st.spp, st.cpart, st.fold})
         dfree(c, p);
-    st.su = st.sv = st.sp = st.cu = st.cv = st.cp_ = st.cpart = nullptr;
+    st.su = st.sv = st.sp = st.cu = st.cv = st.cp_ = st.cpart = st.fold = nullptr;
     st.spu = st.spv = st.spw = st.spuv = st.spp = nullptr;
     int s = stats_scratch(c);
     if (s) return s;
@@ -1912,7 +1997,12 @@ int cfd_stats_configure(cfd_ctx* c, const cfd_stats_config* sc) {
     AL(st.cp_, double, 2 * 2 * st.nbp * tsz);
     // conditional sums: tile rows split into segments so that a plane has about 1024 threads
     st.nseg = tsz ? (int)std::max<size_t>(1, std::min<size_t>({16, (size_t)(d.ngal2 / st.dnz), 1024 / tsz})) : 1;
-    if (st.nseg > 1) AL(st.cpart, double, (size_t)st.cp * 2 * st.nseg * 6 * tsz);
+    if (tsz && st.hs) {  // folded rows of a chunk, at most about 128 MB
+        const size_t row = (size_t)d.ngal2 * kStQ * st.dnx;
+        st.lcpc = (int)std::max<size_t>(1, std::min<size_t>(st.lcp, ((size_t)128 << 20) / (row * sizeof(double))));
+        AL(st.fold, double, st.lcpc * row);
+    }
+    if (st.nseg > 1 && !st.hs) AL(st.cpart, double, (size_t)st.cp * 2 * st.nseg * 6 * tsz);
     if (sc->spectra) {
         AL(st.spu, double, (size_t)d.nyu * d.ncol);
         AL(st.spv, double, (size_t)d.nyv * d.ncol);

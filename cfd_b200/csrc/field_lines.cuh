@@ -1,0 +1,336 @@
+// field_lines.cuh - FP64 two-step transforms of the statistics pass, the CFL query and the plane
+// entry points (sm_100a).
+//
+// Statistics (stats.f90:1-253) and dtc_calc (FOU3D.f90:516-544) reduce physical planes of u, v, w,
+// the y-interpolated v and w, omega_x and p.  Interpolation and dw/dy are linear in y and commute
+// with the transforms, so each field is transformed in z once on its own planes (k_st_z; dv/dz
+// takes its i kz there), and k_st_x forms the sources of a row from the transformed planes,
+// transforms them in x and reduces the physical values in registers: no physical plane is stored.
+// The planes go through in chunks whose transformed fields stay in L2.  The passes they replace
+// (planes built, transformed in place by radix-by-radix kernels and read again by the sums) moved 17
+// GB at 384 x 257(+90) x 384, 19.2 ms for a statistics call and a CFL query; here 3.8 ms, bound by the
+// FP64 transforms' latency at 12 warps an SM (k_st_x 86 us, k_st_z 27 us per 16 planes).  The plane
+// entry points (k_pl_cft, k_pl_rft) take a line through shared memory once instead of once a radix,
+// and two real lines a transform in both directions: 193 planes of 192 x 192, both ways, 264 -> 94 us.
+#pragma once
+
+#include "transform_kernels.cuh"
+
+namespace cfd {
+
+// One chunk: u planes j0..j0+cp-1, v and p planes of the same index, and the neighbours their
+// interpolations read.  Field f (u, w, v, dv/dz, p) holds planes first[f]..first[f]+n[f]-1 of its
+// grid (those that exist) from slot off[f] on.
+struct StChunk {
+    int j0, cp;
+    int off[5], first[5], n[5];
+};
+constexpr int kStQ = 13;  // conditional quantities: U U2 W W2 UV UW, V V2 wx wx2 VW, P P2
+
+template <int TN1, int TN2>
+__global__ void __launch_bounds__(8 * (TN1 > TN2 ? TN1 : TN2), (TN1 > TN2 ? TN1 : TN2) <= 24 ? 3 : 2)
+    k_st_z(Dims d, Geo g, StChunk s, const double2* __restrict__ u1, const double2* __restrict__ u2,
+           const double2* __restrict__ u3, const double2* __restrict__ p, double2* __restrict__ Hs,
+           const double2* __restrict__ twz, int lb) {
+    constexpr int N = TN1 * TN2;
+    const int f = blockIdx.y;
+    const int nlines = s.n[f] * d.nkx;
+    const int line0 = blockIdx.x << lb;
+    if (line0 >= nlines) return;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    double2* twt = reinterpret_cast<double2*>(smem_raw);
+    double2* ex = twt + N;
+    load_twiddles<double2, TN1, TN2>(twt, twz);
+    const int b = threadIdx.x & ((1 << lb) - 1);
+    const int line = min(line0 + b, nlines - 1);
+    const int pl = line / d.nkx, i = line - pl * d.nkx;
+    const int ny = f < 2 ? d.nyu : (f < 4 ? d.nyv : d.nyp);
+    const int j = s.first[f] + pl;
+    const bool live = line0 + b < nlines && j >= 0 && j < ny;
+    const double2* src = (f == 0 ? u1 : (f == 1 ? u3 : (f < 4 ? u2 : p))) + (size_t)min(max(j, 0), ny - 1) * d.ncol + i;
+    double2* H = Hs + ((size_t)s.off[f] + pl) * N * d.nkx + i;
+    const int r = threadIdx.x >> lb;
+    const bool dz = f == 3;
+    __syncthreads();
+    auto load = [&](int e, int) -> double2 {
+        const int q = zrow_q<N, TN2>(e, r);
+        if (q < 0) return dc(0, 0);
+        const double2 v = src[(size_t)q * d.nkx];
+        // the kz = -N2/2 mode of a z derivative is zero (der_z, FOU3D.f90:388-412)
+        return dz ? (q == d.n2 / 2 ? dc(0, 0) : dik(g.kz[q], v)) : v;
+    };
+    auto store = [&](int z, int, double2 v) {
+        if (live) H[(size_t)z * d.nkx] = v;
+    };
+    two_step_lines<double2, TN1, TN2, +1>(lb, ex, twt, load, store);
+}
+
+// |a| as its bit pattern, which orders like the value and puts NaN above all: a maximum that keeps
+// NaN without the FP64 unit
+__device__ __forceinline__ unsigned long long mag_bits(double a) {
+    return (unsigned long long)__double_as_longlong(a) & 0x7fffffffffffffffull;
+}
+
+// complex lines of a k_st_x CTA, and the pitch of a line's exchange
+__host__ __device__ constexpr int st_x_lines(int n1, int n2) { return (n1 > n2 ? n1 : n2) >= 16 ? 8 : 16; }
+__host__ __device__ constexpr int st_x_row(int n1, int n2) { return n1 * (n2 + 1) > n1 * n2 ? n1 * (n2 + 1) + 1 : n1 * n2 + 1; }
+
+// A CTA: RW rows of plane index jr = j0 + blockIdx.y, NLR complex lines a row, each two real
+// signals:  ACC: u + i w, v(centre) + i p, v + i w(face), omega_x;  else: u + i w, v.
+// part[(jr*gridDim.x + blockIdx.x)*NLR*8 + l*8 + q]: of line l, the sums of a, a^2, c, c^2,
+// a * (a of the neighbour line), a*c and the maxima of |a| and |c| (a + i c the line's values;
+// omega_x over the first N1 x N2 points, stats.f90:53-60).  With pc, on the planes of a band (its
+// nbu, nbv, nbp planes from either end): pc[((pl*ngal2 + z)*kStQ + q)*dnx + ti], row z folded
+// onto a tile of dnx points.
+template <int TN1, int TN2, bool ACC>
+__global__ void __launch_bounds__((st_x_lines(TN1, TN2) * (TN1 > TN2 ? TN1 : TN2) + 31) / 32 * 32, 2)
+    k_st_x(Dims d, Geo g, StChunk s, const double2* __restrict__ Hs, const double2* __restrict__ twx, int RW, int lrw,
+           double* __restrict__ part, double* __restrict__ pc, int dnx, int nbu, int nbv, int nbp) {
+    constexpr int N = TN1 * TN2, HX = N / 3, NK = HX + 1, NLR = ACC ? 4 : 2;
+    constexpr int LX = st_x_row(TN1, TN2);
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    __shared__ double red[16][NLR][8];
+    double2* twt = reinterpret_cast<double2*>(smem_raw);
+    double2* ex = twt + N;
+    load_twiddles<double2, TN1, TN2>(twt, twx);
+    const int t = threadIdx.x, B = NLR * RW;
+    const int z0 = blockIdx.x * RW, jr = s.j0 + blockIdx.y;
+    __syncthreads();
+    // ---- inverse N1-point DFTs, thread (line b, column n2)
+    if (t < B * TN2) {
+        const int b = (unsigned)t / TN2, n2 = t - b * TN2;
+        const int l = b & (NLR - 1), z = min(z0 + b / NLR, d.ngal2 - 1);
+        auto P = [&](int f, int j) { return Hs + ((size_t)(s.off[f] + j - s.first[f]) * d.ngal2 + z) * NK; };
+        // a = a0 A0 + a1 A1 + a2 A2, c = c0 C0 + c1 C1
+        const double2* none = P(0, jr);
+        const double2 *A0 = none, *A1 = none, *A2 = none, *C0 = none, *C1 = none;
+        double a0 = 0, a1 = 0, a2 = 0, c0 = 0, c1 = 0;
+        if (l == 0) {
+            A0 = P(0, jr); a0 = 1.0;
+            C0 = P(1, jr); c0 = 1.0;
+        } else if (ACC && l == 1) {  // interp_v with its ghost centres (FOU3D.f90:285-308)
+            int j;
+            if (jr == 0) {
+                j = 1; a0 = (1.0 - g.gwib) * g.vca[1]; a1 = g.gwib + (1.0 - g.gwib) * g.vcb[1];
+            } else if (jr == d.nyu - 1) {
+                j = jr - 1; a0 = g.gwit + (1.0 - g.gwit) * g.vca[j]; a1 = (1.0 - g.gwit) * g.vcb[j];
+            } else {
+                j = jr; a0 = g.vca[jr]; a1 = g.vcb[jr];
+            }
+            A0 = P(2, j); A1 = P(2, j - 1);
+            if (jr < d.nyp) { C0 = P(4, jr); c0 = 1.0; }
+        } else if (jr < d.nyv) {
+            if (!ACC || l == 2) {
+                A0 = P(2, jr); a0 = 1.0;
+                if (ACC) { C0 = P(1, jr + 1); c0 = g.ufa[jr]; C1 = P(1, jr); c1 = g.ufb[jr]; }
+            } else {  // omega_x = dw/dy - dv/dz at the face
+                A0 = P(1, jr + 1); a0 = g.dthdyv[jr];
+                A1 = P(1, jr); a1 = -a0;
+                A2 = P(3, jr); a2 = -1.0;
+            }
+        }
+        const bool ta1 = a1 != 0.0, ta2 = a2 != 0.0, tc0 = c0 != 0.0, tc1 = c1 != 0.0;
+        auto fetch = [&](int k, double2& a, double2& c) {
+            a = dscl(a0, A0[k]);
+            if (ta1) a = dadd(a, dscl(a1, A1[k]));
+            if (ta2) a = dadd(a, dscl(a2, A2[k]));
+            c = tc0 ? dscl(c0, C0[k]) : dc(0, 0);
+            if (tc1) c = dadd(c, dscl(c1, C1[k]));
+        };
+        double2 v[TN1];
+#pragma unroll
+        for (int n1 = 0; n1 < TN1; ++n1) {
+            const int e0 = n1 * TN2, e = e0 + n2;
+            const bool lo = (e0 + TN2 - 1 <= HX) || (e0 <= HX && e <= HX);
+            const bool hi = (e0 >= N - HX) || (e0 + TN2 - 1 >= N - HX && e >= N - HX);
+            double2 val = dc(0, 0), a, c;
+            if (lo) {  // the inverse real transform ignores Im of kx = 0
+                fetch(e, a, c);
+                if (n1 == 0 && n2 == 0) { a.y = 0; c.y = 0; }
+                val = dc(a.x - c.y, a.y + c.x);
+            } else if (hi) {
+                fetch(N - e, a, c);
+                val = dc(a.x + c.y, -a.y + c.x);
+            }
+            v[n1] = val;
+        }
+        rdft_z<TN1, +1, gap_blocks<TN1, TN2, HX>()>(v);
+        double2* o = ex + (size_t)b * LX + n2;
+#pragma unroll
+        for (int k1 = 0; k1 < TN1; ++k1) o[k1 * (TN2 + 1)] = k1 == 0 ? v[0] : cmulc(v[k1], twt[k1 * TN2 + n2]);
+    }
+    __syncthreads();
+    // ---- inverse N2-point DFTs -> x = k1 + N1 k2; the lines of a row in adjacent lanes
+    const bool act = t < B * TN1;
+    const int l = t & (NLR - 1), rest = t / NLR, rr = rest & (RW - 1), k1 = min(rest >> lrw, TN1 - 1);
+    const int b = rr * NLR + l, z = z0 + rr;
+    double2 y[TN2];
+    double q[6] = {0, 0, 0, 0, 0, 0};
+    unsigned long long ma = 0, mc = 0;
+    if ((t & ~31) < B * TN1) {
+        const double2* o = ex + (size_t)b * LX + k1 * (TN2 + 1);
+#pragma unroll
+        for (int n2 = 0; n2 < TN2; ++n2) y[n2] = o[n2];
+        rdft<TN2, +1>(y);
+        const bool in = act && z < d.ngal2;
+#pragma unroll
+        for (int k2 = 0; k2 < TN2; ++k2) {
+            const double a = y[k2].x, c = y[k2].y;
+            const double o2 = ACC ? __shfl_xor_sync(0xffffffffu, a, 1) : 0.0;
+            const bool wx = ACC && l == 3;
+            if (in && (!wx || (k1 + TN1 * k2 < d.n1 && z < d.n2))) {
+                if (ACC) {
+                    q[0] += a; q[1] += a * a; q[2] += c; q[3] += c * c; q[4] += a * o2; q[5] += a * c;
+                }
+                ma = max(ma, mag_bits(a));
+                mc = max(mc, mag_bits(c));
+            }
+        }
+#pragma unroll
+        for (int o2 = NLR; o2 < 32; o2 <<= 1) {
+#pragma unroll
+            for (int k = 0; k < 6; ++k)
+                if (ACC) q[k] += __shfl_xor_sync(0xffffffffu, q[k], o2);
+            ma = max(ma, __shfl_xor_sync(0xffffffffu, ma, o2));
+            mc = max(mc, __shfl_xor_sync(0xffffffffu, mc, o2));
+        }
+    }
+    if ((t & 31) < NLR) {
+        double* o = red[t >> 5][t & 31];
+#pragma unroll
+        for (int k = 0; k < 6; ++k) o[k] = q[k];
+        o[6] = __longlong_as_double((long long)ma);
+        o[7] = __longlong_as_double((long long)mc);
+    }
+    __syncthreads();
+    if (t < NLR * 8) {
+        const int lr = t >> 3, k = t & 7, nw = (blockDim.x + 31) >> 5;
+        double v = red[0][lr][k];
+        for (int w = 1; w < nw; ++w) v = k < 6 ? v + red[w][lr][k] : nan_max(v, red[w][lr][k]);
+        part[((size_t)jr * gridDim.x + blockIdx.x) * NLR * 8 + t] = v;
+    }
+    if constexpr (ACC) {
+        auto band = [&](int ny, int nb) { return jr < ny && (jr < nb || ny - 1 - jr < nb); };
+        if (pc == nullptr || !(band(d.nyu, nbu) || band(d.nyv, nbv) || band(d.nyp, nbp))) return;
+        if (act)  // the exchange has been read: it takes the physical rows
+#pragma unroll
+            for (int k2 = 0; k2 < TN2; ++k2) ex[(size_t)b * LX + k1 + TN1 * k2] = y[k2];
+        __syncthreads();
+        const int ntx = N / dnx;
+        for (int it = t; it < RW * 3 * dnx; it += blockDim.x) {
+            const int ti = it % dnx, gq = (it / dnx) % 3, row = it / (3 * dnx);
+            if (z0 + row >= d.ngal2) break;
+            const double2* L0 = ex + (size_t)(row * 4 + (gq == 1 ? 2 : 0)) * LX + ti;
+            const double2* L1 = L0 + LX;
+            double f[6] = {0, 0, 0, 0, 0, 0};
+            for (int ix = 0; ix < ntx; ++ix) {
+                const double2 m = L0[ix * dnx], n = L1[ix * dnx];
+                if (gq == 0) {  // u + i w, v(centre) + i p
+                    f[0] += m.x; f[1] += m.x * m.x; f[2] += m.y; f[3] += m.y * m.y; f[4] += m.x * n.x; f[5] += m.x * m.y;
+                } else if (gq == 1) {  // v + i w(face), omega_x
+                    f[0] += m.x; f[1] += m.x * m.x; f[2] += n.x; f[3] += n.x * n.x; f[4] += m.x * m.y;
+                } else {
+                    f[0] += n.y; f[1] += n.y * n.y;
+                }
+            }
+            double* o = pc + (((size_t)blockIdx.y * d.ngal2 + z0 + row) * kStQ + (gq == 0 ? 0 : (gq == 1 ? 6 : 11))) * dnx + ti;
+            const int nq = gq == 0 ? 6 : (gq == 1 ? 5 : 2);
+#pragma unroll
+            for (int k = 0; k < 6; ++k)
+                if (k < nq) o[(size_t)k * dnx] = f[k];
+        }
+    }
+}
+
+// ---- plane entry points ---------------------------------------------------------------
+// cft (cft_buff.f:1-65): complex lines of length N in place, element stride ise and line stride isa
+// in doubles, batch stride bstride; inverse (SIGN +1) unscaled, forward x 1/N.  A2: pairs lie on 16
+// bytes.  grid: x = line chunk, y = batch.
+template <int TN1, int TN2, int SIGN, bool A2>
+__global__ void __launch_bounds__(8 * (TN1 > TN2 ? TN1 : TN2), (TN1 > TN2 ? TN1 : TN2) <= 24 ? 3 : 2)
+    k_pl_cft(double* __restrict__ c, int ise, int isa, int m, long long bstride, const double2* __restrict__ tw, int lb) {
+    constexpr int N = TN1 * TN2;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    double2* twt = reinterpret_cast<double2*>(smem_raw);
+    double2* ex = twt + N;
+    load_twiddles<double2, TN1, TN2>(twt, tw);
+    const int l = (blockIdx.x << lb) + (threadIdx.x & ((1 << lb) - 1));
+    const bool live = l < m;
+    double* x = c + (size_t)blockIdx.y * bstride + (size_t)min(l, m - 1) * isa;
+    __syncthreads();
+    auto load = [&](int e, int) -> double2 {
+        double* a = x + (size_t)e * ise;
+        if (A2) return *reinterpret_cast<double2*>(a);
+        return dc(a[0], a[1]);
+    };
+    auto store = [&](int e, int, double2 v) {
+        if (!live) return;
+        double* a = x + (size_t)e * ise;
+        if (SIGN < 0) v = dscl(1.0 / N, v);
+        if (A2) *reinterpret_cast<double2*>(a) = v;
+        else { a[0] = v.x; a[1] = v.y; }
+    };
+    two_step_lines<double2, TN1, TN2, SIGN>(lb, ex, twt, load, store);
+}
+
+// rft (rft_buff.f:24-86): real lines of length N in place, stride isa doubles, two lines 2b and 2b+1
+// a complex transform.  Inverse: x_a + i x_b from the Hermitian extensions of the half spectra (Im
+// of modes 0 and N/2 ignored); forward: x 1/N, Re and Im of modes 0..N/2 with zero Im at both ends.
+// nl transforms a CTA; grid: x = line chunk, y = batch.
+template <int TN1, int TN2, int SIGN, bool A2>
+__global__ void __launch_bounds__((8 * (TN1 > TN2 ? TN1 : TN2) + 31) / 32 * 32)
+    k_pl_rft(double* __restrict__ c, int isa, int m, long long bstride, const double2* __restrict__ tw, int nl) {
+    constexpr int N = TN1 * TN2;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    double2* twt = reinterpret_cast<double2*>(smem_raw);
+    double2* ex = twt + N;
+    load_twiddles<double2, TN1, TN2>(twt, tw);
+    double* base = c + (size_t)blockIdx.y * bstride;
+    const int l0 = blockIdx.x * nl;
+    // (a line past the last repeats it in the transform and is not stored)
+    auto line = [&](int i) { return base + (size_t)min(i, m - 1) * isa; };
+    __syncthreads();
+    if constexpr (SIGN > 0) {
+        auto load = [&](int e, int b) -> double2 {
+            const int k = e <= N / 2 ? e : N - e;
+            const double *xa = line(2 * (l0 + b)) + 2 * k, *xb = line(2 * (l0 + b) + 1) + 2 * k;
+            double2 A, Bv;
+            if (A2) { A = *reinterpret_cast<const double2*>(xa); Bv = *reinterpret_cast<const double2*>(xb); }
+            else { A = dc(xa[0], xa[1]); Bv = dc(xb[0], xb[1]); }
+            if (k == 0 || k == N / 2) { A.y = 0; Bv.y = 0; }
+            if (e > N / 2) { A.y = -A.y; Bv.y = -Bv.y; }
+            return dc(A.x - Bv.y, A.y + Bv.x);
+        };
+        auto store = [&](int x, int b, double2 v) {
+            const int i = 2 * (l0 + b);
+            if (i < m) base[(size_t)i * isa + x] = v.x;
+            if (i + 1 < m) base[(size_t)(i + 1) * isa + x] = v.y;
+        };
+        two_step_lines<double2, TN1, TN2, +1, false>(0, ex, twt, load, store, nl);
+    } else {
+        constexpr int LU = N + 1;
+        double2* ub = ex + (size_t)nl * exch_row<TN1, TN2>();
+        auto load = [&](int x, int b) -> double2 { return dc(line(2 * (l0 + b))[x], line(2 * (l0 + b) + 1)[x]); };
+        auto store = [&](int k, int b, double2 v) { ub[(size_t)b * LU + k] = v; };
+        two_step_lines<double2, TN1, TN2, -1, false>(0, ex, twt, load, store, nl);
+        constexpr int NK = N / 2 + 1;
+        const double hs = 0.5 / N;
+        for (int it = threadIdx.x; it < nl * NK; it += blockDim.x) {
+            const int b = (unsigned)it / NK, k = it - b * NK, i = 2 * (l0 + b);
+            const double2 Pk = ub[(size_t)b * LU + k], Q = ub[(size_t)b * LU + (k == 0 ? 0 : N - k)];
+            const bool edge = k == 0 || k == N / 2;
+            const double2 xa = dc((Pk.x + Q.x) * hs, edge ? 0.0 : (Pk.y - Q.y) * hs);
+            const double2 xb = dc((Pk.y + Q.y) * hs, edge ? 0.0 : (Q.x - Pk.x) * hs);
+            auto put = [&](int r, double2 v) {
+                if (r >= m) return;
+                double* a = base + (size_t)r * isa + 2 * k;
+                if (A2) *reinterpret_cast<double2*>(a) = v;
+                else { a[0] = v.x; a[1] = v.y; }
+            };
+            put(i, xa);
+            put(i + 1, xb);
+        }
+    }
+}
+
+}  // namespace cfd

