@@ -15,6 +15,7 @@
 #include <cstdlib>
 #include <cstring>
 #include <string>
+#include <unordered_map>
 #include <vector>
 
 #include "../../include/cfd_b200.h"
@@ -60,6 +61,12 @@ struct IBDev {
     int nact = 0;
     int* arow = nullptr;
     unsigned char* rowflag = nullptr;
+    // z rows in groups closed under the stencils of their points (ib_rows)
+    int ng = 0;
+    int* grows = nullptr;
+    int* gptr = nullptr;
+    uint4* gpts = nullptr;
+    double* gw = nullptr;
 };
 
 }  // namespace
@@ -106,6 +113,8 @@ struct cfd_ctx {
     double* part = nullptr;
     int npart = 0;
     IBDev ibu, ibv;
+    int RWG = 0;            // rows of a group of the fused forcing pass (0: not used)
+    size_t SMG = 0;
     void* Hib = nullptr;    // IB round-trip planes of the u grid (u, w: 4 fields)
     void* Hib_v = nullptr;  // and of the v grid (2 fields), so the two round trips can overlap
     void* phys_v = nullptr;
@@ -385,6 +394,11 @@ int set_smem_attrs(cfd_ctx* c) {
         set(kn->zfwd2, c->SMZN);
         set(kn->zinv2s_r, c->SMZN);
         set(kn->zfwd2_r, c->SMZN);
+    }
+    if (c->RWG) {
+        set(line_kernels<T2>(n2)->ib_zin, c->SMZ2);
+        set(line_kernels<T2>(n2)->ib_zout, c->SMZ2);
+        set(line_kernels<T2>(n1)->ib_force_x, c->SMG);
     }
     if (c->RWIX2) {
         set(line_kernels<T2>(n1)->ib_xinv, c->SMIX2);
@@ -693,8 +707,41 @@ int ib_grid(cfd_ctx* c, const IBDev& ib, int j0, int nb, double2* rhs_a, double2
 // disjoint fields and buffers, so the v-grid one runs on a side stream forked from and joined
 // back into the context stream (two parallel branches when captured in a graph).  With the
 // per-kernel profiler on they run one after the other on the context stream.
+// The same in three launches (k_ib_zin, k_ib_force_x, k_ib_zout), where the points fall into groups
+// of few rows.
+template <typename T2>
+int ib_groups(cfd_ctx* c) {
+    const Dims& d = c->d;
+    const auto *kz = line_kernels<T2>(d.ngal2), *kx = line_kernels<T2>(d.ngal1);
+    const size_t pl = (size_t)d.ngal2 * d.nkx;
+    const size_t nu = c->ibu.npl * pl, nv = c->ibv.npl * pl;
+    IBJobs a{{{c->du1, c->du1, 0, 0}, {c->du3, c->du3, 0, nu}, {c->du2, c->du2, 1, 2 * nu},
+              {c->u1, nullptr, 0, 2 * nu + nv}, {c->u3, nullptr, 0, 3 * nu + nv}, {c->u2, nullptr, 1, 4 * nu + nv}},
+             {c->ibu.planes, c->ibv.planes}, {c->ibu.rowflag, c->ibv.rowflag}, {c->ibu.npl, c->ibv.npl}, {d.ju0, d.jv0}};
+    // the velocities' inverse z transforms are those of the nonlinear pass when it left them
+    const IBVels vel{c->hx_valid && c->RW2 ? c->Hx : nullptr, {0, d.nyu, 2 * d.nyu}};
+    auto rows = [](const IBDev& b) { return IBRows{b.grows, b.gptr, b.gpts, b.gw, b.ng}; };
+    const int np = std::max(c->ibu.npl, c->ibv.npl), CH = 1 << c->LZ2;
+    const dim3 gz((np * d.nkx + CH - 1) / CH, vel.Hx ? 3 : 6), go(gz.x, 3);
+    prof_mark(c);
+    kz->ib_zin<<<gz, c->NTZ2, c->SMZ2, c->stream>>>(d, a, (T2*)c->Hib, twz<T2>(c), c->LZ2);
+    LK("k_ib_zin");
+    prof_mark(c);
+    const int ng = std::max(c->ibu.ng, c->ibv.ng);
+    if (ng > 0) {
+        kx->ib_force_x<<<dim3(ng, np, 3), (c->RWG * std::max(kx->n1, kx->n2) + 31) / 32 * 32, c->SMG, c->stream>>>(
+            d, a, rows(c->ibu), rows(c->ibv), vel, (T2*)c->Hib, twx<T2>(c), c->RWG);
+        LK("k_ib_force_x");
+        prof_mark(c);
+    }
+    kz->ib_zout<<<go, c->NTZ2, c->SMZ2, c->stream>>>(d, a, (const T2*)c->Hib, twz<T2>(c), c->LZ2);
+    LK("k_ib_zout");
+    return CFD_OK;
+}
+
 template <typename T2>
 int ib_all(cfd_ctx* c) {
+    if (c->RWG) return c->ibu.npl || c->ibv.npl ? ib_groups<T2>(c) : CFD_OK;
     const bool par = c->side && c->ibu.npl > 0 && c->ibv.npl > 0 && !c->profiling;
     if (!par) {
         int s = ib_grid<T2>(c, c->ibu, c->d.ju0, 2, c->du1, c->u1, c->du3, c->u3, c->Hib, c->phys, 0, c->d.nyu);
@@ -983,14 +1030,8 @@ int setup_ib(cfd_ctx* c, const cfd_ib_list* l, int j0, int j1, IBDev& ib, const 
         }
     }
     ib.n = l->n;
-    AL(ib.idx, int, 9 * (size_t)l->n);
-    AL(ib.w, double, 3 * (size_t)l->n);
     AL(ib.planes, int, ib.npl);
     AL(ib.slot_of_j, int, slot.size());
-    if (l->n > 0) {
-        CK(cudaMemcpy(ib.idx, l->idx, 9 * sizeof(int) * (size_t)l->n, cudaMemcpyHostToDevice));
-        CK(cudaMemcpy(ib.w, l->w, 3 * sizeof(double) * (size_t)l->n, cudaMemcpyHostToDevice));
-    }
     if (ib.npl > 0) CK(cudaMemcpy(ib.planes, ib.h_planes.data(), sizeof(int) * ib.npl, cudaMemcpyHostToDevice));
     CK(cudaMemcpy(ib.slot_of_j, slot.data(), sizeof(int) * slot.size(), cudaMemcpyHostToDevice));
     std::vector<unsigned char> flag(ng2, 0);
@@ -1004,6 +1045,108 @@ int setup_ib(cfd_ctx* c, const cfd_ib_list* l, int j0, int j1, IBDev& ib, const 
     AL(ib.rowflag, unsigned char, ng2);
     if (ib.nact > 0) CK(cudaMemcpy(ib.arow, rows.data(), sizeof(int) * ib.nact, cudaMemcpyHostToDevice));
     CK(cudaMemcpy(ib.rowflag, flag.data(), ng2, cudaMemcpyHostToDevice));
+    return CFD_OK;
+}
+
+// Groups of z rows for k_ib_force_x.  Rows that a point ties together (its target and its two
+// stencil rows, in one plane) form a component; components are packed into groups of at most rw
+// rows.  Fails (false) if a point reaches into another plane or a component has more than rw rows.
+bool ib_components(const cfd_ib_list* l, int ng2, std::vector<std::vector<int>>& comp) {
+    std::vector<int> root(ng2), used(ng2, 0);
+    for (int k = 0; k < ng2; ++k) root[k] = k;
+    auto find = [&](int k) {
+        while (root[k] != k) k = root[k] = root[root[k]];
+        return k;
+    };
+    for (int p = 0; p < l->n; ++p) {
+        const int32_t* id = l->idx + 9 * (size_t)p;
+        if (id[5] != id[2] || id[8] != id[2]) return false;
+        if (p > 0 && id[1] == id[1 - 9] && id[4] == id[4 - 9] && id[7] == id[7 - 9]) continue;
+        for (int t = 0; t < 3; ++t) used[id[3 * t + 1] - 1] = 1;
+        for (int t = 1; t < 3; ++t) root[find(id[3 * t + 1] - 1)] = find(id[1] - 1);
+    }
+    std::vector<int> where(ng2, -1);
+    comp.clear();
+    for (int k = 0; k < ng2; ++k) {
+        if (!used[k]) continue;
+        const int r = find(k);
+        if (where[r] < 0) {
+            where[r] = (int)comp.size();
+            comp.emplace_back();
+        }
+        comp[where[r]].push_back(k);
+    }
+    return true;
+}
+
+std::vector<std::vector<int>> ib_pack(const std::vector<std::vector<int>>& comp, int rw) {
+    std::vector<std::vector<int>> g;
+    for (const auto& c : comp) {
+        if ((int)c.size() > rw) return {};
+        if (g.empty() || (int)(g.back().size() + c.size()) > rw) g.emplace_back();
+        g.back().insert(g.back().end(), c.begin(), c.end());
+    }
+    return g;
+}
+
+int ib_rows(cfd_ctx* c, const cfd_ib_list* l, const std::vector<std::vector<int>>& g, int rw, int j0, IBDev& ib) {
+    ib.ng = (int)g.size();
+    const int ng2 = c->d.ngal2, ng = ib.ng;
+    if (!l || ng == 0) return CFD_OK;
+    std::vector<int> rows((size_t)ng * rw, -1), group(ng2, 0), local(ng2, 0), slot(c->d.nyu, 0);
+    for (int q = 0; q < ng; ++q)
+        for (size_t r = 0; r < g[q].size(); ++r) {
+            rows[(size_t)q * rw + r] = g[q][r];
+            group[g[q][r]] = q;
+            local[g[q][r]] = (int)r;
+        }
+    for (int p = 0; p < ib.npl; ++p) slot[ib.h_planes[p] - j0] = p;
+    std::vector<int> bucket(l->n);
+    std::vector<int> ptr((size_t)ib.npl * ng + 1, 0);
+    for (int p = 0; p < l->n; ++p) {
+        const int32_t* id = l->idx + 9 * (size_t)p;
+        bucket[p] = slot[id[2] - j0] * ng + group[id[1] - 1];
+        ptr[bucket[p] + 1]++;
+    }
+    for (size_t k = 1; k < ptr.size(); ++k) ptr[k] += ptr[k - 1];
+    std::vector<uint4> pts(l->n);
+    // the lattices repeat a few triples of weights: looked up in a hash of their bits
+    std::vector<double> w;
+    std::unordered_multimap<uint64_t, unsigned> seen;
+    unsigned last = 0;
+    auto weight = [&](const double* x) -> unsigned {
+        auto same = [&](unsigned q) { return std::memcmp(&w[3 * (size_t)q], x, 3 * sizeof(double)) == 0; };
+        if (!w.empty() && same(last)) return last;
+        uint64_t h = 0, v;
+        for (int k = 0; k < 3; ++k) {
+            std::memcpy(&v, x + k, 8);
+            h = (h ^ v) * 0x9e3779b97f4a7c15ull;
+        }
+        const auto r = seen.equal_range(h);
+        for (auto it = r.first; it != r.second; ++it)
+            if (same(it->second)) return last = it->second;
+        last = (unsigned)(w.size() / 3);
+        w.insert(w.end(), x, x + 3);
+        seen.emplace(h, last);
+        return last;
+    };
+    std::vector<int> at(ptr.begin(), ptr.end() - 1);
+    for (int p = 0; p < l->n; ++p) {  // list order within a bucket: runs of equal targets stay together
+        const int32_t* id = l->idx + 9 * (size_t)p;
+        uint4& o = pts[at[bucket[p]]++];
+        o.x = (unsigned)(id[0] - 1) | (unsigned)(id[3] - 1) << 16;
+        o.y = (unsigned)(id[6] - 1) | (unsigned)local[id[1] - 1] << 16 | (unsigned)local[id[4] - 1] << 24;
+        o.z = (unsigned)local[id[7] - 1];
+        o.w = weight(l->w + 3 * (size_t)p);
+    }
+    AL(ib.grows, int, rows.size());
+    AL(ib.gptr, int, ptr.size());
+    AL(ib.gpts, uint4, pts.size());
+    AL(ib.gw, double, w.size());
+    CK(cudaMemcpy(ib.grows, rows.data(), rows.size() * sizeof(int), cudaMemcpyHostToDevice));
+    CK(cudaMemcpy(ib.gptr, ptr.data(), ptr.size() * sizeof(int), cudaMemcpyHostToDevice));
+    CK(cudaMemcpy(ib.gpts, pts.data(), pts.size() * sizeof(uint4), cudaMemcpyHostToDevice));
+    CK(cudaMemcpy(ib.gw, w.data(), w.size() * sizeof(double), cudaMemcpyHostToDevice));
     return CFD_OK;
 }
 
@@ -1332,14 +1475,51 @@ int create_impl(const cfd_config* cfg, const cfd_ib_list* ibu, const cfd_ib_list
     if ((s = setup_ib(c, ibv, d.jv0, d.jv1, c->ibv, "ibv")) != CFD_OK) return s;
     const size_t nibu = (size_t)4 * c->ibu.npl, nibv = (size_t)2 * c->ibv.npl;
     const size_t hz = (size_t)d.ngal2 * d.nkx, hx = (size_t)d.ngal2 * d.ngal1;
-    if (mixed) {
+    if (c->LZ2 >= 0 && c->RWIX2 && env_int("CFD_IB_GROUPS", 1, 0, 1)) {
+        // rows per group: the even number up to 8 that leaves the fewest lines in all, the larger
+        // of two that leave as many
+        std::vector<std::vector<int>> cu, cv;
+        const auto* kx = line_kernels<float2>(d.ngal1);
+        const int lx = ib_pitch(kx->n1, kx->n2);
+        if ((!ibu || ib_components(ibu, d.ngal2, cu)) && (!ibv || ib_components(ibv, d.ngal2, cv))) {
+            size_t best = 0;
+            for (int rw : {8, 6, 4, 2}) {
+                const auto gu = ib_pack(cu, rw), gv = ib_pack(cv, rw);
+                if ((!cu.empty() && gu.empty()) || (!cv.empty() && gv.empty())) continue;
+                const size_t lines = rw * (2 * gu.size() + gv.size());
+                const size_t sm = ((size_t)rw * lx + d.ngal1) * esz;
+                if (sm > 200 * 1024 || (c->RWG && lines >= best)) continue;
+                best = lines;
+                c->RWG = rw;
+                c->SMG = sm;
+            }
+            if (c->RWG) {
+                if ((s = ib_rows(c, ibu, ib_pack(cu, c->RWG), c->RWG, d.ju0, c->ibu)) != CFD_OK) return s;
+                if ((s = ib_rows(c, ibv, ib_pack(cv, c->RWG), c->RWG, d.jv0, c->ibv)) != CFD_OK) return s;
+                const size_t n = (nibu + nibv) * hz;
+                if (mixed) AL(c->Hib, float2, n); else AL(c->Hib, double2, n);
+                if ((s = mixed ? set_smem_attrs<float2>(c) : set_smem_attrs<double2>(c)) != CFD_OK) return s;
+            }
+        }
+    }
+    if (!c->RWG)  // the lists themselves, for k_ib_force
+        for (auto b : {std::make_pair(ibu, &c->ibu), std::make_pair(ibv, &c->ibv)}) {
+            if (!b.first || b.first->n <= 0) continue;
+            const size_t n = b.first->n;
+            AL(b.second->idx, int, 9 * n);
+            AL(b.second->w, double, 3 * n);
+            CK(cudaMemcpy(b.second->idx, b.first->idx, 9 * n * sizeof(int), cudaMemcpyHostToDevice));
+            CK(cudaMemcpy(b.second->w, b.first->w, 3 * n * sizeof(double), cudaMemcpyHostToDevice));
+        }
+    if (c->RWG) {
+    } else if (mixed) {
         if (nibu) { AL(c->Hib, float2, nibu * hz); AL(c->phys, float, nibu * hx); }
         if (nibv) { AL(c->Hib_v, float2, nibv * hz); AL(c->phys_v, float, nibv * hx); }
     } else {
         if (nibu) { AL(c->Hib, double2, nibu * hz); AL(c->phys, double, nibu * hx); }
         if (nibv) { AL(c->Hib_v, double2, nibv * hz); AL(c->phys_v, double, nibv * hx); }
     }
-    if (nibu && nibv) {
+    if (nibu && nibv && !c->RWG) {
         CK(cudaStreamCreateWithFlags(&c->side, cudaStreamNonBlocking));
         CK(cudaEventCreateWithFlags(&c->ev_fork, cudaEventDisableTiming));
         CK(cudaEventCreateWithFlags(&c->ev_join, cudaEventDisableTiming));

@@ -33,6 +33,10 @@ struct LineKernels {
     void (*ib_xinv)(Dims, const T2*, int, R*, const int*, int, const T2*, int, IBVel);
     void (*ib_xfwd)(Dims, T2*, int, const R*, const int*, int, const T2*, int);
     void (*ib_zfwd)(Dims, const T2*, int, IBDst, int, const int*, const unsigned char*, const T2*, int);
+    // the forcing of u, w and v together
+    void (*ib_zin)(Dims, IBJobs, T2*, const T2*, int);
+    void (*ib_force_x)(Dims, IBJobs, IBRows, IBRows, IBVels, T2*, const T2*, int);
+    void (*ib_zout)(Dims, IBJobs, const T2*, const T2*, int);
     // FP64 only (field_lines.cuh): statistics (sums, or the maxima alone), plane transforms
     // [inverse, forward][8-byte, 16-byte aligned]
     void (*st_z)(Dims, Geo, StChunk, const double2*, const double2*, const double2*, const double2*, double2*,
@@ -95,6 +99,9 @@ const LineKernels<T2>* line_table() {
             t.ib_xinv = k_ib_xinv2<T2, N1, N2>;
             t.ib_xfwd = k_ib_xfwd2<T2, N1, N2>;
             t.ib_zfwd = k_ib_zfwd2<T2, N1, N2>;
+            t.ib_zin = k_ib_zin<T2, N1, N2>;
+            t.ib_force_x = k_ib_force_x<T2, N1, N2>;
+            t.ib_zout = k_ib_zout<T2, N1, N2>;
         }
         if constexpr (WHAT != kLinesAlt && !F32) {
             t.st_z = k_st_z<N1, N2>;

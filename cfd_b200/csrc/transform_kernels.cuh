@@ -1364,4 +1364,247 @@ __global__ void __launch_bounds__(16 * (TN1 > TN2 ? TN1 : TN2), (sizeof(T2) == 8
     two_step_lines<T2, TN1, TN2, -1>(lb, ex, twt, load, store);
 }
 
+// --------------------------------------------------------------------------------------
+// The forcing in three launches for all of u, w, v: inverse z transforms, one pass over groups of z
+// rows that transforms them in x, forces them and transforms them back, forward z transforms.  A
+// group is a set of rows that hold every stencil point of their own forcing points (ib_rows in
+// cfd_capi.cu), so the physical values of a group live in shared memory only.
+// --------------------------------------------------------------------------------------
+struct IBJobs {
+    struct {
+        const double2* src;  // field of the z pass
+        double2* dst;        // where the forward pass writes (right-hand sides)
+        int grid;            // 0: u grid, 1: v grid
+        size_t off;          // its planes in Hib
+    } j[6];                  // right-hand sides u, w, v, then velocities u, w, v
+    const int* planes[2];
+    const unsigned char* rowflag[2];
+    int npl[2], j0[2];
+};
+struct IBRows {
+    const int* rows;    // [ng][RW] z rows of a group, -1 past its last
+    const int* ptr;     // [npl*ng + 1] forcing points of (plane, group)
+    const uint4* pts;   // x: i, i2; y: i3, row, row 2; z: row 3 (of the group); w: weights
+    const double* w;    // [..][3] Lap, w2, w3
+    int ng;
+};
+// velocities of job k (rhs order): plane of the nonlinear pass's transforms, or the job's own planes
+struct IBVels {
+    const void* Hx;
+    int voff[3];
+};
+
+template <typename T2, int TN1, int TN2>
+__global__ void __launch_bounds__(16 * (TN1 > TN2 ? TN1 : TN2), (sizeof(T2) == 8 && (TN1 > TN2 ? TN1 : TN2) <= 24) ? 3 : 1)
+    k_ib_zin(Dims d, IBJobs a, T2* __restrict__ Hib, const T2* __restrict__ twz, int lb) {
+    using R = decltype(T2::x);
+    constexpr int N = TN1 * TN2;
+    const auto& jb = a.j[blockIdx.y];
+    const int nlines = a.npl[jb.grid] * d.nkx, line0 = blockIdx.x << lb;
+    if (line0 >= nlines) return;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    T2* twt = reinterpret_cast<T2*>(smem_raw);
+    T2* ex = twt + N;
+    load_twiddles<T2, TN1, TN2>(twt, twz);
+    const int b = threadIdx.x & ((1 << lb) - 1);
+    const bool live = line0 + b < nlines;
+    const int line = live ? line0 + b : nlines - 1;
+    const int p = line / d.nkx, i = line - p * d.nkx;
+    const double2* f = jb.src + (size_t)(a.planes[jb.grid][p] - a.j0[jb.grid]) * d.ncol + i;
+    T2* H = Hib + jb.off + (size_t)p * N * d.nkx + i;
+    const int r = threadIdx.x >> lb;
+    __syncthreads();
+    auto load = [&](int e, int) -> T2 {
+        const int q = zrow_q<N, TN2>(e, r);
+        return q >= 0 ? to_t2<T2>(f[(size_t)q * d.nkx]) : cx<T2>((R)0, (R)0);
+    };
+    auto store = [&](int z, int, T2 v) {
+        if (live) H[(size_t)z * d.nkx] = v;
+    };
+    two_step_lines<T2, TN1, TN2, +1>(lb, ex, twt, load, store);
+}
+
+template <typename T2, int TN1, int TN2>
+__global__ void __launch_bounds__(16 * (TN1 > TN2 ? TN1 : TN2), (sizeof(T2) == 8 && (TN1 > TN2 ? TN1 : TN2) <= 24) ? 3 : 1)
+    k_ib_zout(Dims d, IBJobs a, const T2* __restrict__ Hib, const T2* __restrict__ twz, int lb) {
+    using R = decltype(T2::x);
+    constexpr int N = TN1 * TN2;
+    const auto& jb = a.j[blockIdx.y];
+    const int nlines = a.npl[jb.grid] * d.nkx, line0 = blockIdx.x << lb;
+    if (line0 >= nlines) return;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    T2* twt = reinterpret_cast<T2*>(smem_raw);
+    T2* ex = twt + N;
+    load_twiddles<T2, TN1, TN2>(twt, twz);
+    const int b = threadIdx.x & ((1 << lb) - 1);
+    const bool live = line0 + b < nlines;
+    const int line = live ? line0 + b : nlines - 1;
+    const int p = line / d.nkx, i = line - p * d.nkx;
+    const T2* H = Hib + jb.off + (size_t)p * N * d.nkx + i;
+    double2* out = jb.dst + (size_t)(a.planes[jb.grid][p] - a.j0[jb.grid]) * d.ncol + i;
+    const unsigned char* rowflag = a.rowflag[jb.grid];
+    const int r = threadIdx.x >> lb;
+    const R sc = (R)1 / (R)N;
+    const bool first = i == 0;
+    __syncthreads();
+    // rows no group holds still lose Im of kx = 0, which the inverse real transform ignores
+    // (rft_buff.f:78-80)
+    auto load = [&](int z, int) -> T2 {
+        T2 v = H[(size_t)z * d.nkx];
+        if (first && !rowflag[z]) v.y = (R)0;
+        return v;
+    };
+    auto store = [&](int e, int, T2 v) {
+        const int q = zrow_q<N, TN1>(e, r);
+        if (q >= 0 && live) out[(size_t)q * d.nkx] = to_d2(cscale(v, sc));
+    };
+    two_step_lines<T2, TN1, TN2, -1>(lb, ex, twt, load, store);
+}
+
+// pitch of a line of k_ib_force_x: exchange, physical row or spectrum
+__host__ __device__ constexpr int ib_pitch(int n1, int n2) { return (n1 * (n2 + 1) > n2 * (n1 + 1) ? n1 * (n2 + 1) : n2 * (n1 + 1)) | 1; }
+
+// grid: x = group, y = plane, z = right-hand side (u, w, v).  RW lines, RW even, at most 8.
+// Against the four launches it stands for on either grid (inverse x of right-hand sides and
+// velocities to memory, forcing, forward x), microseconds a substep with their z passes on B200: 384 x
+// 257(+90) x 384 FP32 285 -> 178, FP64 549 -> 317; 64 x 97(+56) x 64 FP64 31 -> 15 and ten launches to
+// three.
+template <typename T2, int TN1, int TN2>
+__global__ void __launch_bounds__(((sizeof(T2) == 8 ? 16 : 8) * (TN1 > TN2 ? TN1 : TN2) + 31) / 32 * 32, sizeof(T2) == 8 ? 0 : ((TN1 > TN2 ? TN1 : TN2) <= 24 ? 3 : 2))
+    k_ib_force_x(Dims d, IBJobs a, IBRows gu, IBRows gv, IBVels vel, T2* __restrict__ Hib, const T2* __restrict__ twx, int RW) {
+    using R = decltype(T2::x);
+    constexpr int N = TN1 * TN2, HX = N / 3, NK = HX + 1, LX = ib_pitch(TN1, TN2);
+    const auto& jb = a.j[blockIdx.z];
+    const IBRows& G = jb.grid ? gv : gu;
+    const int p = blockIdx.y;
+    if (p >= a.npl[jb.grid] || (int)blockIdx.x >= G.ng) return;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    T2* twt = reinterpret_cast<T2*>(smem_raw);
+    T2* ex = twt + N;
+    load_twiddles<T2, TN1, TN2>(twt, twx);
+    const int* rows = G.rows + (size_t)blockIdx.x * RW;
+    const size_t pl = (size_t)d.ngal2 * NK;
+    T2* Hr = Hib + jb.off + p * pl;
+    const T2* Hu = vel.Hx ? (const T2*)vel.Hx + (size_t)(vel.voff[blockIdx.z] + a.planes[jb.grid][p] - a.j0[jb.grid]) * pl
+                          : Hib + a.j[3 + blockIdx.z].off + p * pl;
+    const int t = threadIdx.x;
+    __syncthreads();
+    // ---- inverse: line b = rhs + i u of row b
+    if (t < RW * TN2) {
+        const int b = t / TN2, n2 = t - b * TN2;
+        const int row = rows[b];
+        const T2 *A = Hr + (size_t)max(row, 0) * NK, *C = Hu + (size_t)max(row, 0) * NK;
+        T2 v[TN1];
+#pragma unroll
+        for (int n1 = 0; n1 < TN1; ++n1) {
+            const int e0 = n1 * TN2, e = e0 + n2;
+            const bool lo = (e0 + TN2 - 1 <= HX) || (e0 <= HX && e <= HX);
+            const bool hi = (e0 >= N - HX) || (e0 + TN2 - 1 >= N - HX && e >= N - HX);
+            T2 val = cx<T2>((R)0, (R)0);
+            if (lo) {
+                T2 x = A[e], c = C[e];
+                if (n1 == 0 && n2 == 0) { x.y = 0; c.y = 0; }
+                val = cx<T2>(x.x - c.y, x.y + c.x);
+            } else if (hi) {
+                const T2 x = A[N - e], c = C[N - e];
+                val = cx<T2>(x.x + c.y, -x.y + c.x);
+            }
+            v[n1] = val;
+        }
+        rdft_z<TN1, +1, gap_blocks<TN1, TN2, HX>()>(v);
+        T2* o = ex + (size_t)b * LX + n2;
+#pragma unroll
+        for (int k1 = 0; k1 < TN1; ++k1) o[k1 * (TN2 + 1)] = k1 == 0 ? v[0] : cmulc(v[k1], twt[k1 * TN2 + n2]);
+    }
+    __syncthreads();
+    {
+        const bool act = t < RW * TN1;
+        const int b = t / TN1, k1 = t - b * TN1;
+        T2 y[TN2];
+        if (act) {
+            const T2* o = ex + (size_t)b * LX + k1 * (TN2 + 1);
+#pragma unroll
+            for (int n2 = 0; n2 < TN2; ++n2) y[n2] = o[n2];
+            rdft<TN2, +1>(y);
+        }
+        __syncthreads();
+        if (act)
+#pragma unroll
+            for (int k2 = 0; k2 < TN2; ++k2) ex[(size_t)b * LX + k1 + TN1 * k2] = y[k2];
+    }
+    __syncthreads();
+    // ---- point forcing rhs(p) = Lap*(w2 u(p2) + w3 u(p3) - u(p) + rhs(p))
+    // (tridLU_3D_IB.f90:193-211); the first point of a run of equal targets applies the run in
+    // list order, as k_ib_force does
+    {
+        const int e0 = G.ptr[p * G.ng + blockIdx.x], e1 = G.ptr[p * G.ng + blockIdx.x + 1];
+        for (int e = e0 + t; e < e1; e += blockDim.x) {
+            uint4 q = G.pts[e];
+            const unsigned ti = q.x & 0xffff, tr = (q.y >> 16) & 0xff;
+            if (e > e0) {
+                const uint4 pv = G.pts[e - 1];
+                if ((pv.x & 0xffff) == ti && ((pv.y >> 16) & 0xff) == tr) continue;
+            }
+            T2* tgt = ex + (size_t)tr * LX + ti;
+            R r = tgt->x;
+            const R u0 = tgt->y;
+            for (int f = e;;) {
+                const double* w = G.w + 3 * (size_t)q.w;
+                const R vf = (R)w[1] * ex[(size_t)(q.y >> 24) * LX + (q.x >> 16)].y + (R)w[2] * ex[(size_t)q.z * LX + (q.y & 0xffff)].y;
+                r = (R)w[0] * (vf - u0 + r);
+                if (++f == e1) break;
+                q = G.pts[f];
+                if ((q.x & 0xffff) != ti || ((q.y >> 16) & 0xff) != tr) break;
+            }
+            tgt->x = r;
+        }
+    }
+    __syncthreads();
+    // ---- forward: line m packs rows 2m and 2m + 1
+    const int nl = RW / 2;
+    {
+        const bool act = t < nl * TN2;
+        const int m = t / TN2, n2 = t - m * TN2;
+        T2 v[TN1];
+        if (act) {
+            const T2 *x0 = ex + (size_t)(2 * m) * LX + n2, *x1 = x0 + LX;
+#pragma unroll
+            for (int n1 = 0; n1 < TN1; ++n1) v[n1] = cx<T2>(x0[n1 * TN2].x, x1[n1 * TN2].x);
+            rdft<TN1, -1>(v);
+        }
+        __syncthreads();
+        if (act) {
+            T2* o = ex + (size_t)m * LX + n2;
+#pragma unroll
+            for (int k1 = 0; k1 < TN1; ++k1) o[k1 * (TN2 + 1)] = k1 == 0 ? v[0] : cmul(v[k1], twt[k1 * TN2 + n2]);
+        }
+    }
+    __syncthreads();
+    {
+        const bool act = t < nl * TN1;
+        const int m = t / TN1, k1 = t - m * TN1;
+        T2 y[TN2];
+        if (act) {
+            const T2* o = ex + (size_t)m * LX + k1 * (TN2 + 1);
+#pragma unroll
+            for (int n2 = 0; n2 < TN2; ++n2) y[n2] = o[n2];
+            rdft<TN2, -1>(y);
+        }
+        __syncthreads();
+        if (act)
+#pragma unroll
+            for (int k2 = 0; k2 < TN2; ++k2) ex[(size_t)m * LX + k1 + TN1 * k2] = y[k2];
+    }
+    __syncthreads();
+    const R hs = (R)0.5 / (R)N;
+    for (int it = t; it < nl * NK; it += blockDim.x) {
+        const int m = (unsigned)it / NK, k = it - m * NK;
+        const T2* L = ex + (size_t)m * LX;
+        const T2 Pk = L[k], Qc = cconj(L[k == 0 ? 0 : N - k]);
+        const int ra = rows[2 * m], rb = rows[2 * m + 1];
+        if (ra >= 0) Hr[(size_t)ra * NK + k] = cx<T2>((Pk.x + Qc.x) * hs, (Pk.y + Qc.y) * hs);
+        if (rb >= 0) Hr[(size_t)rb * NK + k] = cx<T2>((Pk.y - Qc.y) * hs, -(Pk.x - Qc.x) * hs);
+    }
+}
+
 }  // namespace cfd
