@@ -140,6 +140,7 @@ struct cfd_ctx {
     // three bands: the launch dimensions of the nonlinear pass over the bottom wall band,
     // the middle band and the top wall band; the middle band's transforms
     bool mb = false;
+    int RWB[2] = {0, 0};    // rows per CTA of k_xline2b in the wall bands and the middle band
     Dims dB{}, dM{}, dT{};
     FFTDesc fxm{};
     double2 *twxm_d = nullptr, *twzm_d = nullptr;
@@ -315,20 +316,13 @@ void line_split(int n, int& n1, int& n2, bool alt = false) {
     n1 = k ? k->n1 : 0;
     n2 = k ? k->n2 : 0;
 }
+// lengths with the FP32 x-line pass marching in y
+bool line_march_f32(int n) {
+    const auto* k = line_kernels<float2>(n);
+    return k && k->xmarch;
+}
 // lengths a z plane of a three-band channel can have
 bool band_length(int n) { return n == 64 || n == 96 || n == 128 || n == 192 || n == 384 || n == 768; }
-
-// Splits of the marching x-line kernel (x-line path 6): its second step holds N2 = 8 or 16
-// points per lane, so that the unpack partners kb and N2 - kb share a warp
-#define MARCH_SWITCH(n, ok, ...)                                             \
-    switch (n) {                                                             \
-        case 64: { constexpr int TN1 = 8, TN2 = 8; __VA_ARGS__; } break;     \
-        case 96: { constexpr int TN1 = 12, TN2 = 8; __VA_ARGS__; } break;    \
-        case 128: { constexpr int TN1 = 8, TN2 = 16; __VA_ARGS__; } break;   \
-        case 192: { constexpr int TN1 = 12, TN2 = 16; __VA_ARGS__; } break;  \
-        case 384: { constexpr int TN1 = 24, TN2 = 16; __VA_ARGS__; } break;  \
-        default: ok = false; break;                                          \
-    }
 
 // shared memory of k_xline2 (elements): B*LX + N
 // Launch-shape overrides (unset: the built-in choice; a cfd_tuning field takes precedence).
@@ -409,17 +403,22 @@ int set_smem_attrs(cfd_ctx* c) {
         if (c->XR64) set(line_kernels<T2>(n1, c->XALT)->xline2_r, c->SM2);
         if (c->XL3) set(line_kernels<T2>(n1)->xline3, c->SM3);
         if (c->RW4) set(line_kernels<T2>(n1)->xline4, c->SM4);
-        if constexpr (std::is_same<T2, float2>::value)
-            if (c->XMRW) {
-                bool ok = true;
-                MARCH_SWITCH(n1, ok, set(k_xmarch<float2, TN1, TN2>, c->SMXM););
-            }
+        if (c->XMRW) set(line_kernels<T2>(n1)->xmarch, c->SMXM);
     }
     if (c->mb && c->LZ2 >= 0) {
         const auto* k = line_kernels<T2>(c->dM.ngal2);
         const size_t smz = std::max(c->SMZ2, c->SMZm);
         set(k->zinv2, smz);
         set(k->zfwd2, smz);
+        const int nx[2] = {n1, c->dM.ngal1};
+        size_t smb = 0;  // (equal lengths share a kernel)
+        for (int m = 0; m < 2; ++m)
+            if (const auto* kb = line_kernels<T2>(nx[m])) {
+                c->RWB[m] = 4;
+                while (c->RWB[m] > 1 && xline2_smem(kb->n1, kb->n2, c->RWB[m], esz) > 110 * 1024) c->RWB[m] /= 2;
+                smb = std::max(nx[0] == nx[1] ? smb : 0, xline2_smem(kb->n1, kb->n2, c->RWB[m], esz));
+                set(kb->xline2b, smb);
+            }
         FFT_SWITCH(c->dM.ngal1, {
             if (e == cudaSuccess) e = cudaFuncSetAttribute(k_xline<T2, NF>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sx);
         });
@@ -478,6 +477,13 @@ int nl_transforms_mb(cfd_ctx* c) {
     for (const Dims* bp : bands) {
         const Dims& d = *bp;
         const bool mid = bp == &c->dM;
+        if (const auto* k = line_kernels<T2>(d.ngal1)) {
+            const int rw = c->RWB[mid];
+            k->xline2b<<<dim3((d.ngal2 + rw - 1) / rw, d.nsu + d.nsv), (2 * rw * std::max(k->n1, k->n2) + 31) / 32 * 32,
+                         xline2_smem(k->n1, k->n2, rw, e), c->stream>>>(
+                d, c->g, (T2*)c->H[0], (T2*)c->H[1], (T2*)c->H[2], (T2*)c->H[3], twx_b(mid), rw, ilog2(rw));
+            continue;
+        }
         dim3 gx(d.ngal2 / c->RWx, d.nsu + d.nsv);
         FFT_SWITCH(d.ngal1, {
             k_xline<T2, NF><<<gx, 256, (size_t)(2 * (2 * c->RWx) * d.ngal1 + d.ngal1) * e, c->stream>>>(
@@ -540,18 +546,13 @@ int nl_transforms(cfd_ctx* c) {
         LK("k_xline4");
         xdone = true;
     }
-    if constexpr (std::is_same<T2, float2>::value) {
-        if (!xdone && c->XMRW) {
-            dim3 gxm(d.ngal2 / c->XMRW, (d.nyu - 1 + c->XMC - 1) / c->XMC);
-            bool ok = true;
-            MARCH_SWITCH(d.ngal1, ok, {
-                k_xmarch<float2, TN1, TN2><<<gxm, c->NTXM, c->SMXM, c->stream>>>(
-                    d, c->g, (const float2*)c->Hx, (float2*)c->H[0], (float2*)c->H[1], (float2*)c->H[2],
-                    (float2*)c->H[3], twx<float2>(c), c->XMRW, c->XMC);
-            });
-            LK("k_xmarch");
-            xdone = true;
-        }
+    if (!xdone && c->XMRW) {
+        dim3 gxm(d.ngal2 / c->XMRW, (d.nyu - 1 + c->XMC - 1) / c->XMC);
+        line_kernels<T2>(d.ngal1)->xmarch<<<gxm, c->NTXM, c->SMXM, c->stream>>>(
+            d, c->g, (const T2*)c->Hx, (T2*)c->H[0], (T2*)c->H[1], (T2*)c->H[2], (T2*)c->H[3], twx<T2>(c), c->XMRW,
+            c->XMC);
+        LK("k_xmarch");
+        xdone = true;
     }
     if (xdone) {
     } else if (c->RW2 && c->XL3) {
@@ -1288,15 +1289,22 @@ int create_impl(const cfd_config* cfg, const cfd_ib_list* ibu, const cfd_ib_list
         c->RWibf /= 2;
     if (d.ngal2 % c->RWibf) return fail(c, CFD_ERR_SIZE, "Ngal2 must be even");
     // the transposed split of the x-line transform (tuning xsplit = 2) is for path 1 only
-    const int xpath = g_tuning && g_tuning->xline_path ? g_tuning->xline_path : env_int("CFD_XLINE_PATH", (mixed && d.ngal1 == 384) ? 6 : 1, 1, 6);
+    const int xpath = g_tuning && g_tuning->xline_path ? g_tuning->xline_path : env_int("CFD_XLINE_PATH", mixed && d.ngal1 >= 256 && line_march_f32(d.ngal1) ? 6 : (mixed && d.ngal1 == 192 ? 5 : 1), 1, 6);
     // (the tuning variants exist for the six named lengths; the others run path 1)
     const bool named = line_kernels_named<float2>(d.ngal1) != nullptr;
-    const bool xalt = named && (xpath == 1 || xpath == 5) && tune_int(&cfd_tuning::xsplit, "CFD_XSPLIT", 1, 1, 2) == 2;
+    // (at 768 points the transposed splits are the default: FP32 x lines 24 * 32 in 8 rows 736 us
+    // against 818 for 32 * 24 in 4, z lines 166 + 298 against 200 + 331 FP32, 326 + 627 in 4 lines
+    // against 361 + 811 FP64, at
+    // 768 x 65 x 768; at 192 points too: a step of 192 x 193(+90) x 192 2.36 -> 2.24 ms FP64, of 192 x
+    // 161(+76) x 192 1.34 -> 1.25 ms FP32 with the 64-register x-line)
+    const bool x768 = d.ngal1 == 768 && mixed, z768 = d.ngal2 == 768;
+    const bool xalt = named && (xpath == 1 || xpath == 5) &&
+                      tune_int(&cfd_tuning::xsplit, "CFD_XSPLIT", x768 || d.ngal1 == 192 ? 2 : 1, 1, 2) == 2;
     {
         int n1s = 0, n2s = 0;
         line_split(d.ngal1, n1s, n2s, xalt);
         if (n1s) {
-            int rw = tune_int(&cfd_tuning::xline_rows, "CFD_XLINE_ROWS", 4, 2, 8);
+            int rw = tune_int(&cfd_tuning::xline_rows, "CFD_XLINE_ROWS", x768 ? 8 : 4, 2, 8);
             rw = 1 << (31 - __builtin_clz(rw));  // a power of two
             while (rw >= 2 && ((named && d.ngal2 % rw) || xline2_smem(n1s, n2s, rw, esz) > budget)) rw /= 2;
             if (rw >= 2) {
@@ -1337,7 +1345,7 @@ int create_impl(const cfd_config* cfg, const cfd_ib_list* ibu, const cfd_ib_list
         line_split(d.ngal2, n1s, n2s);
         if (n1s) {
             const int zl = g_tuning && (g_tuning->zlines == 4 || g_tuning->zlines == 8 || g_tuning->zlines == 16) ? g_tuning->zlines : 0;
-            const int lb = zl ? ilog2(zl) : env_int("CFD_ZLINES_LOG2", mixed ? 4 : 3, 2, 4);
+            const int lb = zl ? ilog2(zl) : env_int("CFD_ZLINES_LOG2", z768 ? (mixed ? 3 : 2) : (mixed ? 4 : 3), 2, 4);
             c->LZ2 = lb;
             c->NTZ2 = (1 << lb) * std::max(n1s, n2s);
             c->SMZ2 = ((size_t)(1 << lb) * ((n1s * (n2s + 1)) | 1) + (size_t)n1s * n2s) * esz;
@@ -1349,19 +1357,28 @@ int create_impl(const cfd_config* cfg, const cfd_ib_list* ibu, const cfd_ib_list
     if (!c->RW2) c->RW4 = 0;
     c->XALT = c->RW2 && xalt;  // (xalt implies path 1: neither k_xline3 nor k_xline4)
     c->XR64 = c->RW2 && !c->XL3 && !c->RW4 && mixed && named && xpath == 5;
-    // the x-line pass marching in y (FP32-mixed, one band; the default for 384-point x lines,
-    // where it measured 0.607 against 0.811 ms per launch; at 64 and 192 points the per-slot
-    // kernels were faster; FP64 contexts and lengths without its split run path 1): rows per
-    // CTA from xline_rows (2 or 4); emission steps per CTA from CFD_XMARCH_STEPS, by default
-    // the longest chunk that keeps 20 CTAs per SM (re550: 16 steps, 0.621 ms per launch
-    // against 0.625-0.636 at 8, 12, 20 and 0.65 at 32; re395: 8 steps)
-    if (c->RW2 && mixed && xpath == 6 && !c->mb && d.nyu >= 4) {
-        bool ok = true;
+    // the x-line pass marching in y (one band).  FP32-mixed: x-line path 6, the default from 256 to 576
+    // points where the length has an 8- or 16-point second step, microseconds a launch against the
+    // per-slot kernels: 256 x 193 x 256 197 and 217, 288 225 and 308, 384 x 257 470 and 637, 432 x 193 492
+    // and 667, 512 772 and 996, 576 899 and 1084; 128 x 129 62 and 46.  FP64: path 1 takes it from 256 to
+    // 512 points: 256 332 and 345, 288 463 and 562, 384 x 257 947 and 1124, 432 1062 and 1273, 512 x 97 841
+    // and 1153; 192 x 193 230 and 232, 128 99 and 82.  Rows per CTA from xline_rows (2 or 4; FP64 2);
+    // emission steps per CTA from CFD_XMARCH_STEPS, by default the longest chunk that keeps 20 CTAs
+    // per SM (re550: 16 steps, 0.621 ms per launch against 0.625-0.636 at 8, 12, 20 and 0.65 at 32;
+    // re395: 8 steps)
+    const bool march = mixed ? xpath == 6 : (xpath == 1 || xpath == 6) && !xalt && env_int("CFD_MARCH", 1, 0, 1);
+    if (c->RW2 && march && !c->mb && d.nyu >= 4) {
         int n1s = 0, n2s = 0;
-        MARCH_SWITCH(d.ngal1, ok, { n1s = TN1; n2s = TN2; });
-        if (ok) {
-            int rw = tune_int(&cfd_tuning::xline_rows, "CFD_XLINE_ROWS", 2, 2, 8) >= 4 ? 4 : 2;
-            auto smx = [&](int r) { return (size_t)xmarch_smem_elems(n1s, n2s, r) * sizeof(float2); };
+        if (mixed) {
+            const auto* k = line_kernels<float2>(d.ngal1);
+            n1s = k->m1; n2s = k->m2;
+        } else {
+            const auto* k = line_kernels<double2>(d.ngal1);
+            n1s = k->m1; n2s = k->m2;
+        }
+        if (n1s) {
+            int rw = mixed && tune_int(&cfd_tuning::xline_rows, "CFD_XLINE_ROWS", 2, 2, 8) >= 4 ? 4 : 2;
+            auto smx = [&](int r) { return (size_t)xmarch_smem_elems(n1s, n2s, r, mixed) * esz; };
             if (rw == 4 && (d.ngal2 % 4 || smx(4) > budget)) rw = 2;
             if (d.ngal2 % rw == 0 && smx(rw) <= budget) {
                 c->XMRW = rw;
@@ -1379,7 +1396,7 @@ int create_impl(const cfd_config* cfg, const cfd_ib_list* ibu, const cfd_ib_list
     // FP64 z kernels at 112 registers (3 CTAs of 8 lines per SM): measured 0.31 / 0.59 against
     // 0.34 / 0.61 ms per launch at re550; the 768-point split spills at that cap
     c->ZR = c->RW2 && c->precision == CFD_PREC_FP64 && d.ngal2 <= 384 && env_int("CFD_Z_R112", 1, 0, 1);
-    if (c->RW2 && c->LZ2 >= 0 && tune_int(&cfd_tuning::zsplit, "CFD_ZSPLIT", 1, 1, 2) == 2) {
+    if (c->RW2 && c->LZ2 >= 0 && tune_int(&cfd_tuning::zsplit, "CFD_ZSPLIT", z768 || d.ngal2 == 192 ? 2 : 1, 1, 2) == 2) {
         int n1s = 0, n2s = 0;
         line_split(d.ngal2, n1s, n2s, true);
         if (n1s) {
@@ -1806,8 +1823,8 @@ int cfd_create_tuned(const cfd_config* cfg, const cfd_ib_list* ibu, const cfd_ib
 
 int cfd_get_tuning(const cfd_ctx* c, cfd_tuning* t) {
     if (!c || !t) return CFD_ERR_ARG;
-    t->xline_path = c->RW2 ? (c->XMRW ? 6 : (c->RW4 ? 4 : (c->XL3 ? 3 : (c->XR64 ? 5 : 1)))) : 2;
-    t->xline_rows = c->XMRW ? c->XMRW : (c->RW4 ? c->RW4 : (c->RW2 ? c->RW2 : 0));
+    t->xline_path = c->RW2 ? (c->XMRW && c->precision == CFD_PREC_MIXED ? 6 : (c->RW4 ? 4 : (c->XL3 ? 3 : (c->XR64 ? 5 : 1)))) : 2;
+    t->xline_rows = c->XMRW && c->precision == CFD_PREC_MIXED ? c->XMRW : (c->RW4 ? c->RW4 : (c->RW2 ? c->RW2 : 0));
     t->zlines = c->LZ2 >= 0 ? (1 << c->LZ2) : 0;
     t->solve_kind = 1;
     t->solve_cols = c->SNT;

@@ -11,6 +11,7 @@
 #pragma once
 
 #include "field_lines.cuh"
+#include "xmarch.cuh"
 
 namespace cfd {
 
@@ -29,6 +30,11 @@ struct LineKernels {
     void (*xline2_r)(Dims, Geo, const T2*, T2*, T2*, T2*, T2*, const T2*, int, int);
     void (*xline3)(Dims, Geo, const T2*, T2*, T2*, T2*, T2*, const T2*, int);
     void (*xline4)(Dims, Geo, const T2*, T2*, T2*, T2*, T2*, const T2*, int);
+    // three bands: the x-line pass on planes interpolated already
+    void (*xline2b)(Dims, Geo, T2*, T2*, T2*, T2*, const T2*, int, int);
+    // the x-line pass marching in y, with a split of its own (null where it has none)
+    void (*xmarch)(Dims, Geo, const T2*, T2*, T2*, T2*, T2*, const T2*, int, int);
+    int m1, m2;
     void (*ib_zinv)(Dims, IBSrc, int, const int*, int, T2*, const T2*, int, int);
     void (*ib_xinv)(Dims, const T2*, int, R*, const int*, int, const T2*, int, IBVel);
     void (*ib_xfwd)(Dims, T2*, int, const R*, const int*, int, const T2*, int);
@@ -72,6 +78,25 @@ template <> const LineKernels<double2>* line_kernels_large2<double2>(int n);
 template <> const LineKernels<float2>* line_kernels<float2>(int n, bool alt);
 template <> const LineKernels<double2>* line_kernels<double2>(int n, bool alt);
 
+// Splits of the marching x-line pass: its second step holds 8 or 16 points per lane, so that the
+// unpack partners kb and N2 - kb share a warp
+template <int N> struct MarchSplit { static constexpr int N1 = 0, N2 = 0; };
+template <> struct MarchSplit<64> { static constexpr int N1 = 8, N2 = 8; };
+template <> struct MarchSplit<96> { static constexpr int N1 = 12, N2 = 8; };
+template <> struct MarchSplit<128> { static constexpr int N1 = 8, N2 = 16; };
+template <> struct MarchSplit<192> { static constexpr int N1 = 12, N2 = 16; };
+template <> struct MarchSplit<256> { static constexpr int N1 = 16, N2 = 16; };
+template <> struct MarchSplit<288> { static constexpr int N1 = 18, N2 = 16; };
+template <> struct MarchSplit<384> { static constexpr int N1 = 24, N2 = 16; };
+template <> struct MarchSplit<432> { static constexpr int N1 = 27, N2 = 16; };
+template <> struct MarchSplit<576> { static constexpr int N1 = 36, N2 = 16; };
+template <> struct MarchSplit<512> { static constexpr int N1 = 32, N2 = 16; };
+
+// where it is built: FP32 as x-line path 6 of its lengths, FP64 where it is the default
+template <typename T2> constexpr bool march_length(int n) {
+    return sizeof(T2) == 8 ? true : n >= 256 && n <= 512;
+}
+
 enum { kLinesAll, kLinesNamed, kLinesAlt };
 
 template <typename T2, int N1, int N2, int WHAT>
@@ -93,8 +118,15 @@ const LineKernels<T2>* line_table() {
             t.xline3 = k_xline3<T2, N1, N2>;
             if constexpr (F32) t.xline4 = k_xline4<N1, N2>;
         }
+        using MS = MarchSplit<N1 * N2>;
+        if constexpr (WHAT != kLinesAlt && MS::N1 > 0 && march_length<T2>(N1 * N2)) {
+            t.xmarch = k_xmarch<T2, MS::N1, MS::N2>;
+            t.m1 = MS::N1;
+            t.m2 = MS::N2;
+        }
         if constexpr (WHAT != kLinesAlt) {
             t.zinv2 = k_zinv2<T2, N1, N2>;
+            t.xline2b = k_xline2b<T2, N1, N2>;
             t.ib_zinv = k_ib_zinv2<T2, N1, N2>;
             t.ib_xinv = k_ib_xinv2<T2, N1, N2>;
             t.ib_xfwd = k_ib_xfwd2<T2, N1, N2>;

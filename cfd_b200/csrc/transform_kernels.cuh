@@ -224,7 +224,10 @@ __global__ void __launch_bounds__(256) k_xline(Dims d, T2* __restrict__ H0, T2* 
 // The retained modes are kx = 0..N/3 (N1 = 2*(Ngal1/3)), a compile-time bound, so which
 // elements of a subsequence are zero, direct or conjugated is resolved at compile time
 // except in the two blocks that straddle a boundary.
-template <typename T2, int N1, int N2, int TPAD = 1>
+// DIRECT (three bands): u, w, v of every slot of the launch lie interpolated in H0, H1, H2 already,
+// and the products take their place (128-point rows of 128 x 97(+56) x 128 FP64: 36 -> 27 us a band
+// against the radix-by-radix k_xline).
+template <typename T2, int N1, int N2, int TPAD = 1, bool DIRECT = false>
 __device__ __forceinline__ void xline2_body(Dims d, Geo g, const T2* __restrict__ Hx, T2* __restrict__ H0, T2* __restrict__ H1, T2* __restrict__ H2,
                          T2* __restrict__ H3, const T2* __restrict__ twx, int RW, int lrw) {
     using R = decltype(T2::x);
@@ -244,7 +247,8 @@ __device__ __forceinline__ void xline2_body(Dims d, Geo g, const T2* __restrict_
     T2* twt = ex + (size_t)B * LX;
     // u- and v-slots interleaved in y (nyu = nyv + 1), so that the y-neighbour planes read
     // by the interpolation are still in L2 from the adjacent slots
-    const int slot = (blockIdx.y & 1) ? d.nyu + (blockIdx.y >> 1) : (blockIdx.y >> 1);
+    int slot = (blockIdx.y & 1) ? d.nyu + (blockIdx.y >> 1) : (blockIdx.y >> 1);
+    if (DIRECT) slot = (int)blockIdx.y < d.nsu ? d.su0 + blockIdx.y : d.nyu + d.sv0 + (blockIdx.y - d.nsu);
     const int z0 = blockIdx.x * RW;
     const bool uplane = slot < d.nyu;
     const int t = threadIdx.x;
@@ -252,7 +256,7 @@ __device__ __forceinline__ void xline2_body(Dims d, Geo g, const T2* __restrict_
         const int b = i / N2, a = i - b * N2;
         twt[TPAD ? b * TP + a : i] = twx[(a * b) % N];
     }
-    const size_t pbase = (size_t)slot * d.ngal2 * NK;
+    const size_t pbase = DIRECT ? (size_t)slot * d.hstride : (size_t)slot * d.ngal2 * NK;
     // y-interpolated sources of this slot, each ca * plane a + cb * plane b of Hx:
     // u-plane j: u, w direct; v at the centre (ghost centres: the extrapolation of
     // FOU3D.f90:261-283 folded into the weights).  v-plane j: v direct; u, w at the face.
@@ -262,7 +266,11 @@ __device__ __forceinline__ void xline2_body(Dims d, Geo g, const T2* __restrict_
     const T2* Hv = Hx + (size_t)(2 * d.nyu) * pls;
     const T2 *ua, *ub, *va, *vb, *wa, *wb;
     R uca = 1, ucb = 0, vca = 1, vcb = 0;
-    if (uplane) {
+    if (DIRECT) {
+        ua = ub = H0 + pbase;
+        wa = wb = H1 + pbase;
+        va = vb = H2 + pbase;
+    } else if (uplane) {
         const int sl = slot;
         ua = ub = Hu + sl * pls;
         wa = wb = Hw + sl * pls;
@@ -303,7 +311,10 @@ __device__ __forceinline__ void xline2_body(Dims d, Geo g, const T2* __restrict_
             constexpr bool VP = decltype(vplane)::value;
             auto fetch = [&](int k, T2& a, T2& c) {
                 const T2 z = cx<T2>((R)0, (R)0);
-                if (VP) {
+                if (DIRECT) {
+                    a = A0[k];
+                    c = hasc ? C0[k] : z;
+                } else if (VP) {
                     const T2 a0 = A0[k], a1 = A1[k];
                     a = cx<T2>(uca * a0.x + ucb * a1.x, uca * a0.y + ucb * a1.y);
                     c = hasc ? C0[k] : z;
@@ -420,6 +431,12 @@ template <typename T2, int N1, int N2>
 __global__ void __launch_bounds__((16 * (N1 > N2 ? N1 : N2) + 31) / 32 * 32, (sizeof(T2) == 8 && (N1 > N2 ? N1 : N2) <= 24) ? 2 : 1) k_xline2(Dims d, Geo g, const T2* __restrict__ Hx, T2* __restrict__ H0, T2* __restrict__ H1, T2* __restrict__ H2,
                          T2* __restrict__ H3, const T2* __restrict__ twx, int RW, int lrw) {
     xline2_body<T2, N1, N2>(d, g, Hx, H0, H1, H2, H3, twx, RW, lrw);
+}
+
+template <typename T2, int N1, int N2>
+__global__ void __launch_bounds__((16 * (N1 > N2 ? N1 : N2) + 31) / 32 * 32, (sizeof(T2) == 8 && (N1 > N2 ? N1 : N2) <= 24) ? 2 : 1)
+    k_xline2b(Dims d, Geo g, T2* H0, T2* H1, T2* H2, T2* H3, const T2* __restrict__ twx, int RW, int lrw) {
+    xline2_body<T2, N1, N2, 1, true>(d, g, nullptr, H0, H1, H2, H3, twx, RW, lrw);
 }
 
 // The FP32 x-line kernel held to 64 registers per thread: with 4 rows per CTA (192 threads

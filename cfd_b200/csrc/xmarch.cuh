@@ -1,4 +1,5 @@
-// xmarch.cuh - the x-line pass of the nonlinear term marching in y (x-line path 6, FP32).
+// xmarch.cuh - the x-line pass of the nonlinear term marching in y (FP32: x-line path 6; FP64: path 1
+// of the lengths from 256 to 512 that have its split).
 //
 // The products of ops_in_planes (FOU3D.f90:1529-1617) need, on every u-plane, u and w and v
 // interpolated to the centre, and on every v-plane, v and u, w interpolated to the face
@@ -18,7 +19,10 @@
 // In the physical phase the three lanes of a (pair, k1) triple are adjacent (10 triples per
 // warp, lanes 30 and 31 idle) and pass u (A, B -> C) and the face value of w (C -> A, B)
 // with two shuffles, so every lane runs two forward lines, as one packed-pair transform
-// (fft_pair.cuh: each .f32x2 instruction serves both lines).  The forward N1-point step holds
+// (fft_pair.cuh: each .f32x2 instruction serves both lines); in FP64 one line after the other, and the
+// forward exchange takes the place of the inverse one, so that three 96-thread CTAs at 224 registers
+// share an SM: 1534 -> 1290 us a launch at 384 x 257(+90) x 384 (4.5 instead of 7 complex lines a row and
+// plane pair, at 9 instead of 12 warps an SM).  The forward N1-point step holds
 // X[kb + N2 ka] in registers; the unpack of the two real spectra pairs X_k with X_N-k, which
 // lane N2 - kb of the same warp holds (N2 divides 32), so it needs no shared memory.
 //
@@ -39,12 +43,12 @@
 namespace cfd {
 
 template <typename T2, int N1, int N2>
-__global__ void __launch_bounds__(256) k_xmarch(Dims d, Geo g, const T2* __restrict__ Hx, T2* __restrict__ H0,
+__global__ void __launch_bounds__(std::is_same<T2, float2>::value ? 256 : xmarch_threads(N1, N2, 2), std::is_same<T2, float2>::value ? 0 : 3) k_xmarch(Dims d, Geo g, const T2* __restrict__ Hx, T2* __restrict__ H0,
                                                  T2* __restrict__ H1, T2* __restrict__ H2, T2* __restrict__ H3,
                                                  const T2* __restrict__ twx, int RW, int csteps) {
     using R = decltype(T2::x);
     static_assert(N2 == 8 || N2 == 16, "the shuffle unpack pairs lanes kb and N2-kb inside a warp");
-    static_assert(std::is_same<T2, float2>::value, "FP32 only: the forward step runs on packed FP32 pairs");
+    constexpr bool F32 = std::is_same<T2, float2>::value;
     constexpr int N = N1 * N2;
     constexpr int HX = N / 3;               // highest retained kx
     constexpr int NK = HX + 1;              // kx columns per row
@@ -57,8 +61,9 @@ __global__ void __launch_bounds__(256) k_xmarch(Dims d, Geo g, const T2* __restr
     const int NLI = 3 * pairs, NLF = 6 * pairs;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     T2* exi = reinterpret_cast<T2*>(smem_raw);
-    T2* exf = exi + (size_t)NLI * L1;
-    T2* hist = exf + (size_t)NLF * L2;      // hist[k2 * NT + thread]
+    // FP64: the forward exchange takes the inverse one's place
+    T2* exf = F32 ? exi + (size_t)NLI * L1 : exi;
+    T2* hist = F32 ? exf + (size_t)NLF * L2 : exi + xmarch_exchange(N1, N2, RW, false);  // hist[k2 * NT + thread]
     T2* twt = hist + (size_t)N2 * NT;       // twt[b * TP + a] = w^(a*b)
     const int t = threadIdx.x;
     for (int i = t; i < N; i += NT) {
@@ -170,7 +175,7 @@ __global__ void __launch_bounds__(256) k_xmarch(Dims d, Geo g, const T2* __restr
             if (!emit) {
 #pragma unroll
                 for (int k2 = 0; k2 < N2; ++k2) hist[k2 * NT + t] = y[k2];
-            } else {
+            } else if constexpr (F32) {
                 cpair P[N2];  // the lane's two forward lines: x = (Re la, Re lb), y = (Im la, Im lb)
 #pragma unroll
                 for (int k2 = 0; k2 < N2; ++k2) {
@@ -202,6 +207,35 @@ __global__ void __launch_bounds__(256) k_xmarch(Dims d, Geo g, const T2* __restr
                         ob[q * (N1 + 1)] = cx<T2>(v.x.v.y, v.y.v.y);
                     }
                 }
+            } else {
+                // FP64: one output line after the other, la then lb
+                T2 P[N2];
+                auto put = [&](int line) {
+                    rdft<N2, -1>(P);
+                    if (act2) {
+                        T2* o = exf + (size_t)(6 * p2 + 2 * role + line) * L2 + k1;
+#pragma unroll
+                        for (int q = 0; q < N2; ++q) o[q * (N1 + 1)] = q == 0 ? P[0] : cmul(P[q], twt[k1 * TP + q]);
+                    }
+                };
+#pragma unroll
+                for (int k2 = 0; k2 < N2; ++k2) {
+                    const R x2 = isC ? y[k2].y : pa * y[k2].y + pb * hist[k2 * NT + t].y;
+                    P[k2] = cx<T2>(y[k2].x * y[k2].x, x2 * x2);
+                }
+                __syncthreads();  // every lane has read the inverse exchange
+                put(0);
+#pragma unroll
+                for (int k2 = 0; k2 < N2; ++k2) {
+                    const T2 h = hist[k2 * NT + t];
+                    hist[k2 * NT + t] = y[k2];
+                    const R f = fa * y[k2].x + fb * h.x, f2 = fa * y[k2].y + fb * h.y;
+                    const R r1 = __shfl_sync(0xffffffffu, isC ? f : y[k2].x, src1);
+                    const R r2 = __shfl_sync(0xffffffffu, isC ? f2 : y[k2].x, src2);
+                    P[k2] = cx<T2>((isC ? r1 : f) * (isC ? y[k2].x : h.y),
+                                   (isC ? r2 : h.y) * (isC ? y[k2].y : (isA ? r1 : r2)));
+                }
+                put(1);
             }
         }
         __syncthreads();
@@ -214,6 +248,7 @@ __global__ void __launch_bounds__(256) k_xmarch(Dims d, Geo g, const T2* __restr
             const T2* o = exf + (size_t)bfc * L2 + kb * (N1 + 1);
 #pragma unroll
             for (int q = 0; q < N1; ++q) z[q] = o[q];
+            if (!F32) __syncthreads();  // the next step's inverse exchange takes the place of this one
             rdft<N1, -1>(z);
             const size_t ub = (size_t)tu * d.ngal2 * NK;
             const size_t vsb = (size_t)(d.nyu + tu - 1) * d.ngal2 * NK;

@@ -29,13 +29,16 @@ __host__ __device__ constexpr int xmarch_threads(int n1, int n2, int rw) {
     return (nt + 31) / 32 * 32;
 }
 
-// dynamic shared memory (elements of the complex type): inverse and forward exchanges,
-// the per-thread history and the twiddle table
-__host__ __device__ constexpr long long xmarch_smem_elems(int n1, int n2, int rw) {
-    const int pairs = rw / 2;
-    const long long l1 = xmarch_l1(n1, n2), l2 = xmarch_l2(n1, n2);
-    return 3LL * pairs * l1 + 6LL * pairs * l2 + (long long)n2 * xmarch_threads(n1, n2, rw) +
-           (long long)n1 * (n2 + 1);
+// elements of the inverse and forward exchanges: side by side in FP32, in the same place in FP64
+__host__ __device__ constexpr long long xmarch_exchange(int n1, int n2, int rw, bool f32 = true) {
+    const long long a = 3LL * (rw / 2) * xmarch_l1(n1, n2), b = 6LL * (rw / 2) * xmarch_l2(n1, n2);
+    return f32 ? a + b : (a > b ? a : b);
+}
+
+// dynamic shared memory (elements of the complex type): exchanges, the per-thread history and the
+// twiddle table
+__host__ __device__ constexpr long long xmarch_smem_elems(int n1, int n2, int rw, bool f32 = true) {
+    return xmarch_exchange(n1, n2, rw, f32) + (long long)n2 * xmarch_threads(n1, n2, rw) + (long long)n1 * (n2 + 1);
 }
 
 // The roles of thread t of a CTA with RW rows and the split N1 x N2.

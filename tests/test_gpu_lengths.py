@@ -54,3 +54,52 @@ def test_two_step_lengths(torch_cuda, ng1, ng2):
     for k in ("u1", "u2", "u3"):
         assert rel(st[k], ref[k]) < 1e-5, (k, rel(st[k], ref[k]))
     m.close()
+
+
+@pytest.mark.parametrize("chunk", ["2", "3", "32"])
+@pytest.mark.parametrize("ng1", [256, 288, 384, 432, 512])
+def test_marching_xline_fp64(torch_cuda, monkeypatch, ng1, chunk):
+    """The FP64 x-line pass marching in y, with chunk boundaries at every position of its stencil:
+    the nonlinear term to 1e-11 relative L2 of the oracle, and the per-slot kernel it replaces."""
+    from cfd_b200.channel import Channel, build_channel
+    from cfd_b200.config import tiny
+    from oracle.oracle import OracleChannel
+    s = build_channel(tiny(ngal1=ng1, ngal2=18, ny=17, posth=0.0, cyl_diameter=0.0, seed=ng1))
+    o = OracleChannel(s)
+    o.upload_state()
+    o.rhs0(1)
+    o.nonlinear(1)
+    for march in ("1", "0"):
+        monkeypatch.setenv("CFD_XMARCH_STEPS", chunk)
+        monkeypatch.setenv("CFD_MARCH", march)
+        g = Channel(s)
+        g.upload_state()
+        g.rhs0(1)
+        g.nonlinear(1)
+        for k in ("nu1", "nu2", "nu3", "du1", "du2", "du3"):
+            assert rel(g.download(k), o.download(k)) < 1e-11, (march, k)
+        g.close()
+
+
+@pytest.mark.parametrize("chunk", ["2", "3", "32"])
+@pytest.mark.parametrize("ng1", [256, 288, 432, 512, 576])
+def test_marching_xline_fp32(torch_cuda, monkeypatch, ng1, chunk):
+    """The FP32 form at the lengths that take it by default: u, v, w after one step within 1e-5 relative
+    L2 of the oracle, the bound of the FP32-mixed path."""
+    from cfd_b200.channel import Channel, build_channel
+    from cfd_b200.config import tiny
+    from oracle.oracle import OracleChannel
+    s = build_channel(tiny(ngal1=ng1, ngal2=18, ny=17, posth=0.0, cyl_diameter=0.0, seed=ng1))
+    o = OracleChannel(s)
+    o.upload_state()
+    o.step(1)
+    ref = o.download_state()
+    monkeypatch.setenv("CFD_XMARCH_STEPS", chunk)
+    g = Channel(s, precision="mixed")
+    assert g.tuning()["xline_path"] == 6
+    g.upload_state()
+    g.step(1)
+    st = g.download_state()
+    for k in ("u1", "u2", "u3"):
+        assert rel(st[k], ref[k]) < 1e-5, k
+    g.close()
