@@ -1469,7 +1469,11 @@ int create_impl(const cfd_config* cfg, const cfd_ib_list* ibu, const cfd_ib_list
         AL(c->cs, double, nc * nyu);
         AL(c->cs_v, double, nc * nyv);
     }
-    c->JC = tune_int(&cfd_tuning::rhs_chunk, "CFD_RHS_CHUNK", 4, 2, 64);
+    // planes per thread of k_rhs: 4, fewer where that leaves an SM without two CTAs (24 x 17(+6) x 18,
+    // one plane a thread: 7.1 -> 3.1 us)
+    c->JC = 4;
+    while (c->JC > 1 && (long long)((d.ncol + 255) / 256) * ((d.nyu + c->JC - 1) / c->JC) < 2LL * c->nsm) c->JC /= 2;
+    c->JC = tune_int(&cfd_tuning::rhs_chunk, "CFD_RHS_CHUNK", c->JC, 2, 64);
     c->SNT = 1 << ilog2(tune_int(&cfd_tuning::solve_cols, "CFD_SOLVE_THREADS", 64, 32, 256));
     c->nch = (d.nyu - 2 + c->JC - 1) / c->JC;
     AL(c->scal, double, 4);
