@@ -390,8 +390,8 @@ int set_smem_attrs(cfd_ctx* c) {
         set(kn->zfwd2_r, c->SMZN);
     }
     if (c->RWG) {
-        set(line_kernels<T2>(n2)->ib_zin, c->SMZ2);
-        set(line_kernels<T2>(n2)->ib_zout, c->SMZ2);
+        set(line_kernels<T2>(n2, c->ZALT)->ib_zin, c->SMZN);
+        set(line_kernels<T2>(n2, c->ZALT)->ib_zout, c->SMZN);
         set(line_kernels<T2>(n1)->ib_force_x, c->SMG);
     }
     if (c->RWIX2) {
@@ -713,7 +713,7 @@ int ib_grid(cfd_ctx* c, const IBDev& ib, int j0, int nb, double2* rhs_a, double2
 template <typename T2>
 int ib_groups(cfd_ctx* c) {
     const Dims& d = c->d;
-    const auto *kz = line_kernels<T2>(d.ngal2), *kx = line_kernels<T2>(d.ngal1);
+    const auto *kz = line_kernels<T2>(d.ngal2, c->ZALT), *kx = line_kernels<T2>(d.ngal1);
     const size_t pl = (size_t)d.ngal2 * d.nkx;
     const size_t nu = c->ibu.npl * pl, nv = c->ibv.npl * pl;
     IBJobs a{{{c->du1, c->du1, 0, 0}, {c->du3, c->du3, 0, nu}, {c->du2, c->du2, 1, 2 * nu},
@@ -725,7 +725,7 @@ int ib_groups(cfd_ctx* c) {
     const int np = std::max(c->ibu.npl, c->ibv.npl), CH = 1 << c->LZ2;
     const dim3 gz((np * d.nkx + CH - 1) / CH, vel.Hx ? 3 : 6), go(gz.x, 3);
     prof_mark(c);
-    kz->ib_zin<<<gz, c->NTZ2, c->SMZ2, c->stream>>>(d, a, (T2*)c->Hib, twz<T2>(c), c->LZ2);
+    kz->ib_zin<<<gz, c->NTZN, c->SMZN, c->stream>>>(d, a, (T2*)c->Hib, twz<T2>(c), c->LZ2);
     LK("k_ib_zin");
     prof_mark(c);
     const int ng = std::max(c->ibu.ng, c->ibv.ng);
@@ -735,7 +735,7 @@ int ib_groups(cfd_ctx* c) {
         LK("k_ib_force_x");
         prof_mark(c);
     }
-    kz->ib_zout<<<go, c->NTZ2, c->SMZ2, c->stream>>>(d, a, (const T2*)c->Hib, twz<T2>(c), c->LZ2);
+    kz->ib_zout<<<go, c->NTZN, c->SMZN, c->stream>>>(d, a, (const T2*)c->Hib, twz<T2>(c), c->LZ2);
     LK("k_ib_zout");
     return CFD_OK;
 }
@@ -851,6 +851,11 @@ int meanflow_kernel(cfd_ctx* c, int krk, bool ghosts = false) {
     const double beta = kRKb[krk - 1] * c->dt / c->re;
     const double bdt = -kRKd[krk - 1] * c->dt;
     prof_mark(c);
+    if (c->ctpress == 0 && col_rows_per_lane(c->ny + 1)) {
+        col_meanflow(col_rows_per_lane(c->ny + 1), c->stream, c->d, c->g, beta, bdt, c->qxt, c->u1, c->scal, ghosts);
+        LK("k_meanflow");
+        return CFD_OK;
+    }
     k_meanflow<<<1, 32, 0, c->stream>>>(c->d, c->g, beta, bdt, c->qxt, c->ctpress, c->u1, c->scal, c->mf_work, ghosts);
     LK("k_meanflow");
     return CFD_OK;
@@ -875,25 +880,35 @@ int solvep_kernel(cfd_ctx* c, int krk, bool with_div) {
     return CFD_OK;
 }
 
-int vcorr_kernel(cfd_ctx* c, int krk, bool with_div) {
+int divergence_kernel(cfd_ctx* c) {
+    const Dims& d = c->d;
+    dim3 gb((d.ncol + 255) / 256);
+    prof_mark(c);
+    if (c->mb) {
+        k_mb_divergence<<<gb, 256, 0, c->stream>>>(d, c->g, c->u1, c->u2, c->u3, c->div);
+    } else {
+        gb.y = (d.nyp + c->JC - 1) / c->JC;
+        k_divergence<<<gb, 256, 0, c->stream>>>(d, c->g, c->u1, c->u2, c->u3, c->div, c->JC);
+    }
+    LK("k_divergence");
+    return CFD_OK;
+}
+
+// v_corr and its closing divergence
+int vcorr_kernel(cfd_ctx* c, int krk) {
     const Dims& d = c->d;
     const double dtrk = c->dt * (kRKa[krk - 1] + kRKb[krk - 1]);
     dim3 gb((d.ncol + 255) / 256);
     prof_mark(c);
     if (c->mb) {
-        k_mb_vcorr<<<gb, 256, 0, c->stream>>>(d, c->g, dtrk, c->u1, c->u2, c->u3, c->psi, with_div ? c->div : nullptr);
+        k_mb_vcorr<<<gb, 256, 0, c->stream>>>(d, c->g, dtrk, c->u1, c->u2, c->u3, c->psi, c->div);
         LK("k_mb_vcorr");
         return CFD_OK;
     }
-    if (with_div) {
-        k_vcorr<<<gb, 256, 0, c->stream>>>(d, c->g, dtrk, c->u1, c->u2, c->u3, c->psi, c->div);
-        LK("k_vcorr");
-    } else {
-        gb.y = c->nch;
-        k_vcorr_chunk<<<gb, 256, 0, c->stream>>>(d, c->g, dtrk, c->u1, c->u2, c->u3, c->psi, c->JC);
-        LK("k_vcorr_chunk");
-    }
-    return CFD_OK;
+    gb.y = c->nch;
+    k_vcorr_chunk<<<gb, 256, 0, c->stream>>>(d, c->g, dtrk, c->u1, c->u2, c->u3, c->psi, c->JC);
+    LK("k_vcorr_chunk");
+    return divergence_kernel(c);
 }
 
 template <typename T2>
@@ -2083,7 +2098,7 @@ int cfd_solve_p(cfd_ctx* c, int32_t krk) {
 int cfd_vcorr(cfd_ctx* c, int32_t krk) {
     int s = check_krk(c, krk);
     if (s) return s;
-    return vcorr_kernel(c, krk, true);
+    return vcorr_kernel(c, krk);
 }
 
 int cfd_rk_substep(cfd_ctx* c, int32_t krk) {
@@ -2142,12 +2157,8 @@ int cfd_divergence_max(cfd_ctx* c, double* errmax) {
     if (!c || !errmax) return CFD_ERR_ARG;
     const Dims& d = c->d;
     // recompute div from the current state (divergence, littleharsh.f90:209-244)
-    prof_mark(c);
-    if (c->mb)
-        k_mb_divergence<<<(d.ncol + 255) / 256, 256, 0, c->stream>>>(d, c->g, c->u1, c->u2, c->u3, c->div);
-    else
-        k_divergence<<<(d.ncol + 255) / 256, 256, 0, c->stream>>>(d, c->g, c->u1, c->u2, c->u3, c->div);
-    LK("k_divergence");
+    int s = divergence_kernel(c);
+    if (s) return s;
     prof_mark(c);
     k_absmax<<<c->npart, 256, 0, c->stream>>>(c->div, (size_t)d.ncol * d.nyp, c->part);
     LK("k_absmax");

@@ -413,8 +413,10 @@ __global__ void __launch_bounds__(256) k_solve_p(Dims d, Geo g, double dtirk, do
     }
 }
 
-// v_corr without the closing divergence, one thread per column and a chunk of JC planes
-// (the fused substep; cfd_vcorr keeps the sequential k_vcorr that also returns div).
+// v_corr (littleharsh.f90:796-907) of the stage entry point: u -= dt(a+b) ikx psi, w -= dt(a+b) ikz
+// psi, v -= dt(a+b) dthdyv (psi(j+1)-psi(j)), ghost rows by gridweighting, v walls 0; one thread per
+// column and a chunk of JC planes.  Its closing divergence follows in k_divergence.  One thread per
+// column walking all planes took 366 us at 192 x 193(+90) x 192 FP64, the two launches take 41 + 23.
 __global__ void __launch_bounds__(256) k_vcorr_chunk(Dims d, Geo g, double dtrk, double2* __restrict__ u1,
                                                      double2* __restrict__ u2, double2* __restrict__ u3,
                                                      const double2* __restrict__ psi, int JC) {
@@ -452,62 +454,12 @@ __global__ void __launch_bounds__(256) k_vcorr_chunk(Dims d, Geo g, double dtrk,
     }
 }
 
-// v_corr (littleharsh.f90:796-907): u -= dt(a+b) ikx psi, w -= dt(a+b) ikz psi,
-// v -= dt(a+b) dthdyv (psi(j+1)-psi(j)), ghost rows by gridweighting, v walls 0, and the
-// closing divergence (optional).
-__global__ void __launch_bounds__(256) k_vcorr(Dims d, Geo g, double dtrk, double2* __restrict__ u1,
-                                               double2* __restrict__ u2, double2* __restrict__ u3,
-                                               const double2* __restrict__ psi, double2* __restrict__ divo) {
-    const int col = blockIdx.x * blockDim.x + threadIdx.x;
-    if (col >= d.ncol) return;
-    const int i = col % d.nkx, q = col / d.nkx;
-    const double kxv = g.kx[i], kzv = g.kz[q];
-    const size_t nc = d.ncol;
-    double2 psim = dc(0, 0);
-    double2 vprev = dc(0, 0);
-    for (int j = d.ju0 + 1; j <= d.ju1 - 1; ++j) {
-        const size_t ju = (size_t)(j - d.ju0), jp = (size_t)(j - d.jp0), jv = (size_t)(j - d.jv0);
-        const double2 ps = psi[jp * nc + col];
-        const double2 a = dsub(u1[ju * nc + col], dik(dtrk * kxv, ps));
-        const double2 w = dsub(u3[ju * nc + col], dik(dtrk * kzv, ps));
-        u1[ju * nc + col] = a;
-        u3[ju * nc + col] = w;
-        // v at face j-1 (interior faces jv0+1..jv1-1) uses psi(j) - psi(j-1)
-        if (j - 1 >= d.jv0 + 1) {
-            const size_t jvm = jv - 1;
-            const double2 vn = dsub(u2[jvm * nc + col], dscl(dtrk * g.dthdyv[jvm], dsub(ps, psim)));
-            u2[jvm * nc + col] = vn;
-            if (divo) {
-                // divergence at p-point j-1 now that u(j-1), w(j-1), v(j-1), v(j-2) are final
-                const double2 am = u1[(ju - 1) * nc + col], wm = u3[(ju - 1) * nc + col];
-                divo[(jp - 1) * nc + col] = dadd(dadd(dik(kxv, am), dik(kzv, wm)), dscl(g.dthdyu[ju - 1], dsub(vn, vprev)));
-            }
-            vprev = vn;
-        } else {
-            vprev = dc(0, 0);  // wall v(jv0) = 0
-        }
-        psim = ps;
-    }
-    u2[col] = dc(0, 0);
-    u2[(size_t)(d.nyv - 1) * nc + col] = dc(0, 0);
-    u1[col] = dscl(-g.gwb, u1[nc + col]);
-    u3[col] = dscl(-g.gwb, u3[nc + col]);
-    u1[(size_t)(d.nyu - 1) * nc + col] = dscl(-g.gwt, u1[(size_t)(d.nyu - 2) * nc + col]);
-    u3[(size_t)(d.nyu - 1) * nc + col] = dscl(-g.gwt, u3[(size_t)(d.nyu - 2) * nc + col]);
-    if (divo) {
-        // last p-point j = jp1: v(jv1) = 0 (wall)
-        const int j = d.jp1;
-        const size_t ju = (size_t)(j - d.ju0), jp = (size_t)(j - d.jp0);
-        const double2 am = u1[ju * nc + col], wm = u3[ju * nc + col];
-        divo[jp * nc + col] = dadd(dadd(dik(kxv, am), dik(kzv, wm)), dscl(g.dthdyu[ju], dsub(dc(0, 0), vprev)));
-    }
-}
-
 // --------------------------------------------------------------------------------------
 // Mean mode: flowrate_corr with LUsol0/LU_build0/LU_dec0 (littleharsh.f90:452-484,
 // tridLU_3D_IB.f90:320-346, 493-519, 605-622) and flowrateIm (littleharsh.f90:411-430).
-// scal[0] = mpgx, scal[1] = Qx, scal[2] = dgx.  One thread.  The unit-response column
-// spans j = 0..ny (cells between the crests plus one each side), as in the reference.
+// scal[0] = mpgx, scal[1] = Qx, scal[2] = dgx.  The unit-response column spans j = 0..ny (cells
+// between the crests plus one each side), as in the reference.  Constant flow rate on columns
+// that k_meanflow_warp (colsolve.cuh) holds runs that kernel instead.
 // --------------------------------------------------------------------------------------
 __global__ void k_meanflow(Dims d, Geo g, double beta, double bdt, double qxt, int ctpress, double2* __restrict__ u1,
                            double* __restrict__ scal, double* __restrict__ work, bool ghosts) {
@@ -593,15 +545,17 @@ __global__ void k_transpose(const double2* __restrict__ in, double2* __restrict_
     }
 }
 
-// divergence at every p-point (littleharsh.f90:209-244), no state change
+// divergence at every p-point (littleharsh.f90:209-244), no state change; one thread per column and
+// a chunk of JC planes (blockIdx.y)
 __global__ void __launch_bounds__(256) k_divergence(Dims d, Geo g, const double2* __restrict__ u1,
                                                     const double2* __restrict__ u2, const double2* __restrict__ u3,
-                                                    double2* __restrict__ divo) {
+                                                    double2* __restrict__ divo, int JC) {
     const int col = blockIdx.x * blockDim.x + threadIdx.x;
     if (col >= d.ncol) return;
     const double kxv = g.kx[col % d.nkx], kzv = g.kz[col / d.nkx];
     const size_t nc = d.ncol;
-    for (int j = d.jp0; j <= d.jp1; ++j) {
+    const int j0 = d.jp0 + blockIdx.y * JC;
+    for (int j = j0; j <= min(j0 + JC - 1, d.jp1); ++j) {
         const size_t ju = (size_t)(j - d.ju0), jv = (size_t)(j - d.jv0);
         divo[(size_t)(j - d.jp0) * nc + col] =
             dadd(dadd(dik(kxv, u1[ju * nc + col]), dik(kzv, u3[ju * nc + col])),

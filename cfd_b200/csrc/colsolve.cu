@@ -23,6 +23,11 @@ bool col_map(CUtensorMap* map, const void* field, int ncol, int n, int m, int co
                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+void col_meanflow(int m, cudaStream_t st, const Dims& d, const Geo& g, double beta, double bdt, double qxt, double2* u1,
+                  double* scal, bool ghosts) {
+    COL_SWITCH(m, { k_meanflow_warp<MR><<<1, 32, 0, st>>>(d, g, beta, bdt, qxt, u1, scal, ghosts); });
+}
+
 cudaError_t col_prepare(int m, bool mb) { return mb ? col_prepare_mb(m) : prepare<false>(m); }
 
 void col_launch(int mode, int m, int cols, bool mb, int nsm, cudaStream_t st, const Dims& d, const Geo& g,

@@ -449,6 +449,65 @@ __global__ void __launch_bounds__(32 * C * col_groups(M, C))
     if (lead) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
 }
 
+// Mean mode at constant flow rate: flowrate_corr with LUsol0/LU_build0/LU_dec0
+// (littleharsh.f90:452-484, tridLU_3D_IB.f90:320-346, 493-519, 605-622), the unit response of the
+// cells between the crests and one each side (j = 0..ny) solved by the warp's partition.  One lane
+// walking the column through memory took 42 us at 194 rows, the warp takes 7.5.  scal[0] = mpgx,
+// scal[2] = dgx.  ghosts: extrapolate the column's ghost rows as v_corr does.
+template <int M>
+__global__ void __launch_bounds__(32) k_meanflow_warp(Dims d, Geo g, double beta, double bdt, double qxt,
+                                                      double2* __restrict__ u1, double* __restrict__ scal, bool ghosts) {
+    const int lane = threadIdx.x, n = d.ny + 1, row0 = lane * M;
+    double2 x[1][M];
+    double q0 = 0.0, q1 = 0.0;
+    // cell width between the faces below and above centre j, for the cells between the crests
+    auto width = [&](int j) { return j >= 1 && j <= n - 2 ? g.yv[j - d.jv0] - g.yv[j - 1 - d.jv0] : 0.0; };
+#pragma unroll
+    for (int i = 0; i < M; ++i) {
+        const int j = row0 + i;
+        x[0][i] = dc(j >= 1 && j <= n - 2 ? bdt : 0.0, 0.0);
+        if (j >= 1 && j <= n - 2) q0 += width(j) * u1[(size_t)(j - d.ju0) * d.ncol].x;
+    }
+    warp_tridiag<M, 1>(x, [&](int i, double& a, double& c, double& s) {
+        const int j = row0 + i;
+        a = c = 0.0;
+        s = 1.0;
+        if (j >= 1 && j <= n - 2) {
+            const double* w = g.dyu2i + 3 * (j - d.ju0);
+            a = beta * w[0];
+            c = beta * w[2];
+            s = 1.0 - beta * ((w[0] + w[2]) + w[1]);
+        } else if (j == 0) {
+            c = -g.gwb;
+            s = 1.0 - c;
+        } else if (j == n - 1) {
+            a = -g.gwt;
+            s = 1.0 - a;
+        }
+    });
+#pragma unroll
+    for (int i = 0; i < M; ++i) q1 += width(row0 + i) * x[0][i].x;
+    for (int o = 16; o > 0; o >>= 1) {
+        q0 += __shfl_xor_sync(0xffffffffu, q0, o);
+        q1 += __shfl_xor_sync(0xffffffffu, q1, o);
+    }
+    const double gg = (qxt - q0) / q1;
+    if (lane == 0) {
+        scal[0] += gg;
+        scal[2] = gg;
+    }
+#pragma unroll
+    for (int i = 0; i < M; ++i)
+        if (row0 + i < n) u1[(size_t)(row0 + i - d.ju0) * d.ncol].x += gg * x[0][i].x;
+    if (ghosts) {
+        __syncwarp();
+        if (lane == 0) {
+            u1[0] = dscl(-g.gwb, u1[d.ncol]);
+            u1[(size_t)(d.nyu - 1) * d.ncol] = dscl(-g.gwt, u1[(size_t)(d.nyu - 2) * d.ncol]);
+        }
+    }
+}
+
 // Host side (colsolve.cu; the _mb forms in colsolve_mb.cu): m rows per lane, cols columns a group
 // (4 in three bands), mb three bands
 cudaError_t col_prepare(int m, bool mb);  // raises the shared-memory limit of the kernels
@@ -457,6 +516,9 @@ cudaError_t col_prepare_mb(int m);
 bool col_map(CUtensorMap* map, const void* field, int ncol, int n, int m, int cols);
 void col_launch(int mode, int m, int cols, bool mb, int nsm, cudaStream_t st, const Dims& d, const Geo& g,
                 const ColMaps& maps, const ColArgs& a);
+// k_meanflow_warp with m rows per lane, m = col_rows_per_lane(ny + 1)
+void col_meanflow(int m, cudaStream_t st, const Dims& d, const Geo& g, double beta, double bdt, double qxt, double2* u1,
+                  double* scal, bool ghosts);
 void col_launch_mb(int mode, int m, int nsm, cudaStream_t st, const Dims& d, const Geo& g, const ColMaps& maps,
                    const ColArgs& a);
 

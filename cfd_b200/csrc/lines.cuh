@@ -53,7 +53,7 @@ struct LineKernels {
 };
 
 // The kernels of length n, null where it has none; alt: the transposed split of the six named
-// lengths (only zinv2s, zfwd2, xline2 and their variants).
+// lengths (only zinv2s, zfwd2, xline2, their variants, ib_zin and ib_zout).
 template <typename T2> const LineKernels<T2>* line_kernels(int n, bool alt = false);
 
 // what each unit holds (null for the lengths it does not)
@@ -109,6 +109,8 @@ const LineKernels<T2>* line_table() {
         t.zinv2s = k_zinv2s<T2, N1, N2>;
         t.zfwd2 = k_zfwd2<T2, N1, N2>;
         t.xline2 = k_xline2<T2, N1, N2>;
+        t.ib_zin = k_ib_zin<T2, N1, N2>;
+        t.ib_zout = k_ib_zout<T2, N1, N2>;
         if constexpr (!F32 && N1 * N2 <= 384) {
             t.zinv2s_r = k_zinv2sd<N1, N2>;
             t.zfwd2_r = k_zfwd2d<N1, N2>;
@@ -131,9 +133,7 @@ const LineKernels<T2>* line_table() {
             t.ib_xinv = k_ib_xinv2<T2, N1, N2>;
             t.ib_xfwd = k_ib_xfwd2<T2, N1, N2>;
             t.ib_zfwd = k_ib_zfwd2<T2, N1, N2>;
-            t.ib_zin = k_ib_zin<T2, N1, N2>;
             t.ib_force_x = k_ib_force_x<T2, N1, N2>;
-            t.ib_zout = k_ib_zout<T2, N1, N2>;
         }
         if constexpr (WHAT != kLinesAlt && !F32) {
             t.st_z = k_st_z<N1, N2>;
