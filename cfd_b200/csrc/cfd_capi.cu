@@ -14,6 +14,7 @@
 #include <cstdint>
 #include <cstdlib>
 #include <cstring>
+#include <mutex>
 #include <string>
 #include <unordered_map>
 #include <vector>
@@ -355,6 +356,19 @@ size_t xline2_smem(int n1s, int n2s, int rw, size_t esz) {
 }
 
 // ---------------------------------------------------------------------------------------
+// Lets a kernel take `bytes` of dynamic shared memory.  The limit belongs to the kernel, which other
+// contexts launch with sizes of their own, so it is raised and never lowered.
+template <typename F>
+cudaError_t smem_limit(F* f, int bytes) {
+    static std::mutex mu;
+    std::lock_guard<std::mutex> hold(mu);
+    cudaFuncAttributes a;
+    cudaError_t e = cudaFuncGetAttributes(&a, f);
+    if (e == cudaSuccess && bytes > a.maxDynamicSharedSizeBytes)
+        e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    return e;
+}
+
 template <typename T2>
 int set_smem_attrs(cfd_ctx* c) {
     const size_t esz = sizeof(T2);
@@ -365,18 +379,18 @@ int set_smem_attrs(cfd_ctx* c) {
     size_t sf = (size_t)(2 * (c->RWibf / 2) * n1 + n1) * esz;
     cudaError_t e = cudaSuccess;
     FFT_SWITCH(n2, {
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(k_zinv<T2, NF>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sz);
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(k_zfwd<T2, NF>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sz);
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(k_ib_zinv<T2, NF>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sz);
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(k_ib_zfwd<T2, NF>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sz);
+        if (e == cudaSuccess) e = smem_limit(k_zinv<T2, NF>, (int)sz);
+        if (e == cudaSuccess) e = smem_limit(k_zfwd<T2, NF>, (int)sz);
+        if (e == cudaSuccess) e = smem_limit(k_ib_zinv<T2, NF>, (int)sz);
+        if (e == cudaSuccess) e = smem_limit(k_ib_zfwd<T2, NF>, (int)sz);
     });
     FFT_SWITCH(n1, {
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(k_xline<T2, NF>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sx);
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(k_ib_xinv<T2, NF>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)si);
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(k_ib_xfwd<T2, NF>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sf);
+        if (e == cudaSuccess) e = smem_limit(k_xline<T2, NF>, (int)sx);
+        if (e == cudaSuccess) e = smem_limit(k_ib_xinv<T2, NF>, (int)si);
+        if (e == cudaSuccess) e = smem_limit(k_ib_xfwd<T2, NF>, (int)sf);
     });
     auto set = [&](auto* f, size_t n) {
-        if (f && e == cudaSuccess) e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)n);
+        if (f && e == cudaSuccess) e = smem_limit(f, (int)n);
     };
     if (c->LZ2 >= 0) {
         const auto* k = line_kernels<T2>(n2);
@@ -420,7 +434,7 @@ int set_smem_attrs(cfd_ctx* c) {
                 set(kb->xline2b, smb);
             }
         FFT_SWITCH(c->dM.ngal1, {
-            if (e == cudaSuccess) e = cudaFuncSetAttribute(k_xline<T2, NF>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sx);
+            if (e == cudaSuccess) e = smem_limit(k_xline<T2, NF>, (int)sx);
         });
     }
     CK(e);
@@ -1575,7 +1589,7 @@ int strided_cft(cfd_ctx* c, double* dptr, int n, int ise, int isa, int m, long l
         const bool a2 = ((uintptr_t)dptr & 15) == 0 && !((ise | isa | bstride) & 1);
         auto* f = k->pl_cft[iopt < 0][a2];
         const int lsm = (int)(((size_t)8 * ((k->n1 * (k->n2 + 1)) | 1) + n) * sizeof(double2));
-        CK(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, lsm));
+        CK(smem_limit(f, lsm));
         prof_mark(c);
         f<<<dim3((m + 7) / 8, nb), 8 * std::max(k->n1, k->n2), lsm, c->stream>>>(dptr, ise, isa, m, bstride, tw, 3);
         LK("k_pl_cft");
@@ -1583,7 +1597,7 @@ int strided_cft(cfd_ctx* c, double* dptr, int n, int ise, int isa, int m, long l
     }
     const int CH = 8;
     const int sm = fft_generic_smem(n, CH);
-    CK(cudaFuncSetAttribute(k_cft_strided, cudaFuncAttributeMaxDynamicSharedMemorySize, sm));
+    CK(smem_limit(k_cft_strided, sm));
     dim3 grid((m + CH - 1) / CH, nb);
     prof_mark(c);
     k_cft_strided<<<grid, 256, sm, c->stream>>>(dptr, ise, isa, m, bstride, fd, tw, iopt, CH);
@@ -1605,7 +1619,7 @@ int strided_rft(cfd_ctx* c, double* dptr, int n, int isa, int m, long long bstri
         };
         int nl = 8;
         while (nl > 1 && lsm(nl) > 72 * 1024) nl /= 2;
-        CK(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, lsm(nl)));
+        CK(smem_limit(f, lsm(nl)));
         const int pairs = (m + 1) / 2;
         prof_mark(c);
         f<<<dim3((pairs + nl - 1) / nl, nb), (nl * std::max(k->n1, k->n2) + 31) / 32 * 32, lsm(nl), c->stream>>>(
@@ -1615,7 +1629,7 @@ int strided_rft(cfd_ctx* c, double* dptr, int n, int isa, int m, long long bstri
     }
     const int CH = 8;
     const int sm = fft_generic_smem(n, CH);
-    CK(cudaFuncSetAttribute(k_rft_strided, cudaFuncAttributeMaxDynamicSharedMemorySize, sm));
+    CK(smem_limit(k_rft_strided, sm));
     // the inverse transforms two lines per complex transform
     const int lines = iopt > 0 ? (m + 1) / 2 : m;
     dim3 grid((lines + CH - 1) / CH, nb);
@@ -1718,8 +1732,8 @@ int stats_pass_lines(cfd_ctx* c, bool acc) {
     const size_t smz = ((size_t)8 * ((kz->n1 * (kz->n2 + 1)) | 1) + d.ngal2) * sizeof(double2);
     const size_t smx = ((size_t)nlr * rw * st_x_row(kx->n1, kx->n2) + d.ngal1) * sizeof(double2);
     const int ntx = (nlr * rw * std::max(kx->n1, kx->n2) + 31) / 32 * 32;
-    CK(cudaFuncSetAttribute(kz->st_z, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smz));
-    CK(cudaFuncSetAttribute(kx->st_x[acc], cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smx));
+    CK(smem_limit(kz->st_z, (int)smz));
+    CK(smem_limit(kx->st_x[acc], (int)smx));
     for (int j0 = 0; j0 < d.nyu; j0 += cp) {
         const int n = std::min(cp, d.nyu - j0);
         StChunk s{j0, n, {0, cp, 2 * cp + 1, 3 * cp + 4, 4 * cp + 4}, {j0, j0, j0 - 2, j0, j0}, {n, n + 1, n + 3, n, n}};

@@ -61,3 +61,29 @@ def test_point_lists(monkeypatch, which, groups):
         for k in ("du1", "du2", "du3", "u1", "u2", "u3"):
             assert rel(g.download(k), o.download(k)) < 1e-11, (upload, k)
     g.close()
+
+
+def test_contexts_with_other_group_sizes():
+    """A kernel's shared-memory limit holds for every context that launches it: groups of eight rows
+    (58 KB at 384 points) still run after a context of six (45 KB) is made."""
+    torch = pytest.importorskip("torch")
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    from cfd_b200.channel import Channel, build_channel
+    from cfd_b200.config import tiny
+    sets = []
+    for which in ("seven", "single"):
+        s = build_channel(tiny(ngal1=384, ngal2=54, ny=17, cyl_diameter=0.3, cyl_spacing=0.9, seed=3))
+        s.ibu, s.ibv = points(np.random.default_rng(7), s, s.ibu, which), points(np.random.default_rng(8), s, s.ibv, which)
+        sets.append(s)
+
+    def substep(ch):
+        ch.upload_state()
+        ch.rk_substep(1)
+        return ch.download("u1")
+
+    a = Channel(sets[0])
+    before = substep(a)
+    b = Channel(sets[1])
+    substep(b)
+    np.testing.assert_array_equal(substep(a), before)
