@@ -65,7 +65,7 @@ struct IBDev {
     // z rows in groups closed under the stencils of their points (ib_rows)
     int ng = 0;
     int* grows = nullptr;
-    int* gptr = nullptr;
+    int2* gptr = nullptr;
     uint4* gpts = nullptr;
     double* gw = nullptr;
 };
@@ -1078,22 +1078,59 @@ int setup_ib(cfd_ctx* c, const cfd_ib_list* l, int j0, int j1, IBDev& ib, const 
     return CFD_OK;
 }
 
+// The points of a list by plane (lists are sorted by plane).  The lattices repeat from plane to plane:
+// one whose points and weights are those of the plane before, the plane itself aside, is listed as
+// that one, so the host packs and the device reads its points once.
+struct IBPlanes {
+    std::vector<int> begin;  // first point of every plane, and the list's end
+    std::vector<int> as;     // plane (of this list) that it repeats
+    bool flat = true;        // no point reaches into another plane
+};
+
+IBPlanes ib_planes(const cfd_ib_list* l) {
+    IBPlanes q;
+    auto id = [&](int p) { return l->idx + 9 * (size_t)p; };
+    for (int p = 0; p < l->n; ++p) {
+        const int32_t* x = id(p);
+        if (p == 0 || x[2] != id(p - 1)[2]) q.begin.push_back(p);
+        q.flat = q.flat && x[5] == x[2] && x[8] == x[2];
+    }
+    q.begin.push_back(l->n);
+    const int n = (int)q.begin.size() - 1;
+    for (int k = 0; k < n; ++k) {
+        q.as.push_back(k);
+        if (k == 0) continue;
+        const int b = q.begin[k], r = q.begin[q.as[k - 1]], m = q.begin[k + 1] - b;
+        bool same = m == q.begin[q.as[k - 1] + 1] - r &&
+                    std::memcmp(l->w + 3 * (size_t)b, l->w + 3 * (size_t)r, 3 * sizeof(double) * m) == 0;
+        for (int e = 0; same && e < m; ++e) {
+            const int32_t *x = id(b + e), *y = id(r + e);
+            same = x[0] == y[0] && x[1] == y[1] && x[3] == y[3] && x[4] == y[4] && x[6] == y[6] && x[7] == y[7];
+        }
+        if (same) q.as[k] = q.as[k - 1];
+    }
+    return q;
+}
+
 // Groups of z rows for k_ib_force_x.  Rows that a point ties together (its target and its two
 // stencil rows, in one plane) form a component; components are packed into groups of at most rw
 // rows.  Fails (false) if a point reaches into another plane or a component has more than rw rows.
-bool ib_components(const cfd_ib_list* l, int ng2, std::vector<std::vector<int>>& comp) {
+bool ib_components(const cfd_ib_list* l, const IBPlanes& pl, int ng2, std::vector<std::vector<int>>& comp) {
+    if (!pl.flat) return false;
     std::vector<int> root(ng2), used(ng2, 0);
     for (int k = 0; k < ng2; ++k) root[k] = k;
     auto find = [&](int k) {
         while (root[k] != k) k = root[k] = root[root[k]];
         return k;
     };
-    for (int p = 0; p < l->n; ++p) {
-        const int32_t* id = l->idx + 9 * (size_t)p;
-        if (id[5] != id[2] || id[8] != id[2]) return false;
-        if (p > 0 && id[1] == id[1 - 9] && id[4] == id[4 - 9] && id[7] == id[7 - 9]) continue;
-        for (int t = 0; t < 3; ++t) used[id[3 * t + 1] - 1] = 1;
-        for (int t = 1; t < 3; ++t) root[find(id[3 * t + 1] - 1)] = find(id[1] - 1);
+    for (size_t q = 0; q < pl.as.size(); ++q) {
+        if (pl.as[q] != (int)q) continue;
+        for (int p = pl.begin[q]; p < pl.begin[q + 1]; ++p) {
+            const int32_t* id = l->idx + 9 * (size_t)p;
+            if (p > 0 && id[1] == id[1 - 9] && id[4] == id[4 - 9] && id[7] == id[7 - 9]) continue;
+            for (int t = 0; t < 3; ++t) used[id[3 * t + 1] - 1] = 1;
+            for (int t = 1; t < 3; ++t) root[find(id[3 * t + 1] - 1)] = find(id[1] - 1);
+        }
     }
     std::vector<int> where(ng2, -1);
     comp.clear();
@@ -1119,7 +1156,8 @@ std::vector<std::vector<int>> ib_pack(const std::vector<std::vector<int>>& comp,
     return g;
 }
 
-int ib_rows(cfd_ctx* c, const cfd_ib_list* l, const std::vector<std::vector<int>>& g, int rw, int j0, IBDev& ib) {
+int ib_rows(cfd_ctx* c, const cfd_ib_list* l, const IBPlanes& pl, const std::vector<std::vector<int>>& g, int rw, int j0,
+            IBDev& ib) {
     ib.ng = (int)g.size();
     const int ng2 = c->d.ngal2, ng = ib.ng;
     if (!l || ng == 0) return CFD_OK;
@@ -1131,15 +1169,9 @@ int ib_rows(cfd_ctx* c, const cfd_ib_list* l, const std::vector<std::vector<int>
             local[g[q][r]] = (int)r;
         }
     for (int p = 0; p < ib.npl; ++p) slot[ib.h_planes[p] - j0] = p;
-    std::vector<int> bucket(l->n);
-    std::vector<int> ptr((size_t)ib.npl * ng + 1, 0);
-    for (int p = 0; p < l->n; ++p) {
-        const int32_t* id = l->idx + 9 * (size_t)p;
-        bucket[p] = slot[id[2] - j0] * ng + group[id[1] - 1];
-        ptr[bucket[p] + 1]++;
-    }
-    for (size_t k = 1; k < ptr.size(); ++k) ptr[k] += ptr[k - 1];
-    std::vector<uint4> pts(l->n);
+    // points by (plane, group), in list order within one: runs of equal targets stay together
+    std::vector<int2> ptr((size_t)ib.npl * ng, make_int2(0, 0));
+    std::vector<uint4> pts;
     // the lattices repeat a few triples of weights: looked up in a hash of their bits
     std::vector<double> w;
     std::unordered_multimap<uint64_t, unsigned> seen;
@@ -1160,21 +1192,38 @@ int ib_rows(cfd_ctx* c, const cfd_ib_list* l, const std::vector<std::vector<int>
         seen.emplace(h, last);
         return last;
     };
-    std::vector<int> at(ptr.begin(), ptr.end() - 1);
-    for (int p = 0; p < l->n; ++p) {  // list order within a bucket: runs of equal targets stay together
-        const int32_t* id = l->idx + 9 * (size_t)p;
-        uint4& o = pts[at[bucket[p]]++];
-        o.x = (unsigned)(id[0] - 1) | (unsigned)(id[3] - 1) << 16;
-        o.y = (unsigned)(id[6] - 1) | (unsigned)local[id[1] - 1] << 16 | (unsigned)local[id[4] - 1] << 24;
-        o.z = (unsigned)local[id[7] - 1];
-        o.w = weight(l->w + 3 * (size_t)p);
+    std::vector<int> at(ng);
+    for (size_t q = 0; q < pl.as.size(); ++q) {
+        int2* pr = ptr.data() + (size_t)slot[l->idx[9 * (size_t)pl.begin[q] + 2] - j0] * ng;
+        if (pl.as[q] != (int)q) {
+            const int2* r = ptr.data() + (size_t)slot[l->idx[9 * (size_t)pl.begin[pl.as[q]] + 2] - j0] * ng;
+            std::copy(r, r + ng, pr);
+            continue;
+        }
+        std::fill(at.begin(), at.end(), 0);
+        for (int p = pl.begin[q]; p < pl.begin[q + 1]; ++p) at[group[l->idx[9 * (size_t)p + 1] - 1]]++;
+        int e = (int)pts.size();
+        for (int k = 0; k < ng; ++k) {
+            pr[k] = make_int2(e, e + at[k]);
+            at[k] = e;
+            e = pr[k].y;
+        }
+        pts.resize(e);
+        for (int p = pl.begin[q]; p < pl.begin[q + 1]; ++p) {
+            const int32_t* id = l->idx + 9 * (size_t)p;
+            uint4& o = pts[at[group[id[1] - 1]]++];
+            o.x = (unsigned)(id[0] - 1) | (unsigned)(id[3] - 1) << 16;
+            o.y = (unsigned)(id[6] - 1) | (unsigned)local[id[1] - 1] << 16 | (unsigned)local[id[4] - 1] << 24;
+            o.z = (unsigned)local[id[7] - 1];
+            o.w = weight(l->w + 3 * (size_t)p);
+        }
     }
     AL(ib.grows, int, rows.size());
-    AL(ib.gptr, int, ptr.size());
+    AL(ib.gptr, int2, ptr.size());
     AL(ib.gpts, uint4, pts.size());
     AL(ib.gw, double, w.size());
     CK(cudaMemcpy(ib.grows, rows.data(), rows.size() * sizeof(int), cudaMemcpyHostToDevice));
-    CK(cudaMemcpy(ib.gptr, ptr.data(), ptr.size() * sizeof(int), cudaMemcpyHostToDevice));
+    CK(cudaMemcpy(ib.gptr, ptr.data(), ptr.size() * sizeof(int2), cudaMemcpyHostToDevice));
     CK(cudaMemcpy(ib.gpts, pts.data(), pts.size() * sizeof(uint4), cudaMemcpyHostToDevice));
     CK(cudaMemcpy(ib.gw, w.data(), w.size() * sizeof(double), cudaMemcpyHostToDevice));
     return CFD_OK;
@@ -1531,7 +1580,8 @@ int create_impl(const cfd_config* cfg, const cfd_ib_list* ibu, const cfd_ib_list
         std::vector<std::vector<int>> cu, cv;
         const auto* kx = line_kernels<float2>(d.ngal1);
         const int lx = ib_pitch(kx->n1, kx->n2);
-        if ((!ibu || ib_components(ibu, d.ngal2, cu)) && (!ibv || ib_components(ibv, d.ngal2, cv))) {
+        const IBPlanes pu = ibu ? ib_planes(ibu) : IBPlanes(), pv = ibv ? ib_planes(ibv) : IBPlanes();
+        if ((!ibu || ib_components(ibu, pu, d.ngal2, cu)) && (!ibv || ib_components(ibv, pv, d.ngal2, cv))) {
             size_t best = 0;
             for (int rw : {8, 6, 4, 2}) {
                 const auto gu = ib_pack(cu, rw), gv = ib_pack(cv, rw);
@@ -1544,8 +1594,8 @@ int create_impl(const cfd_config* cfg, const cfd_ib_list* ibu, const cfd_ib_list
                 c->SMG = sm;
             }
             if (c->RWG) {
-                if ((s = ib_rows(c, ibu, ib_pack(cu, c->RWG), c->RWG, d.ju0, c->ibu)) != CFD_OK) return s;
-                if ((s = ib_rows(c, ibv, ib_pack(cv, c->RWG), c->RWG, d.jv0, c->ibv)) != CFD_OK) return s;
+                if ((s = ib_rows(c, ibu, pu, ib_pack(cu, c->RWG), c->RWG, d.ju0, c->ibu)) != CFD_OK) return s;
+                if ((s = ib_rows(c, ibv, pv, ib_pack(cv, c->RWG), c->RWG, d.jv0, c->ibv)) != CFD_OK) return s;
                 const size_t n = (nibu + nibv) * hz;
                 if (mixed) AL(c->Hib, float2, n); else AL(c->Hib, double2, n);
                 if ((s = mixed ? set_smem_attrs<float2>(c) : set_smem_attrs<double2>(c)) != CFD_OK) return s;

@@ -1400,7 +1400,7 @@ struct IBJobs {
 };
 struct IBRows {
     const int* rows;    // [ng][RW] z rows of a group, -1 past its last
-    const int* ptr;     // [npl*ng + 1] forcing points of (plane, group)
+    const int2* ptr;    // [npl*ng] forcing points of (plane, group): first, past the last
     const uint4* pts;   // x: i, i2; y: i3, row, row 2; z: row 3 (of the group); w: weights
     const double* w;    // [..][3] Lap, w2, w3
     int ng;
@@ -1554,7 +1554,8 @@ __global__ void __launch_bounds__(((sizeof(T2) == 8 ? 16 : 8) * (TN1 > TN2 ? TN1
     // (tridLU_3D_IB.f90:193-211); the first point of a run of equal targets applies the run in
     // list order, as k_ib_force does
     {
-        const int e0 = G.ptr[p * G.ng + blockIdx.x], e1 = G.ptr[p * G.ng + blockIdx.x + 1];
+        const int2 pr = G.ptr[p * G.ng + blockIdx.x];
+        const int e0 = pr.x, e1 = pr.y;
         for (int e = e0 + t; e < e1; e += blockDim.x) {
             uint4 q = G.pts[e];
             const unsigned ti = q.x & 0xffff, tr = (q.y >> 16) & 0xff;
