@@ -1030,7 +1030,41 @@ int fill_tw(cfd_ctx* c, int n, double2** dd, float2** df) {
     return CFD_OK;
 }
 
-int setup_ib(cfd_ctx* c, const cfd_ib_list* l, int j0, int j1, IBDev& ib, const char* name) {
+// The points of a list by plane (lists are sorted by plane).  The lattices repeat from plane to plane:
+// one whose points and weights are those of the plane before, the plane itself aside, is listed as
+// that one, so the host packs and the device reads its points once.
+struct IBPlanes {
+    std::vector<int> begin;  // first point of every plane, and the list's end
+    std::vector<int> as;     // plane (of this list) that it repeats
+    bool flat = true;        // no point reaches into another plane
+};
+
+IBPlanes ib_planes(const cfd_ib_list* l) {
+    IBPlanes q;
+    auto id = [&](int p) { return l->idx + 9 * (size_t)p; };
+    for (int p = 0; p < l->n; ++p) {
+        const int32_t* x = id(p);
+        if (p == 0 || x[2] != x[2 - 9]) q.begin.push_back(p);
+        q.flat = q.flat && x[5] == x[2] && x[8] == x[2];
+    }
+    q.begin.push_back(l->n);
+    const int n = (int)q.begin.size() - 1;
+    for (int k = 0; k < n; ++k) {
+        q.as.push_back(k);
+        if (k == 0 || !q.flat) continue;
+        const int b = q.begin[k], r = q.begin[q.as[k - 1]], m = q.begin[k + 1] - b;
+        bool same = m == q.begin[q.as[k - 1] + 1] - r &&
+                    std::memcmp(l->w + 3 * (size_t)b, l->w + 3 * (size_t)r, 3 * sizeof(double) * m) == 0;
+        for (int e = 0; same && e < m; ++e) {
+            const int32_t *x = id(b + e), *y = id(r + e);
+            same = x[0] == y[0] && x[1] == y[1] && x[3] == y[3] && x[4] == y[4] && x[6] == y[6] && x[7] == y[7];
+        }
+        if (same) q.as[k] = q.as[k - 1];
+    }
+    return q;
+}
+
+int setup_ib(cfd_ctx* c, const cfd_ib_list* l, int j0, int j1, IBDev& ib, IBPlanes& pl, const char* name) {
     if (!l) return CFD_OK;
     if (l->n < 0) return fail(c, CFD_ERR_ARG, "%s: negative point count", name);
     if (l->n > 0 && (!l->idx || !l->w)) return fail(c, CFD_ERR_ARG, "%s: null list arrays", name);
@@ -1044,7 +1078,10 @@ int setup_ib(cfd_ctx* c, const cfd_ib_list* l, int j0, int j1, IBDev& ib, const 
             }
     ib.npl = (int)ib.h_planes.size();
     const int ng1 = c->d.ngal1, ng2 = c->d.ngal2;
-    for (int p = 0; p < l->n; ++p) {
+    pl = ib_planes(l);
+    // (of a plane that repeats another, the first point stands for the rest)
+    for (size_t q = 0; q < pl.as.size(); ++q)
+    for (int p = pl.begin[q], e = pl.as[q] == (int)q ? pl.begin[q + 1] : p + 1; p < e; ++p) {
         const int32_t* id = l->idx + 9 * (size_t)p;
         for (int t = 0; t < 3; ++t) {
             const int i = id[3 * t], k = id[3 * t + 1], j = id[3 * t + 2];
@@ -1065,8 +1102,10 @@ int setup_ib(cfd_ctx* c, const cfd_ib_list* l, int j0, int j1, IBDev& ib, const 
     if (ib.npl > 0) CK(cudaMemcpy(ib.planes, ib.h_planes.data(), sizeof(int) * ib.npl, cudaMemcpyHostToDevice));
     CK(cudaMemcpy(ib.slot_of_j, slot.data(), sizeof(int) * slot.size(), cudaMemcpyHostToDevice));
     std::vector<unsigned char> flag(ng2, 0);
-    for (int p = 0; p < l->n; ++p)
-        for (int t = 0; t < 3; ++t) flag[l->idx[9 * (size_t)p + 3 * t + 1] - 1] = 1;
+    for (size_t q = 0; q < pl.as.size(); ++q)
+        if (pl.as[q] == (int)q)
+            for (int p = pl.begin[q]; p < pl.begin[q + 1]; ++p)
+                for (int t = 0; t < 3; ++t) flag[l->idx[9 * (size_t)p + 3 * t + 1] - 1] = 1;
     std::vector<int> rows;
     for (int k = 0; k < ng2; ++k)
         if (flag[k]) rows.push_back(k);
@@ -1076,40 +1115,6 @@ int setup_ib(cfd_ctx* c, const cfd_ib_list* l, int j0, int j1, IBDev& ib, const 
     if (ib.nact > 0) CK(cudaMemcpy(ib.arow, rows.data(), sizeof(int) * ib.nact, cudaMemcpyHostToDevice));
     CK(cudaMemcpy(ib.rowflag, flag.data(), ng2, cudaMemcpyHostToDevice));
     return CFD_OK;
-}
-
-// The points of a list by plane (lists are sorted by plane).  The lattices repeat from plane to plane:
-// one whose points and weights are those of the plane before, the plane itself aside, is listed as
-// that one, so the host packs and the device reads its points once.
-struct IBPlanes {
-    std::vector<int> begin;  // first point of every plane, and the list's end
-    std::vector<int> as;     // plane (of this list) that it repeats
-    bool flat = true;        // no point reaches into another plane
-};
-
-IBPlanes ib_planes(const cfd_ib_list* l) {
-    IBPlanes q;
-    auto id = [&](int p) { return l->idx + 9 * (size_t)p; };
-    for (int p = 0; p < l->n; ++p) {
-        const int32_t* x = id(p);
-        if (p == 0 || x[2] != id(p - 1)[2]) q.begin.push_back(p);
-        q.flat = q.flat && x[5] == x[2] && x[8] == x[2];
-    }
-    q.begin.push_back(l->n);
-    const int n = (int)q.begin.size() - 1;
-    for (int k = 0; k < n; ++k) {
-        q.as.push_back(k);
-        if (k == 0) continue;
-        const int b = q.begin[k], r = q.begin[q.as[k - 1]], m = q.begin[k + 1] - b;
-        bool same = m == q.begin[q.as[k - 1] + 1] - r &&
-                    std::memcmp(l->w + 3 * (size_t)b, l->w + 3 * (size_t)r, 3 * sizeof(double) * m) == 0;
-        for (int e = 0; same && e < m; ++e) {
-            const int32_t *x = id(b + e), *y = id(r + e);
-            same = x[0] == y[0] && x[1] == y[1] && x[3] == y[3] && x[4] == y[4] && x[6] == y[6] && x[7] == y[7];
-        }
-        if (same) q.as[k] = q.as[k - 1];
-    }
-    return q;
 }
 
 // Groups of z rows for k_ib_force_x.  Rows that a point ties together (its target and its two
@@ -1570,8 +1575,9 @@ int create_impl(const cfd_config* cfg, const cfd_ib_list* ibu, const cfd_ib_list
     CK(cudaMemcpy(c->scal, sc, sizeof(sc), cudaMemcpyHostToDevice));
 
     // immersed boundaries
-    if ((s = setup_ib(c, ibu, d.ju0, d.ju1, c->ibu, "ibu")) != CFD_OK) return s;
-    if ((s = setup_ib(c, ibv, d.jv0, d.jv1, c->ibv, "ibv")) != CFD_OK) return s;
+    IBPlanes pu, pv;
+    if ((s = setup_ib(c, ibu, d.ju0, d.ju1, c->ibu, pu, "ibu")) != CFD_OK) return s;
+    if ((s = setup_ib(c, ibv, d.jv0, d.jv1, c->ibv, pv, "ibv")) != CFD_OK) return s;
     const size_t nibu = (size_t)4 * c->ibu.npl, nibv = (size_t)2 * c->ibv.npl;
     const size_t hz = (size_t)d.ngal2 * d.nkx, hx = (size_t)d.ngal2 * d.ngal1;
     if (c->LZ2 >= 0 && c->RWIX2 && env_int("CFD_IB_GROUPS", 1, 0, 1)) {
@@ -1580,7 +1586,6 @@ int create_impl(const cfd_config* cfg, const cfd_ib_list* ibu, const cfd_ib_list
         std::vector<std::vector<int>> cu, cv;
         const auto* kx = line_kernels<float2>(d.ngal1);
         const int lx = ib_pitch(kx->n1, kx->n2);
-        const IBPlanes pu = ibu ? ib_planes(ibu) : IBPlanes(), pv = ibv ? ib_planes(ibv) : IBPlanes();
         if ((!ibu || ib_components(ibu, pu, d.ngal2, cu)) && (!ibv || ib_components(ibv, pv, d.ngal2, cv))) {
             size_t best = 0;
             for (int rw : {8, 6, 4, 2}) {
