@@ -360,6 +360,7 @@ size_t xline2_smem(int n1s, int n2s, int rw, size_t esz) {
 // contexts launch with sizes of their own, so it is raised and never lowered.
 template <typename F>
 cudaError_t smem_limit(F* f, int bytes) {
+    if (bytes <= 40 * 1024) return cudaSuccess;  // (48 KB with the static part are every kernel's)
     static std::mutex mu;
     std::lock_guard<std::mutex> hold(mu);
     cudaFuncAttributes a;
