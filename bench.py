@@ -85,7 +85,7 @@ def kernel_bytes(name, setup, mixed):
     # (`nact` of them) make the round trip; the inverse reads the half-physical rows of the
     # right-hand side and of the velocity and writes both physical rows, the forward reads
     # the forced right-hand side row and writes its half-physical row.
-    ib = []
+    ib, grp = [], 0
     for npl, nb, lst in ((nplu, 2, setup.ibu), (nplv, 1, setup.ibv)):
         if npl:
             nact = int(np.unique(lst.idx[:, [1, 4, 7]]).size) if lst.n else 0
@@ -98,9 +98,15 @@ def kernel_bytes(name, setup, mixed):
                        "k_ib_zfwd": npl * nb * (hpl * ct + ncol * cs),
                        "k_ib_xinv2": xi(nact), "k_ib_xfwd2": xf(nact),          # active rows
                        "k_ib_xinv": xi(cfg.ngal2), "k_ib_xfwd": xf(cfg.ngal2)})  # every row
+            # forcing in row groups, one launch for u, w and v: the active rows of right-hand side
+            # and velocity read, those of the right-hand side written, and 16 bytes a point
+            grp += nb * (npl * nact * 3 * cfg.nkx * ct + lst.n * 16)
     for k in ("k_ib_force", "k_ib_zinv", "k_ib_zfwd", "k_ib_xinv2", "k_ib_xfwd2", "k_ib_xinv", "k_ib_xfwd"):
         if ib:
             b[k] = sum(x[k] for x in ib) / len(ib)
+    if ib:
+        b["k_ib_zin"] = b["k_ib_zout"] = (2 * nplu + nplv) * (ncol * cs + hpl * ct)
+        b["k_ib_force_x"] = grp
     if name in b:
         return b[name]
     return b.get(name[:-1]) if name.endswith("2") else None

@@ -1,8 +1,8 @@
 // stats_kernels.cuh - FP64 statistics and CFL maxima on physical planes (sm_100a).
 //
 // Lengths with two-step transforms go through k_st_z and k_st_x (field_lines.cuh), whose partial
-// sums k_st_fin_lines and k_st_fold add up: 10.9 -> 2.8 ms for a call with conditional sums and 8.1 ->
-// 1.0 ms for a CFL query at 384 x 257(+90) x 384.  What follows describes the other lengths.
+// sums k_st_fin_lines and k_st_fold add up: 10.9 -> 3.0 ms for a call with conditional sums and 8.1 ->
+// 1.15 ms for a CFL query at 384 x 257(+90) x 384.  What follows describes the other lengths.
 //
 // The statistics pass of the reference (stats.f90:1-253, called from nonlinear at kRK = 1,
 // FOU3D.f90:187-217) and dtc_calc (FOU3D.f90:516-544) work on physical planes of

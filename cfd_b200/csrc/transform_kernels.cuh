@@ -1484,7 +1484,7 @@ __host__ __device__ constexpr int ib_pitch(int n1, int n2) { return (n1 * (n2 + 
 // grid: x = group, y = plane, z = right-hand side (u, w, v).  RW lines, RW even, at most 8.
 // Against the four launches it stands for on either grid (inverse x of right-hand sides and
 // velocities to memory, forcing, forward x), microseconds a substep with their z passes on B200: 384 x
-// 257(+90) x 384 FP32 285 -> 178, FP64 549 -> 317; 64 x 97(+56) x 64 FP64 31 -> 15 and ten launches to
+// 257(+90) x 384 FP32 285 -> 177, FP64 549 -> 311; 64 x 97(+56) x 64 FP64 31 -> 15 and ten launches to
 // three.
 template <typename T2, int TN1, int TN2>
 __global__ void __launch_bounds__(((sizeof(T2) == 8 ? 16 : 8) * (TN1 > TN2 ? TN1 : TN2) + 31) / 32 * 32, sizeof(T2) == 8 ? 0 : ((TN1 > TN2 ? TN1 : TN2) <= 24 ? 3 : 2))
