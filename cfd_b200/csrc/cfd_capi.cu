@@ -823,7 +823,7 @@ int col_table(cfd_ctx* c, const cfd_config* cfg) {
     }
     AL(c->coltab, double, h.size());
     CK(cudaMemcpy(c->coltab, h.data(), sizeof(double) * h.size(), cudaMemcpyHostToDevice));
-    CK(col_prepare(m, c->mb));
+    CK(col_prepare(m, c->colC, c->mb));
     ColMaps &a = c->colmap, &b = c->colmap_p;
     const int nu = d.nyu, nv = d.nyv, np = d.nyp;
     const struct { CUtensorMap* map; const void* f; int n; } all[] = {

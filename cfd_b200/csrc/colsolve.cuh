@@ -510,7 +510,7 @@ __global__ void __launch_bounds__(32) k_meanflow_warp(Dims d, Geo g, double beta
 
 // Host side (colsolve.cu; the _mb forms in colsolve_mb.cu): m rows per lane, cols columns a group
 // (4 in three bands), mb three bands
-cudaError_t col_prepare(int m, bool mb);  // raises the shared-memory limit of the kernels
+cudaError_t col_prepare(int m, int cols, bool mb);  // raises the shared-memory limit of the kernels
 cudaError_t col_prepare_mb(int m);
 // tensor map of a field of n planes; false if it cannot be made
 bool col_map(CUtensorMap* map, const void* field, int ncol, int n, int m, int cols);

@@ -26,20 +26,23 @@ namespace cfd {
 
 // m rows per lane, groups of cols columns, one band or three
 template <bool MB>
-static cudaError_t prepare(int m) {
+static cudaError_t prepare(int m, int cols) {
     cudaError_t e = cudaSuccess;
     auto set = [&](auto* f, size_t n) {
         if (e == cudaSuccess) e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)n);
     };
     COL_SWITCH(m, {
+        if constexpr (MR <= 15 && !MB) {
+            if (cols == 8) {
+                set(k_col_solve<MR, 8, 7, MB>, col_smem(MR, 8));
+                set(k_col_solve<MR, 8, 1, MB>, col_smem(MR, 8));
+                set(k_col_solve<MR, 8, 2, MB>, col_smem(MR, 8));
+                return e;
+            }
+        }
         set(k_col_solve<MR, 4, 7, MB>, col_smem(MR, 4));
         set(k_col_solve<MR, 4, 1, MB>, col_smem(MR, 4));
         set(k_col_solve<MR, 4, 2, MB>, col_smem(MR, 4));
-        if constexpr (MR <= 15 && !MB) {
-            set(k_col_solve<MR, 8, 7, MB>, col_smem(MR, 8));
-            set(k_col_solve<MR, 8, 1, MB>, col_smem(MR, 8));
-            set(k_col_solve<MR, 8, 2, MB>, col_smem(MR, 8));
-        }
     });
     return e;
 }

@@ -3,7 +3,7 @@
 
 namespace cfd {
 
-cudaError_t col_prepare_mb(int m) { return prepare<true>(m); }
+cudaError_t col_prepare_mb(int m) { return prepare<true>(m, 4); }
 
 void col_launch_mb(int mode, int m, int nsm, cudaStream_t st, const Dims& d, const Geo& g, const ColMaps& maps,
                    const ColArgs& a) {
