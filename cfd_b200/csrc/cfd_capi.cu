@@ -348,6 +348,11 @@ int tune_int(int32_t cfd_tuning::*field, const char* env, int dflt, int lo, int 
     return env_int(env, dflt, lo, hi);
 }
 
+// shared memory of a two-step z kernel: the exchange of its lines (exch_row) and the twiddles
+size_t z_lines_smem(int n1s, int n2s, int lines, size_t esz) {
+    return ((size_t)lines * ((n1s * (n2s + 1)) | 1) + (size_t)n1s * n2s) * esz;
+}
+
 size_t xline2_smem(int n1s, int n2s, int rw, size_t esz) {
     const int N = n1s * n2s;
     const int L1 = n1s * (n2s + 1) + 1, L2 = n2s * (n1s + 1) + 1, LU = N + 1;
@@ -396,6 +401,12 @@ int set_smem_attrs(cfd_ctx* c) {
     if (c->LZ2 >= 0) {
         const auto* k = line_kernels<T2>(n2);
         const auto* kn = line_kernels<T2>(n2, c->ZALT);
+        // the launches use these sizes with these kernels: a size taken from another split would let
+        // the last lines of a CTA reach past its shared memory
+        const int nl = 1 << c->LZ2;
+        if (c->SMZ2 < z_lines_smem(k->n1, k->n2, nl, esz) || c->SMZN < z_lines_smem(kn->n1, kn->n2, nl, esz) ||
+            c->NTZ2 < nl * std::max(k->n1, k->n2) || c->NTZN < nl * std::max(kn->n1, kn->n2))
+            return fail(c, CFD_ERR_SIZE, "z launch shape of Ngal2=%d does not cover its split %d x %d", n2, kn->n1, kn->n2);
         set(k->zinv2, c->SMZ2);
         set(k->ib_zinv, c->SMZ2);
         set(k->ib_zfwd, c->SMZ2);
@@ -1432,12 +1443,25 @@ int create_impl(const cfd_config* cfg, const cfd_ib_list* ibu, const cfd_ib_list
             const int lb = zl ? ilog2(zl) : env_int("CFD_ZLINES_LOG2", z768 ? (mixed ? 3 : 2) : (mixed ? 4 : 3), 2, 4);
             c->LZ2 = lb;
             c->NTZ2 = (1 << lb) * std::max(n1s, n2s);
-            c->SMZ2 = ((size_t)(1 << lb) * ((n1s * (n2s + 1)) | 1) + (size_t)n1s * n2s) * esz;
-            c->NTZN = c->NTZ2;
-            c->SMZN = c->SMZ2;
+            c->SMZ2 = z_lines_smem(n1s, n2s, 1 << lb, esz);
         }
     }
     if (c->LZ2 < 0) c->RW2 = 0;  // the two-step x-line kernels read the output of k_zinv2s
+    if (c->mb) {
+        // Three bands: a z pass that interpolates (k_zinv2), the x-line pass on interpolated planes
+        // (k_xline2b, or k_xline for x lengths without a two-step split) and k_zfwd2, one launch a
+        // band.  They transform whole planes of their own, so no x-line path that reads the
+        // z-transformed fields (RW2) runs, and with it none of the choices below that hang on RW2:
+        // the forcing's z passes (k_ib_zin, k_ib_zout) keep the plain split too.
+        c->RW2 = 0; c->XL3 = false; c->RW4 = 0;
+        int n1s = 0, n2s = 0;
+        line_split(cfg->ngal2_mid, n1s, n2s);
+        if (!band_length(cfg->ngal2) || !band_length(cfg->ngal2_mid))
+            return fail(c, CFD_ERR_SIZE, "three bands need two-step z lengths (64, 96, 128, 192, 384, 768) in both");
+        c->NTZm = (1 << c->LZ2) * std::max(n1s, n2s);
+        c->SMZm = z_lines_smem(n1s, n2s, 1 << c->LZ2, esz);
+        while (c->RWx > 1 && (cfg->ngal2_mid % c->RWx)) c->RWx /= 2;
+    }
     if (!c->RW2) c->RW4 = 0;
     c->XALT = c->RW2 && xalt;  // (xalt implies path 1: neither k_xline3 nor k_xline4)
     c->XR64 = c->RW2 && !c->XL3 && !c->RW4 && mixed && named && xpath == 5;
@@ -1480,14 +1504,14 @@ int create_impl(const cfd_config* cfg, const cfd_ib_list* ibu, const cfd_ib_list
     // FP64 z kernels at 112 registers (3 CTAs of 8 lines per SM): measured 0.31 / 0.59 against
     // 0.34 / 0.61 ms per launch at re550; the 768-point split spills at that cap
     c->ZR = c->RW2 && c->precision == CFD_PREC_FP64 && d.ngal2 <= 384 && env_int("CFD_Z_R112", 1, 0, 1);
-    if (c->RW2 && c->LZ2 >= 0 && tune_int(&cfd_tuning::zsplit, "CFD_ZSPLIT", z768 || d.ngal2 == 192 ? 2 : 1, 1, 2) == 2) {
+    if (c->LZ2 >= 0) {
         int n1s = 0, n2s = 0;
         line_split(d.ngal2, n1s, n2s, true);
-        if (n1s) {
-            c->ZALT = true;
-            c->NTZN = (1 << c->LZ2) * std::max(n1s, n2s);
-            c->SMZN = ((size_t)(1 << c->LZ2) * ((n1s * (n2s + 1)) | 1) + (size_t)n1s * n2s) * esz;
-        }
+        c->ZALT = n1s && c->RW2 &&
+                  tune_int(&cfd_tuning::zsplit, "CFD_ZSPLIT", z768 || d.ngal2 == 192 ? 2 : 1, 1, 2) == 2;
+        line_split(d.ngal2, n1s, n2s, c->ZALT);
+        c->NTZN = (1 << c->LZ2) * std::max(n1s, n2s);
+        c->SMZN = z_lines_smem(n1s, n2s, 1 << c->LZ2, esz);
     }
     {
         int n1s = 0, n2s = 0;
@@ -1504,18 +1528,6 @@ int create_impl(const cfd_config* cfg, const cfd_ib_list* ibu, const cfd_ib_list
             }
             if (!c->RWIX2 || !c->RWFX2) c->RWIX2 = c->RWFX2 = 0;
         }
-    }
-    if (c->mb) {
-        // three bands: the per-slot interpolating z pass, the Stockham x-line kernel and the
-        // two-step forward z pass, launched once per band; thread-per-column solves
-        c->RW2 = 0; c->XL3 = false; c->RW4 = 0; c->XALT = c->ZALT = false; c->XR64 = false; c->ZR = false;
-        int n1s = 0, n2s = 0;
-        line_split(cfg->ngal2_mid, n1s, n2s);
-        if (!band_length(cfg->ngal2) || !band_length(cfg->ngal2_mid))
-            return fail(c, CFD_ERR_SIZE, "three bands need two-step z lengths (64, 96, 128, 192, 384, 768) in both");
-        c->NTZm = (1 << c->LZ2) * std::max(n1s, n2s);
-        c->SMZm = ((size_t)(1 << c->LZ2) * ((n1s * (n2s + 1)) | 1) + (size_t)n1s * n2s) * esz;
-        while (c->RWx > 1 && (cfg->ngal2_mid % c->RWx)) c->RWx /= 2;
     }
     int s = mixed ? set_smem_attrs<float2>(c) : set_smem_attrs<double2>(c);
     if (s != CFD_OK) return s;
