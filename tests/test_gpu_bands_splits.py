@@ -10,7 +10,7 @@ pytestmark = pytest.mark.gpu
 STAGES = ("rhs0", "nonlinear", "solve_uvw", "meanflow", "solve_p", "vcorr")
 FIELDS = ("u1", "u2", "u3", "p", "du1", "du2", "du3", "nu1", "nu2", "nu3")
 CASES = [(dict(ngal1=48, ngal2=192, ny=29, band_vface=5, ngal1_mid=24, ngal2_mid=96), None),
-         (dict(ngal1=24, ngal2=768, ny=29, band_vface=5, ngal1_mid=16, ngal2_mid=64), None),
+         (dict(ngal1=96, ngal2=768, ny=17, band_vface=4, ngal1_mid=48, ngal2_mid=64, cyl_diameter=0.1, cyl_spacing=0.5), None),
          (dict(ngal1=48, ngal2=96, ny=29, band_vface=5, ngal1_mid=24, ngal2_mid=64), dict(zsplit=2, zlines=16))]
 
 
@@ -26,7 +26,7 @@ def test_forced_bands(kw, tuning):
     from cfd_b200.channel import Channel, build_channel
     from cfd_b200.config import tiny
     from oracle.oracle import OracleChannel
-    s = build_channel(tiny(cyl_diameter=0.3, cyl_spacing=1.5, seed=9, **kw))
+    s = build_channel(tiny(**{"cyl_diameter": 0.3, "cyl_spacing": 1.5, "seed": 9, **kw}))
     assert s.ibu.n > 0 and s.ibv.n > 0
     g, o = Channel(s, precision="fp64", tuning=tuning), OracleChannel(s)
     assert g.tuning()["zsplit"] == 1
