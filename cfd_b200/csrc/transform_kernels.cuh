@@ -1509,7 +1509,10 @@ __global__ void __launch_bounds__(((sizeof(T2) == 8 ? 16 : 8) * (TN1 > TN2 ? TN1
     // ---- inverse: line b = rhs + i u of row b
     if (t < RW * TN2) {
         const int b = t / TN2, n2 = t - b * TN2;
+        // a line past the group's last row is zero: it travels with a row of the group in the forward
+        // step, and any other row may be written by its own group meanwhile
         const int row = rows[b];
+        const bool live = row >= 0;
         const T2 *A = Hr + (size_t)max(row, 0) * NK, *C = Hu + (size_t)max(row, 0) * NK;
         T2 v[TN1];
 #pragma unroll
@@ -1518,11 +1521,11 @@ __global__ void __launch_bounds__(((sizeof(T2) == 8 ? 16 : 8) * (TN1 > TN2 ? TN1
             const bool lo = (e0 + TN2 - 1 <= HX) || (e0 <= HX && e <= HX);
             const bool hi = (e0 >= N - HX) || (e0 + TN2 - 1 >= N - HX && e >= N - HX);
             T2 val = cx<T2>((R)0, (R)0);
-            if (lo) {
+            if (lo && live) {
                 T2 x = A[e], c = C[e];
                 if (n1 == 0 && n2 == 0) { x.y = 0; c.y = 0; }
                 val = cx<T2>(x.x - c.y, x.y + c.x);
-            } else if (hi) {
+            } else if (hi && live) {
                 const T2 x = A[N - e], c = C[N - e];
                 val = cx<T2>(x.x + c.y, -x.y + c.x);
             }
