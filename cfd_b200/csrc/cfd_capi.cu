@@ -100,6 +100,10 @@ struct cfd_ctx {
     int nsm = 1;            // SMs of the device (CTAs of the persistent kernels)
     double* coltab = nullptr;
     cfd::ColMaps colmap, colmap_p;  // of the solves and of cfd_solve_p
+    // set by k_col_solve (mapped host memory) when a transfer did not arrive: the fields are undefined
+    // until a state is uploaded again
+    int *col_err = nullptr, *col_err_dev = nullptr;
+    int col_tries = cfd::kWaitTries;
     double* scal = nullptr;
     double* mf_work = nullptr;
     double2* stage0 = nullptr;
@@ -235,6 +239,13 @@ int cuda_check(cfd_ctx* c, cudaError_t e, const char* what) {
     return CFD_OK;
 }
 
+// whether every column solve so far (of those the host has waited for) got its columns
+int solves_complete(cfd_ctx* c) {
+    if (c->col_err && *(volatile int*)c->col_err)
+        return fail(c, CFD_ERR_CUDA, "a transfer of the column solves did not complete: the fields are undefined");
+    return CFD_OK;
+}
+
 #define CK(call)                                                   \
     do {                                                           \
         int _s = cuda_check(c, (call), #call);                     \
@@ -332,6 +343,8 @@ bool band_length(int n) { return n == 64 || n == 96 || n == 128 || n == 192 || n
 //   CFD_XLINE_STOCKHAM 1: nonlinear through the Stockham x-line kernel and per-slot z pass
 //   CFD_XLINE_PATH   3: packed two-step x-line kernel (1.5 inverse lines per row)
 //   CFD_SOLVE_GROUP  columns of a group of the warp-per-column solves (4 or 8)
+//   CFD_SOLVE_TRIES  limit of their waits for a transfer (0: every wait runs out at once, and the
+//                    call that synchronises next reports it)
 //   CFD_RHS_CHUNK    y-planes per thread of the right-hand-side kernel (2..64)
 int env_int(const char* name, int dflt, int lo, int hi) {
     const char* v = std::getenv(name);
@@ -799,7 +812,8 @@ int col_solve(cfd_ctx* c, int mode, int krk, const char* name) {
     a.dtirk = (1.0 / c->dt) / ab;
     a.dtrk = c->dt * ab;
     a.mean_diag = c->mean_diag;
-    a.err = c->scal + 3;
+    a.err = c->col_err_dev;
+    a.tries = c->col_tries;
     a.ahead = col_ahead(c->colC, c->d.ncol);
     prof_mark(c);
     col_launch(mode, c->colM, c->colC, c->mb, c->nsm, c->stream, c->d, c->g, mode == 2 ? c->colmap_p : c->colmap, a);
@@ -835,6 +849,10 @@ int col_table(cfd_ctx* c, const cfd_config* cfg) {
     AL(c->coltab, double, h.size());
     CK(cudaMemcpy(c->coltab, h.data(), sizeof(double) * h.size(), cudaMemcpyHostToDevice));
     CK(col_prepare(m, c->colC, c->mb));
+    CK(cudaHostAlloc((void**)&c->col_err, sizeof(int), cudaHostAllocMapped));
+    *c->col_err = 0;
+    CK(cudaHostGetDevicePointer((void**)&c->col_err_dev, c->col_err, 0));
+    c->col_tries = env_int("CFD_SOLVE_TRIES", kWaitTries, 0, kWaitTries);
     ColMaps &a = c->colmap, &b = c->colmap_p;
     const int nu = d.nyu, nv = d.nyv, np = d.nyp;
     const struct { CUtensorMap* map; const void* f; int n; } all[] = {
@@ -979,7 +997,7 @@ int check_krk(cfd_ctx* c, int krk) {
     if (!c) return CFD_ERR_ARG;
     if (krk < 1 || krk > 3) return fail(c, CFD_ERR_ARG, "krk must be 1..3 (got %d)", krk);
     if (!c->state_loaded) return fail(c, CFD_ERR_STATE, "state not uploaded");
-    return CFD_OK;
+    return solves_complete(c);
 }
 
 struct FieldInfo {
@@ -1949,6 +1967,7 @@ int cfd_destroy(cfd_ctx* c) {
             if (c->xev[f][k]) cudaEventDestroy(c->xev[f][k]);
     if (c->xin) cudaStreamDestroy(c->xin);
     if (c->xout) cudaStreamDestroy(c->xout);
+    if (c->col_err) cudaFreeHost(c->col_err);
     if (c->ev_fork) cudaEventDestroy(c->ev_fork);
     if (c->ev_join) cudaEventDestroy(c->ev_join);
     if (c->side) cudaStreamDestroy(c->side);
@@ -1971,7 +1990,7 @@ int cfd_set_stream(cfd_ctx* c, void* stream) {
 int cfd_synchronize(cfd_ctx* c) {
     if (!c) return CFD_ERR_ARG;
     CK(cudaStreamSynchronize(c->stream));
-    return CFD_OK;
+    return solves_complete(c);
 }
 
 int cfd_field_shape(const cfd_ctx* c, int32_t field, int64_t* ncomplex, int32_t* j0, int32_t* nplanes, int32_t* ncolumns) {
@@ -2025,6 +2044,10 @@ int cfd_upload_field(cfd_ctx* c, int32_t field, const double* host, int32_t layo
     if (layout != CFD_LAYOUT_REF && layout != CFD_LAYOUT_PLANE) return fail(c, CFD_ERR_ARG, "bad layout %d", layout);
     CK(cudaSetDevice(c->device));
     if (field <= CFD_FIELD_U3) c->hx_valid = false;  // the nonlinear pass's transforms are stale
+    if (field <= CFD_FIELD_P && c->col_err && *(volatile int*)c->col_err) {  // a new state begins
+        CK(cudaStreamSynchronize(c->stream));
+        *c->col_err = 0;
+    }
     const size_t n = (size_t)fi.nplanes * c->d.ncol;
     if (layout == CFD_LAYOUT_REF && field <= CFD_FIELD_P && !fi.single) {
         int s = xfer_ready(c, field);
@@ -2077,6 +2100,7 @@ int cfd_download_field(cfd_ctx* c, int32_t field, double* host, int32_t layout) 
     FieldInfo fi;
     if (!field_info(c, field, fi)) return fail(c, CFD_ERR_ARG, "bad field %d", field);
     if (layout != CFD_LAYOUT_REF && layout != CFD_LAYOUT_PLANE) return fail(c, CFD_ERR_ARG, "bad layout %d", layout);
+    if (int s = solves_complete(c)) return s;
     CK(cudaSetDevice(c->device));
     const size_t n = (size_t)fi.nplanes * c->d.ncol;
     const double2* src = (const double2*)fi.ptr;
@@ -2229,7 +2253,7 @@ int cfd_get_scalars(cfd_ctx* c, double* mpgx, double* qx, double* dgx) {
     if (mpgx) *mpgx = h[0];
     if (qx) *qx = h[1];
     if (dgx) *dgx = h[2];
-    if (h[3] != 0.0) return fail(c, CFD_ERR_CUDA, "a transfer of the column solves did not complete");
+    if (int s = solves_complete(c)) return s;
     if (!std::isfinite(h[0]) || !std::isfinite(h[1]) || !std::isfinite(h[2]))
         return fail(c, CFD_ERR_NONFINITE, "non-finite mean-flow scalars (mpgx %g, Qx %g)", h[0], h[1]);
     return CFD_OK;
@@ -2254,6 +2278,7 @@ int cfd_divergence_max(cfd_ctx* c, double* errmax) {
         m = std::max(m, v);
     }
     *errmax = bad ? NAN : m;
+    if (int s2 = solves_complete(c)) return s2;
     if (bad) return fail(c, CFD_ERR_NONFINITE, "non-finite divergence");
     return CFD_OK;
 }
@@ -2337,7 +2362,8 @@ int cfd_stats_reset(cfd_ctx* c) {
 int cfd_stats_accumulate(cfd_ctx* c) {
     if (!c) return CFD_ERR_ARG;
     if (!c->st.on) return fail(c, CFD_ERR_STATE, "statistics not configured");
-    int s = stats_pass(c, true);
+    int s = solves_complete(c);
+    if (!s) s = stats_pass(c, true);
     if (s) return s;
     auto& st = c->st;
     if (st.spu) {
@@ -2358,6 +2384,7 @@ int cfd_spectra_read(cfd_ctx* c, double* spu, double* spv, double* spw, double* 
     auto& st = c->st;
     if (!st.on || !st.spu) return fail(c, CFD_ERR_STATE, "spectra not configured");
     CK(cudaStreamSynchronize(c->stream));
+    if (int e = solves_complete(c)) return e;
     // device [plane][column] -> the reference's sp(j,column), j fastest
     std::vector<double> h;
     auto get = [&](double* out, const double* dev, int ny) -> int {
@@ -2384,6 +2411,7 @@ int cfd_stats_read(cfd_ctx* c, double* u_sums, double* v_sums, double* p_sums, d
     auto& st = c->st;
     if (!st.on) return fail(c, CFD_ERR_STATE, "statistics not configured");
     CK(cudaStreamSynchronize(c->stream));
+    if (int e = solves_complete(c)) return e;
     if (u_sums) CK(cudaMemcpy(u_sums, st.su, sizeof(double) * 6 * d.nyu, cudaMemcpyDeviceToHost));
     if (v_sums) CK(cudaMemcpy(v_sums, st.sv, sizeof(double) * 5 * d.nyv, cudaMemcpyDeviceToHost));
     if (p_sums) CK(cudaMemcpy(p_sums, st.sp, sizeof(double) * 2 * d.nyp, cudaMemcpyDeviceToHost));
@@ -2506,6 +2534,7 @@ int cfd_ensemble_step(cfd_ensemble* e, int32_t nsteps) {
     bool stale = !e->gexec;
     for (size_t i = 0; i < e->m.size(); ++i) {
         if (!e->m[i]->state_loaded) return efail(e, CFD_ERR_STATE, "member %zu has no state", i);
+        if (int s = solves_complete(e->m[i])) return efail(e, s, "member %zu: %s", i, e->m[i]->err.c_str());
         if (e->m[i]->epoch != e->epochs[i]) stale = true;
     }
     // the members' pending work comes first
@@ -2527,6 +2556,8 @@ int cfd_ensemble_step(cfd_ensemble* e, int32_t nsteps) {
 int cfd_ensemble_synchronize(cfd_ensemble* e) {
     if (!e) return CFD_ERR_ARG;
     ECK(cudaStreamSynchronize(e->master));
+    for (size_t i = 0; i < e->m.size(); ++i)
+        if (int s = solves_complete(e->m[i])) return efail(e, s, "member %zu: %s", i, e->m[i]->err.c_str());
     return CFD_OK;
 }
 
@@ -2583,6 +2614,7 @@ int cfd_cfl(cfd_ctx* c, double* dtc, double* terms) {
     if (s) return s;
     std::vector<double> h((size_t)3 * d.nyu);
     CK(cudaStreamSynchronize(c->stream));  // the pass runs on the (non-blocking) context stream
+    if ((s = solves_complete(c))) return s;
     CK(cudaMemcpy(h.data(), c->st.mx, sizeof(double) * h.size(), cudaMemcpyDeviceToHost));
     double um = 0.0, wm = 0.0, vm = 1e-6;
     bool bad = false;

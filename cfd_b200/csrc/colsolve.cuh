@@ -61,10 +61,10 @@ __host__ __device__ constexpr int col_groups(int m, int cols) {
 }
 __host__ __device__ constexpr int col_tab_elems(int m) { return 32 * m * kColTabs; }
 // bytes of a field's rows of one group (16 a column, 32 M rows) and of the CTA's shared memory:
-// the groups' u, w, v rows, the table, two barriers a group
+// the groups' u, w, v rows, the table, two barriers and four words a group
 __host__ __device__ constexpr int col_region(int m, int cols) { return 32 * m * cols * 16; }
 __host__ __device__ constexpr size_t col_smem(int m, int cols) {
-    return (size_t)col_groups(m, cols) * 3 * col_region(m, cols) + (size_t)col_tab_elems(m) * 8 + 64;
+    return (size_t)col_groups(m, cols) * 3 * col_region(m, cols) + (size_t)col_tab_elems(m) * 8 + 128;
 }
 // boxes a region arrives in: at most 256 rows each, a multiple of 8 (the swizzle's period)
 __host__ __device__ constexpr int col_boxes(int m) { return 32 * m <= 256 ? 1 : (32 * m <= 512 ? 2 : 4); }
@@ -172,9 +172,10 @@ __device__ __forceinline__ void mbar_init(unsigned bar, int n) {
 __device__ __forceinline__ void mbar_expect(unsigned bar, int bytes) {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
 }
-// true when the phase has completed; gives up after about a second
-__device__ __forceinline__ bool mbar_wait(unsigned bar, unsigned parity) {
-    for (int k = 0; k < (1 << 20); ++k) {
+// true when the phase has completed; gives up after `tries` tries (kWaitTries: about a second)
+constexpr int kWaitTries = 1 << 20;
+__device__ __forceinline__ bool mbar_wait(unsigned bar, unsigned parity, int tries) {
+    for (int k = 0; k < tries; ++k) {
         unsigned ok;
         asm volatile(
             "{\n.reg .pred q;\nmbarrier.try_wait.parity.shared::cta.b64 q, [%1], %2, 1000;\nselp.b32 %0, 1, 0, q;\n}\n"
@@ -184,6 +185,12 @@ __device__ __forceinline__ bool mbar_wait(unsigned bar, unsigned parity) {
         if (ok) return true;
     }
     return false;
+}
+// The wait of a group's threads.  Each may find the limit by itself, so none leaves here: one that
+// gives up sets *gave, and the group reads that after its next barrier and leaves as one.  Waits
+// that a barrier apart may still be read take words of their own.
+__device__ __forceinline__ void group_wait(unsigned bar, unsigned parity, int tries, volatile int* gave) {
+    if (!mbar_wait(bar, parity, tries)) *gave = 1;
 }
 __device__ __forceinline__ void tma_load(unsigned dst, const CUtensorMap* m, int x, int y, unsigned bar) {
     asm volatile("cp.async.bulk.tensor.2d.shared::cta.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(dst),
@@ -210,7 +217,8 @@ struct ColArgs {
     double dtirk;       // 1 / (dt (a+b))
     double dtrk;        // dt (a+b)
     double mean_diag;   // bottom row of D.G at kx = kz = 0
-    double* err;        // set if a transfer did not arrive
+    int* err;           // (host memory) set if a transfer did not arrive
+    int tries;          // limit of the waits for one (kWaitTries)
     bool ahead;         // prefetch the next columns into L2 while these are solved
 };
 
@@ -233,12 +241,15 @@ __global__ void __launch_bounds__(32 * C * col_groups(M, C))
     double* stab = reinterpret_cast<double*>(col_smem_raw + G * 3 * RB);
     const unsigned sreg = smem_u32(reg);
     const unsigned bar = smem_u32(stab + col_tab_elems(M)) + 16 * grp, barp = bar + 8;
+    // a wait that was given up: [phase] the columns', [2 + phase] p's
+    volatile int* gave = reinterpret_cast<int*>(stab + col_tab_elems(M) + 8) + 4 * grp;
     const bool lead = t == 0;
     const int nq = (d.ncol + C - 1) / C, stride = G * gridDim.x;
     int q = blockIdx.x + grp * gridDim.x;
     if (lead) {
         mbar_init(bar, 1);
         mbar_init(barp, 1);
+        for (int k = 0; k < 4; ++k) gave[k] = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     for (int i = threadIdx.x; i < col_tab_elems(M); i += blockDim.x) stab[i] = A.tab[i];
@@ -287,8 +298,7 @@ __global__ void __launch_bounds__(32 * C * col_groups(M, C))
         const bool sh = MB && !mb_long(d, col % d.nkx, col / d.nkx);  // a short column
         // the weight of the face above p row r (0 at the ends of the column or segment)
         auto face = [&](int i, int r) { return MB && sh && r >= bu - 2 && r < tu ? 0.0 : T(i, 7); };
-        ok = mbar_wait(bar, phase);
-        if (!ok) break;
+        group_wait(bar, phase, A.tries, gave + phase);
         if (lead) {
             if (PRE) prefetch(&maps.p, q);
             if (A.ahead && q + stride < nq)
@@ -416,6 +426,11 @@ __global__ void __launch_bounds__(32 * C * col_groups(M, C))
         }
         publish();
         group_sync();
+        if (gave[phase]) {  // nothing is stored; the copies still under way end before the CTA does
+            if (lead) mbar_wait(bar, phase, kWaitTries);
+            ok = false;
+            break;
+        }
         if (lead) {
 #pragma unroll
             for (int f = 0; f < (MODE == 2 ? 2 : 3); ++f) store(f, &maps.dst[f], q);
@@ -432,12 +447,22 @@ __global__ void __launch_bounds__(32 * C * col_groups(M, C))
             }
         }
         if constexpr (PRE) {
-            ok = mbar_wait(barp, phase);
-            if (!ok) break;
+            group_wait(barp, phase, A.tries, gave + 2 + phase);
 #pragma unroll
             for (int i = 0; i < M; ++i) R(0, i) = dadd(R(0, i), ps[0][i]);
             publish();
             group_sync();
+            if (gave[2 + phase]) {
+                if (lead) {
+                    mbar_wait(barp, phase, kWaitTries);
+                    if (q + stride < nq) {  // (u completes the next columns' bytes)
+                        load(0, &maps.src[0], q + stride, bar);
+                        mbar_wait(bar, phase ^ 1, kWaitTries);
+                    }
+                }
+                ok = false;
+                break;
+            }
             if (lead) {
                 store(0, &maps.p, q);
                 read_out();
@@ -445,7 +470,10 @@ __global__ void __launch_bounds__(32 * C * col_groups(M, C))
             }
         }
     }
-    if (!ok && lead) *A.err = 1.0;
+    if (!ok && lead) {
+        *A.err = 1;
+        __threadfence_system();
+    }
     if (lead) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
 }
 
