@@ -27,6 +27,16 @@ KNOBS = ((("xline_path", "xsplit"), ((6, 1), (1, 1), (1, 2), (5, 1), (5, 2), (2,
 # x-line paths that only FP32-mixed contexts run (FP64 contexts asked for them run path 1)
 MIXED_ONLY_XLINE = (4, 5, 6)
 
+# lengths at which the library interpolates in FP32 by default in FP32-mixed contexts; the march
+# does so at every length, so elsewhere the search, which nobody asked for less precision,
+# leaves it out
+NAMED = (64, 96, 128, 192, 384, 768)
+
+
+def keeps_precision(setup, tuning) -> bool:
+    return setup is None or tuning.get("xline_path") != 6 or (setup.cfg.ngal1 in NAMED and setup.cfg.ngal2 in NAMED)
+
+
 # knobs that only act with another setting (the library reports them as 0 or 1 otherwise)
 RELEVANT = {"xline_rows": lambda t: t.get("xline_path") != 2,
             "zsplit": lambda t: t.get("xline_path") in (1, 5, 6)}
@@ -73,6 +83,8 @@ def autotune(setup, precision: str, device: int = 0, steps: int = 5, log=None):
                 continue
             cand = dict(best, **(dict(zip(name, v)) if isinstance(name, tuple) else {name: v}))
             if precision == "fp64" and cand.get("xline_path") in MIXED_ONLY_XLINE:
+                continue
+            if not keeps_precision(setup, cand):
                 continue
             k = json.dumps(cand, sort_keys=True)
             if k in tried:

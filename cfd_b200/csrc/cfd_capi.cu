@@ -134,6 +134,7 @@ struct cfd_ctx {
     float2 *twx_f = nullptr, *twz_f = nullptr;
     int CHz = 8, RWx = 4, RWib = 4, RWibf = 4;
     int RW2 = 0, NT2 = 0;
+    int RWD = 0;            // rows per CTA of k_xline2b on the planes of the whole channel (RW2 = 0)
     bool XL3 = false;       // packed two-step x-line kernel (k_xline3) instead of k_xline2
     bool XALT = false, ZALT = false;  // transposed two-step splits (x-line; nonlinear z kernels)
     bool XR64 = false;      // FP32 x-line kernel held to 64 registers (k_xline2r, path 5)
@@ -444,6 +445,7 @@ int set_smem_attrs(cfd_ctx* c) {
         if (c->RW4) set(line_kernels<T2>(n1)->xline4, c->SM4);
         if (c->XMRW) set(line_kernels<T2>(n1)->xmarch, c->SMXM);
     }
+    if (c->RWD) set(line_kernels<T2>(n1)->xline2b, xline2_smem(line_kernels<T2>(n1)->n1, line_kernels<T2>(n1)->n2, c->RWD, esz));
     if (c->mb && c->LZ2 >= 0) {
         const auto* k = line_kernels<T2>(c->dM.ngal2);
         const size_t smz = std::max(c->SMZ2, c->SMZm);
@@ -594,6 +596,12 @@ int nl_transforms(cfd_ctx* c) {
         xdone = true;
     }
     if (xdone) {
+    } else if (c->RWD) {
+        const auto* k = line_kernels<T2>(d.ngal1);
+        k->xline2b<<<dim3((d.ngal2 + c->RWD - 1) / c->RWD, d.nslot), (2 * c->RWD * std::max(k->n1, k->n2) + 31) / 32 * 32,
+                     xline2_smem(k->n1, k->n2, c->RWD, e), c->stream>>>(
+            d, c->g, (T2*)c->H[0], (T2*)c->H[1], (T2*)c->H[2], (T2*)c->H[3], twx<T2>(c), c->RWD, ilog2(c->RWD));
+        LK("k_xline2b");
     } else if (c->RW2 && c->XL3) {
         dim3 gx3(d.ngal2 / c->RW2, d.nslot);
         kx->xline3<<<gx3, c->NT2, c->SM3, c->stream>>>(d, c->g, (const T2*)c->Hx, (T2*)c->H[0], (T2*)c->H[1],
@@ -1402,7 +1410,17 @@ int create_impl(const cfd_config* cfg, const cfd_ib_list* ibu, const cfd_ib_list
         c->RWibf /= 2;
     if (d.ngal2 % c->RWibf) return fail(c, CFD_ERR_SIZE, "Ngal2 must be even");
     // the transposed split of the x-line transform (tuning xsplit = 2) is for path 1 only
-    const int xpath = g_tuning && g_tuning->xline_path ? g_tuning->xline_path : env_int("CFD_XLINE_PATH", mixed && d.ngal1 >= 256 && line_march_f32(d.ngal1) ? 6 : (mixed && d.ngal1 == 192 ? 5 : 1), 1, 6);
+    //
+    // FP32-mixed contexts interpolate in y in FP32, on transformed planes, only where both lengths are
+    // named ones, or where the caller asks for the march.  Everywhere else the FP64 fields are interpolated
+    // and rounded once (k_zinv2), and k_xline2b takes the planes (path 1): that costs a z transform per
+    // field and slot instead of one per plane, 144 x 108 x 131 a step of 302 -> 312 us.
+    const bool named2 = line_kernels_named<float2>(d.ngal1) && line_kernels_named<float2>(d.ngal2);
+    const bool march_asked = line_march_f32(d.ngal1) && std::getenv("CFD_XMARCH_STEPS");
+    const int xpath = g_tuning && g_tuning->xline_path
+                          ? g_tuning->xline_path
+                          : env_int("CFD_XLINE_PATH", !mixed ? 1 : (named2 ? (d.ngal1 == 384 ? 6 : (d.ngal1 == 192 ? 5 : 1))
+                                                                          : (march_asked ? 6 : 1)), 1, 6);
     // (the tuning variants exist for the six named lengths; the others run path 1)
     const bool named = line_kernels_named<float2>(d.ngal1) != nullptr;
     // (at 768 points the transposed splits are the default: FP32 x lines 24 * 32 in 8 rows 736 us
@@ -1480,15 +1498,12 @@ int create_impl(const cfd_config* cfg, const cfd_ib_list* ibu, const cfd_ib_list
         c->SMZm = z_lines_smem(n1s, n2s, 1 << c->LZ2, esz);
         while (c->RWx > 1 && (cfg->ngal2_mid % c->RWx)) c->RWx /= 2;
     }
-    if (!c->RW2) c->RW4 = 0;
-    c->XALT = c->RW2 && xalt;  // (xalt implies path 1: neither k_xline3 nor k_xline4)
-    c->XR64 = c->RW2 && !c->XL3 && !c->RW4 && mixed && named && xpath == 5;
-    // the x-line pass marching in y (one band).  FP32-mixed: x-line path 6, the default from 256 to 576
-    // points where the length has an 8- or 16-point second step, microseconds a launch against the
-    // per-slot kernels: 256 x 193 x 256 197 and 217, 288 225 and 308, 384 x 257 470 and 637, 432 x 193 492
-    // and 667, 512 772 and 996, 576 899 and 1084; 128 x 129 62 and 46.  FP64: path 1 takes it from 256 to
-    // 512 points: 256 332 and 345, 288 463 and 562, 384 x 257 947 and 1124, 432 1062 and 1273, 512 x 97 841
-    // and 1153; 192 x 193 230 and 232, 128 99 and 82.  Rows per CTA from xline_rows (2 or 4; FP64 2);
+    // the x-line pass marching in y (one band).  FP32-mixed: x-line path 6, the default at 384 points
+    // (microseconds a launch against the per-slot kernels, 384 x 257: 470 and 637; 128 x 129 62 and 46);
+    // on request where the length has an 8- or 16-point second step (256 x 193 x 256 197 and 217, 288 225
+    // and 308, 432 x 193 492 and 667, 512 772 and 996, 576 899 and 1084).  FP64: path 1 takes it from 256
+    // to 512 points: 256 332 and 345, 288 463 and 562, 384 x 257 947 and 1124, 432 1062 and 1273, 512 x 97
+    // 841 and 1153; 192 x 193 230 and 232, 128 99 and 82.  Rows per CTA from xline_rows (2 or 4; FP64 2);
     // emission steps per CTA from CFD_XMARCH_STEPS, by default the longest chunk that keeps 20 CTAs
     // per SM (re550: 16 steps, 0.621 ms per launch against 0.625-0.636 at 8, 12, 20 and 0.65 at 32;
     // re395: 8 steps)
@@ -1519,6 +1534,15 @@ int create_impl(const cfd_config* cfg, const cfd_ib_list* ibu, const cfd_ib_list
             }
         }
     }
+    if (mixed && !named2 && c->RW2 && !c->XMRW) {
+        const auto* k = line_kernels<float2>(d.ngal1);
+        c->RWD = 4;
+        while (c->RWD > 1 && xline2_smem(k->n1, k->n2, c->RWD, esz) > budget) c->RWD /= 2;
+        c->RW2 = 0; c->XL3 = false;
+    }
+    if (!c->RW2) c->RW4 = 0;
+    c->XALT = c->RW2 && xalt;  // (xalt implies path 1: neither k_xline3 nor k_xline4)
+    c->XR64 = c->RW2 && !c->XL3 && !c->RW4 && mixed && named && xpath == 5;
     // FP64 z kernels at 112 registers (3 CTAs of 8 lines per SM): measured 0.31 / 0.59 against
     // 0.34 / 0.61 ms per launch at re550; the 768-point split spills at that cap
     c->ZR = c->RW2 && c->precision == CFD_PREC_FP64 && d.ngal2 <= 384 && env_int("CFD_Z_R112", 1, 0, 1);
@@ -1942,8 +1966,8 @@ int cfd_create_tuned(const cfd_config* cfg, const cfd_ib_list* ibu, const cfd_ib
 
 int cfd_get_tuning(const cfd_ctx* c, cfd_tuning* t) {
     if (!c || !t) return CFD_ERR_ARG;
-    t->xline_path = c->RW2 ? (c->XMRW && c->precision == CFD_PREC_MIXED ? 6 : (c->RW4 ? 4 : (c->XL3 ? 3 : (c->XR64 ? 5 : 1)))) : 2;
-    t->xline_rows = c->XMRW && c->precision == CFD_PREC_MIXED ? c->XMRW : (c->RW4 ? c->RW4 : (c->RW2 ? c->RW2 : 0));
+    t->xline_path = c->RWD ? 1 : c->RW2 ? (c->XMRW && c->precision == CFD_PREC_MIXED ? 6 : (c->RW4 ? 4 : (c->XL3 ? 3 : (c->XR64 ? 5 : 1)))) : 2;
+    t->xline_rows = c->XMRW && c->precision == CFD_PREC_MIXED ? c->XMRW : (c->RW4 ? c->RW4 : (c->RWD ? c->RWD : c->RW2));
     t->zlines = c->LZ2 >= 0 ? (1 << c->LZ2) : 0;
     t->solve_kind = 1;
     t->solve_cols = c->SNT;

@@ -224,8 +224,8 @@ __global__ void __launch_bounds__(256) k_xline(Dims d, T2* __restrict__ H0, T2* 
 // The retained modes are kx = 0..N/3 (N1 = 2*(Ngal1/3)), a compile-time bound, so which
 // elements of a subsequence are zero, direct or conjugated is resolved at compile time
 // except in the two blocks that straddle a boundary.
-// DIRECT (three bands): u, w, v of every slot of the launch lie interpolated in H0, H1, H2 already,
-// and the products take their place (128-point rows of 128 x 97(+56) x 128 FP64: 36 -> 27 us a band
+// DIRECT (three bands; FP32-mixed at lengths that are not among the named six): u, w, v of every slot
+// of the launch lie interpolated in H0, H1, H2 already, and the products take their place (128-point rows of 128 x 97(+56) x 128 FP64: 36 -> 27 us a band
 // against the radix-by-radix k_xline).
 template <typename T2, int N1, int N2, int TPAD = 1, bool DIRECT = false>
 __device__ __forceinline__ void xline2_body(Dims d, Geo g, const T2* __restrict__ Hx, T2* __restrict__ H0, T2* __restrict__ H1, T2* __restrict__ H2,
@@ -298,10 +298,11 @@ __device__ __forceinline__ void xline2_body(Dims d, Geo g, const T2* __restrict_
         const int b = (unsigned)t / N2, n2 = t - b * N2;
         const int rr = b >> 1, which = b & 1;
         const size_t ro = (size_t)min(z0 + rr, d.ngal2 - 1) * NK;  // a row past the last repeats it
-        // line 2r: A = u, C = v; line 2r+1: A = w.  u-plane: C interpolated; v-plane: A
-        const T2* A0 = (which == 0 ? ua : wa) + ro;
+        // line 2r: A = u, C = v; line 2r+1: A = w.  u-plane: C interpolated; v-plane: A.  DIRECT: C = w
+        // and A = v, so that v, the smallest, travels alone
+        const T2* A0 = (which == 0 ? ua : (DIRECT ? va : wa)) + ro;
         const T2* A1 = (which == 0 ? ub : wb) + ro;
-        const T2* C0 = va + ro;
+        const T2* C0 = (DIRECT ? wa : va) + ro;
         const T2* C1 = vb + ro;
         const bool hasc = which == 0;
         T2 v[N1];
@@ -363,13 +364,16 @@ __device__ __forceinline__ void xline2_body(Dims d, Geo g, const T2* __restrict_
         for (int n2 = 0; n2 < N2; ++n2) y[n2] = o[n2];
         rdft<N2, +1>(y);
         // lane pair (u + i v, w + i 0); each lane passes its real part to the other:
-        // u-plane (a*a, b*b) on the even lane, (a*a, a*o) on the odd lane; v-plane (a*b, b*o)
+        // u-plane (a*a, b*b) on the even lane, (a*a, a*o) on the odd lane; v-plane (a*b, b*o).
+        // DIRECT, (u + i w, v + i 0): w goes to the odd lane, v to the even one: u-plane (a*a, a*b) and
+        // (a*a, o*o); v-plane (a*o, b*o)
         const bool sa = uplane && par, sb = uplane && !par;
 #pragma unroll
         for (int k2 = 0; k2 < N2; ++k2) {
             const R a = y[k2].x, b = y[k2].y;
-            const R o = __shfl_xor_sync(0xffffffffu, a, 1);
-            y[k2] = cx<T2>(a * (uplane ? a : b), (sa ? a : b) * (sb ? b : o));
+            const R o = __shfl_xor_sync(0xffffffffu, DIRECT && !par ? b : a, 1);
+            if (DIRECT) y[k2] = cx<T2>(a * (uplane ? a : o), (sb ? a : o) * (par ? o : b));
+            else y[k2] = cx<T2>(a * (uplane ? a : b), (sa ? a : b) * (sb ? b : o));
         }
         rdft<N2, -1>(y);
 #pragma unroll
@@ -420,8 +424,9 @@ __device__ __forceinline__ void xline2_body(Dims d, Geo g, const T2* __restrict_
         const T2 Pk = line[k];
         const T2 Qc = cconj(line[k == 0 ? 0 : N - k]);
         // real parts: u-plane uu / ww, v-plane uv; imaginary parts: u-plane vv / uw, v-plane vw
-        T2* da = which == 0 ? H0 : H3;
-        T2* db = which == 0 ? (uplane ? H2 : H1) : H1;
+        // (DIRECT: u-plane uu, uw / vv, ww; v-plane uv, vw)
+        T2* da = which == 0 ? H0 : (DIRECT ? H2 : H3);
+        T2* db = DIRECT ? (which == 0 ? H1 : H3) : (which == 0 ? (uplane ? H2 : H1) : H1);
         da[o] = cx<T2>((Pk.x + Qc.x) * hs, (Pk.y + Qc.y) * hs);
         db[o] = cx<T2>((Pk.y - Qc.y) * hs, -(Pk.x - Qc.x) * hs);
     }

@@ -144,10 +144,15 @@ const char *cfd_last_error(const cfd_ctx *ctx);
  *                   transforms u, w and v of each plane pair once and interpolates in
  *                   physical space (1.5 inverse and 3 forward lines per row and plane pair
  *                   instead of 4 and 3); FP32-mixed one-band contexts with x lengths 64,
- *                   96, 128, 192 and 256 to 576 (the default from 256 on; other lengths and
- *                   three-band channels run path 1).  FP64 one-band contexts march under
- *                   path 1 at x lengths 256 to 512 (CFD_MARCH=0: they do not);
- *                   CFD_XMARCH_STEPS sets the y-chunk
+ *                   96, 128, 192, 256, 288, 384, 432, 512 and 576 (other lengths and three-band
+ *                   channels run path 1).  The default at 384; FP64 one-band contexts march under
+ *                   path 1 at x lengths 256 to 512 (CFD_MARCH=0: they do not).
+ *                   CFD_XMARCH_STEPS sets the y-chunk, and asks for path 6 where xline_path
+ *                   and CFD_XLINE_PATH do not choose one
+ *                FP32-mixed contexts interpolate u, v, w in y in FP32, on transformed planes, on
+ *                paths 1, 3, 4, 5 at the six named lengths (below) and on path 6.  Where either
+ *                length is another, paths 1, 3, 4 and 5 interpolate the FP64 fields and
+ *                round once, as path 2 does at any length
  *   xline_rows   rows per CTA of the two-step x-line kernel: 2, 4 or 8 (path 6: 2 or 4)
  *   zlines       lines per CTA of the two-step z kernels: 4, 8 or 16
  *   solve_kind   1 (the only kind; other values fall back to it): a warp per column on chip up
@@ -156,7 +161,7 @@ const char *cfd_last_error(const cfd_ctx *ctx);
  *   rhs_chunk    y-planes per thread of the right-hand-side kernel: 2 .. 64 (by default 4, fewer on
  *                grids whose CTAs would leave SMs without work)
  *   xsplit       radix order of the x-line transforms (x-line paths 1, 5): 1 = the split
- *                N = N1*N2 of 64 = 8*8, 96 = 8*12, 128 = 8*16, 192 = 16*12, 384 = 16*24,
+ *                N = N1*N2 of the named lengths 64 = 8*8, 96 = 8*12, 128 = 8*16, 192 = 16*12, 384 = 16*24,
  *                768 = 32*24 (first step N1 points); 2 = the transposed split (16*4, 12*8,
  *                16*8, 12*16, 24*16, 24*32; the default at 192 and 768).  Other lengths have one
  *   zsplit       the same for the z transforms of the nonlinear pass (x-line path 1) */
