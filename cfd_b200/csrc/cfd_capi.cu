@@ -1721,19 +1721,21 @@ int strided_rft(cfd_ctx* c, double* dptr, int n, int isa, int m, long long bstri
     const double2* tw = n == c->d.ngal1 ? c->twx_d : (n == c->d.ngal2 ? c->twz_d : nullptr);
     if (!tw) return fail(c, CFD_ERR_SIZE, "rft length must be Ngal1 or Ngal2");
     if (const auto* k = line_kernels<double2>(n)) {
-        // two lines a transform; as many transforms a CTA as keep two or more CTAs on an SM
-        const bool a2 = ((uintptr_t)dptr & 15) == 0 && !((isa | bstride) & 1);
-        auto* f = k->pl_rft[iopt <= 0][a2];
+        // inverse: two lines a transform; as many transforms a CTA as keep two or more CTAs on an SM
+        const bool fwd = iopt <= 0, a2 = ((uintptr_t)dptr & 15) == 0 && !((isa | bstride) & 1);
+        auto* f = k->pl_rft[fwd][a2];
+        const int per = fwd ? rft_rows(k->n1, k->n2) : std::max(k->n1, k->n2);
         auto lsm = [&](int nl) {
-            return (int)((nl * (size_t)(((k->n1 * (k->n2 + 1)) | 1) + (iopt <= 0 ? n + 1 : 0)) + n) * sizeof(double2));
+            const size_t e = fwd ? (size_t)nl * rft_pitch(k->n1, k->n2) + (k->n1 / 2 + 1) * k->n2
+                                 : nl * (size_t)((k->n1 * (k->n2 + 1)) | 1) + n;
+            return (int)(e * sizeof(double2));
         };
         int nl = 8;
         while (nl > 1 && lsm(nl) > 72 * 1024) nl /= 2;
         CK(smem_limit(f, lsm(nl)));
-        const int pairs = (m + 1) / 2;
+        const int items = fwd ? m : (m + 1) / 2;
         prof_mark(c);
-        f<<<dim3((pairs + nl - 1) / nl, nb), (nl * std::max(k->n1, k->n2) + 31) / 32 * 32, lsm(nl), c->stream>>>(
-            dptr, isa, m, bstride, tw, nl);
+        f<<<dim3((items + nl - 1) / nl, nb), (nl * per + 31) / 32 * 32, lsm(nl), c->stream>>>(dptr, isa, m, bstride, tw, nl);
         LK("k_pl_rft");
         return CFD_OK;
     }

@@ -10,8 +10,8 @@
 // (planes built, transformed in place by radix-by-radix kernels and read again by the sums) moved 17
 // GB at 384 x 257(+90) x 384, 19.2 ms for a statistics call and a CFL query; here 3.8 ms, bound by the
 // FP64 transforms' latency at 12 warps an SM (k_st_x 86 us, k_st_z 27 us per 16 planes).  The plane
-// entry points (k_pl_cft, k_pl_rft) take a line through shared memory once instead of once a radix,
-// and two real lines a transform in both directions: 193 planes of 192 x 192, both ways, 264 -> 90 us.
+// entry points (k_pl_cft, k_pl_rft_inv, k_pl_rft_fwd) take a line through shared memory once instead of
+// once a radix: 193 planes of 192 x 192, both ways, 264 -> 82 us.
 #pragma once
 
 #include "transform_kernels.cuh"
@@ -273,15 +273,15 @@ __global__ void __launch_bounds__(8 * (TN1 > TN2 ? TN1 : TN2), (TN1 > TN2 ? TN1 
     two_step_lines<double2, TN1, TN2, SIGN>(lb, ex, twt, load, store);
 }
 
-// rft (rft_buff.f:24-86): real lines of length N in place, stride isa doubles, two lines 2b and 2b+1
-// a complex transform.  Inverse: x_a + i x_b from the Hermitian extensions of the half spectra (Im
-// of modes 0 and N/2 ignored); forward: x 1/N, Re and Im of modes 0..N/2 with zero Im at both ends.
-// nl transforms a CTA; grid: x = line chunk, y = batch.  A stated number of CTAs per SM lets the compiler
-// keep more loads in flight (192 points: 128 registers instead of 92): 193 x 192 lines of 192 points,
-// inverse 27.2 -> 24.2 us and forward 29.0 -> 28.2, 768 points 34.1 -> 30.7.
-template <int TN1, int TN2, int SIGN, bool A2>
+// rft (rft_buff.f:24-86): real lines of length N in place, stride isa doubles.  grid: x = line chunk, y =
+// batch.  A stated number of CTAs per SM lets the compiler keep more loads in flight (inverse at 192
+// points: 128 registers instead of 92, 193 x 192 lines 27.2 -> 24.2 us).
+//
+// Inverse: two lines 2b and 2b+1 a complex transform, x_a + i x_b from the Hermitian extensions of the
+// half spectra (Im of modes 0 and N/2 ignored); nl transforms a CTA.
+template <int TN1, int TN2, bool A2>
 __global__ void __launch_bounds__((8 * (TN1 > TN2 ? TN1 : TN2) + 31) / 32 * 32, (TN1 > TN2 ? TN1 : TN2) <= 16 ? 4 : ((TN1 > TN2 ? TN1 : TN2) <= 24 ? 2 : 1))
-    k_pl_rft(double* __restrict__ c, int isa, int m, long long bstride, const double2* __restrict__ tw, int nl) {
+    k_pl_rft_inv(double* __restrict__ c, int isa, int m, long long bstride, const double2* __restrict__ tw, int nl) {
     constexpr int N = TN1 * TN2;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     double2* twt = reinterpret_cast<double2*>(smem_raw);
@@ -292,45 +292,78 @@ __global__ void __launch_bounds__((8 * (TN1 > TN2 ? TN1 : TN2) + 31) / 32 * 32, 
     // (a line past the last repeats it in the transform and is not stored)
     auto line = [&](int i) { return base + (size_t)min(i, m - 1) * isa; };
     __syncthreads();
-    if constexpr (SIGN > 0) {
-        auto load = [&](int e, int b) -> double2 {
-            const int k = e <= N / 2 ? e : N - e;
-            const double *xa = line(2 * (l0 + b)) + 2 * k, *xb = line(2 * (l0 + b) + 1) + 2 * k;
-            double2 A, Bv;
-            if (A2) { A = *reinterpret_cast<const double2*>(xa); Bv = *reinterpret_cast<const double2*>(xb); }
-            else { A = dc(xa[0], xa[1]); Bv = dc(xb[0], xb[1]); }
-            if (k == 0 || k == N / 2) { A.y = 0; Bv.y = 0; }
-            if (e > N / 2) { A.y = -A.y; Bv.y = -Bv.y; }
-            return dc(A.x - Bv.y, A.y + Bv.x);
-        };
-        auto store = [&](int x, int b, double2 v) {
-            const int i = 2 * (l0 + b);
-            if (i < m) base[(size_t)i * isa + x] = v.x;
-            if (i + 1 < m) base[(size_t)(i + 1) * isa + x] = v.y;
-        };
-        two_step_lines<double2, TN1, TN2, +1, false>(0, ex, twt, load, store, nl);
-    } else {
-        constexpr int LU = N + 1;
-        double2* ub = ex + (size_t)nl * exch_row<TN1, TN2>();
-        auto load = [&](int x, int b) -> double2 { return dc(line(2 * (l0 + b))[x], line(2 * (l0 + b) + 1)[x]); };
-        auto store = [&](int k, int b, double2 v) { ub[(size_t)b * LU + k] = v; };
-        two_step_lines<double2, TN1, TN2, -1, false>(0, ex, twt, load, store, nl);
-        constexpr int NK = N / 2 + 1;
-        const double hs = 0.5 / N;
-        for (int it = threadIdx.x; it < nl * NK; it += blockDim.x) {
-            const int b = (unsigned)it / NK, k = it - b * NK, i = 2 * (l0 + b);
-            const double2 Pk = ub[(size_t)b * LU + k], Q = ub[(size_t)b * LU + (k == 0 ? 0 : N - k)];
-            const bool edge = k == 0 || k == N / 2;
-            const double2 xa = dc((Pk.x + Q.x) * hs, edge ? 0.0 : (Pk.y - Q.y) * hs);
-            const double2 xb = dc((Pk.y + Q.y) * hs, edge ? 0.0 : (Q.x - Pk.x) * hs);
-            auto put = [&](int r, double2 v) {
-                if (r >= m) return;
-                double* a = base + (size_t)r * isa + 2 * k;
-                if (A2) *reinterpret_cast<double2*>(a) = v;
-                else { a[0] = v.x; a[1] = v.y; }
-            };
-            put(i, xa);
-            put(i + 1, xb);
+    auto load = [&](int e, int b) -> double2 {
+        const int k = e <= N / 2 ? e : N - e;
+        const double *xa = line(2 * (l0 + b)) + 2 * k, *xb = line(2 * (l0 + b) + 1) + 2 * k;
+        double2 A, Bv;
+        if (A2) { A = *reinterpret_cast<const double2*>(xa); Bv = *reinterpret_cast<const double2*>(xb); }
+        else { A = dc(xa[0], xa[1]); Bv = dc(xb[0], xb[1]); }
+        if (k == 0 || k == N / 2) { A.y = 0; Bv.y = 0; }
+        if (e > N / 2) { A.y = -A.y; Bv.y = -Bv.y; }
+        return dc(A.x - Bv.y, A.y + Bv.x);
+    };
+    auto store = [&](int x, int b, double2 v) {
+        const int i = 2 * (l0 + b);
+        if (i < m) base[(size_t)i * isa + x] = v.x;
+        if (i + 1 < m) base[(size_t)(i + 1) * isa + x] = v.y;
+    };
+    two_step_lines<double2, TN1, TN2, +1, false>(0, ex, twt, load, store, nl);
+}
+
+// Forward: a line by itself, x 1/N, Re and Im of modes 0..N/2 with zero Im at both ends.  (Two lines in
+// one complex transform share their rounding: a small line would carry that of its neighbour, and a
+// NaN would spoil both.)  The N1-point DFTs of real columns are Hermitian in k1, so the second step
+// takes k1 <= N1/2 only: with X_(N-k) = conj X_k its outputs are the whole half spectrum, half the
+// work and the exchange of a complex line, and nothing is left to unpack: 193 x 192 lines of 192 points
+// 20.5 us (28.2 in pairs), 40 x 384 of 384 25.5, 12 x 768 of 768 34.6.  TN1 is even.
+__host__ __device__ constexpr int rft_rows(int n1, int n2) { return n2 > n1 / 2 + 1 ? n2 : n1 / 2 + 1; }
+__host__ __device__ constexpr int rft_pitch(int n1, int n2) { return ((n1 / 2 + 1) * (n2 + 1)) | 1; }
+template <int TN1, int TN2, bool A2>
+__global__ void __launch_bounds__((8 * rft_rows(TN1, TN2) + 31) / 32 * 32, (TN1 > TN2 ? TN1 : TN2) <= 16 ? 4 : ((TN1 > TN2 ? TN1 : TN2) <= 24 ? 2 : 1))
+    k_pl_rft_fwd(double* __restrict__ c, int isa, int m, long long bstride, const double2* __restrict__ tw, int nl) {
+    static_assert(TN1 % 2 == 0, "an even first step");
+    constexpr int N = TN1 * TN2, H1 = TN1 / 2 + 1, LX = rft_pitch(TN1, TN2);
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    double2* twt = reinterpret_cast<double2*>(smem_raw);  // twt[k1 * TN2 + n2], k1 < H1
+    double2* ex = twt + H1 * TN2;
+    for (int i = threadIdx.x; i < H1 * TN2; i += blockDim.x) twt[i] = tw[(i / TN2) * (i % TN2)];
+    double* base = c + (size_t)blockIdx.y * bstride;
+    const int l0 = blockIdx.x * nl, t = threadIdx.x;
+    __syncthreads();
+    if (t < nl * TN2) {
+        const int b = t / TN2, n2 = t - b * TN2;
+        // (a line past the last repeats it in the transform and is not stored)
+        const double* x = base + (size_t)min(l0 + b, m - 1) * isa + n2;
+        double2 v[TN1];
+#pragma unroll
+        for (int n1 = 0; n1 < TN1; ++n1) v[n1] = dc(x[n1 * TN2], 0.0);
+        rdft<TN1, -1>(v);
+        double2* o = ex + (size_t)b * LX + n2;
+#pragma unroll
+        for (int k1 = 0; k1 < H1; ++k1) o[k1 * (TN2 + 1)] = k1 == 0 ? v[0] : cmul(v[k1], twt[k1 * TN2 + n2]);
+    }
+    __syncthreads();
+    if (t < nl * H1) {
+        const int b = t / H1, k1 = t - b * H1;
+        const double2* o = ex + (size_t)b * LX + k1 * (TN2 + 1);
+        double2 y[TN2];
+#pragma unroll
+        for (int n2 = 0; n2 < TN2; ++n2) y[n2] = o[n2];
+        rdft<TN2, -1>(y);
+        if (l0 + b >= m) return;
+        double* x = base + (size_t)(l0 + b) * isa;
+        const bool self = k1 == 0 || k1 == TN1 / 2;  // holds both k and N - k
+#pragma unroll
+        for (int k2 = 0; k2 < TN2; ++k2) {
+            const int e = k1 + TN1 * k2;
+            const bool low = e <= N / 2;
+            if (!low && self) continue;
+            const int k = low ? e : N - e;
+            double2 v = dscl(1.0 / N, y[k2]);
+            if (!low) v.y = -v.y;
+            if (k == 0 || k == N / 2) v.y = 0.0;
+            if (A2) *reinterpret_cast<double2*>(x + 2 * k) = v;
+            else { x[2 * k] = v.x; x[2 * k + 1] = v.y; }
         }
     }
 }

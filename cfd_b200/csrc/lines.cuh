@@ -143,10 +143,10 @@ const LineKernels<T2>* line_table() {
             t.pl_cft[0][1] = k_pl_cft<N1, N2, +1, true>;
             t.pl_cft[1][0] = k_pl_cft<N1, N2, -1, false>;
             t.pl_cft[1][1] = k_pl_cft<N1, N2, -1, true>;
-            t.pl_rft[0][0] = k_pl_rft<N1, N2, +1, false>;
-            t.pl_rft[0][1] = k_pl_rft<N1, N2, +1, true>;
-            t.pl_rft[1][0] = k_pl_rft<N1, N2, -1, false>;
-            t.pl_rft[1][1] = k_pl_rft<N1, N2, -1, true>;
+            t.pl_rft[0][0] = k_pl_rft_inv<N1, N2, false>;
+            t.pl_rft[0][1] = k_pl_rft_inv<N1, N2, true>;
+            t.pl_rft[1][0] = k_pl_rft_fwd<N1, N2, false>;
+            t.pl_rft[1][1] = k_pl_rft_fwd<N1, N2, true>;
         }
         return t;
     }();
