@@ -100,9 +100,9 @@ struct cfd_ctx {
     int nsm = 1;            // SMs of the device (CTAs of the persistent kernels)
     double* coltab = nullptr;
     cfd::ColMaps colmap, colmap_p;  // of the solves and of cfd_solve_p
-    // set by k_col_solve (mapped host memory) when a transfer did not arrive: the fields are undefined
-    // until a state is uploaded again
-    int *col_err = nullptr, *col_err_dev = nullptr;
+    // scal[3] is set by k_col_solve when a transfer did not arrive; col_new: solves were issued since the
+    // host last read it, col_bad: it read it set (the fields are undefined until a state is uploaded again)
+    bool col_new = false, col_bad = false;
     int col_tries = cfd::kWaitTries;
     double* scal = nullptr;
     double* mf_work = nullptr;
@@ -240,13 +240,6 @@ int cuda_check(cfd_ctx* c, cudaError_t e, const char* what) {
     return CFD_OK;
 }
 
-// whether every column solve so far (of those the host has waited for) got its columns
-int solves_complete(cfd_ctx* c) {
-    if (c->col_err && *(volatile int*)c->col_err)
-        return fail(c, CFD_ERR_CUDA, "a transfer of the column solves did not complete: the fields are undefined");
-    return CFD_OK;
-}
-
 #define CK(call)                                                   \
     do {                                                           \
         int _s = cuda_check(c, (call), #call);                     \
@@ -278,6 +271,20 @@ void prof_mark(cfd_ctx* c) {
             c->prof.push_back({"", {ev, ev}});
         }
     }
+}
+
+// Whether every column solve got its columns, of those the host has read the flag of: `wait` reads it on
+// stream st after what was issued there (a caller that synchronises), else what is known.
+int solves_complete(cfd_ctx* c, cudaStream_t st = nullptr, bool wait = false) {
+    if (wait && c->col_new) {
+        double e = 0.0;
+        CK(cudaMemcpyAsync(&e, c->scal + 3, sizeof(e), cudaMemcpyDeviceToHost, st));
+        CK(cudaStreamSynchronize(st));
+        c->col_new = false;
+        c->col_bad = c->col_bad || e != 0.0;
+    }
+    if (c->col_bad) return fail(c, CFD_ERR_CUDA, "a transfer of the column solves did not complete: the fields are undefined");
+    return CFD_OK;
 }
 
 #define LK(name)                                    \
@@ -820,7 +827,8 @@ int col_solve(cfd_ctx* c, int mode, int krk, const char* name) {
     a.dtirk = (1.0 / c->dt) / ab;
     a.dtrk = c->dt * ab;
     a.mean_diag = c->mean_diag;
-    a.err = c->col_err_dev;
+    a.err = c->scal + 3;
+    c->col_new = true;
     a.tries = c->col_tries;
     a.ahead = col_ahead(c->colC, c->d.ncol);
     prof_mark(c);
@@ -857,9 +865,6 @@ int col_table(cfd_ctx* c, const cfd_config* cfg) {
     AL(c->coltab, double, h.size());
     CK(cudaMemcpy(c->coltab, h.data(), sizeof(double) * h.size(), cudaMemcpyHostToDevice));
     CK(col_prepare(m, c->colC, c->mb));
-    CK(cudaHostAlloc((void**)&c->col_err, sizeof(int), cudaHostAllocMapped));
-    *c->col_err = 0;
-    CK(cudaHostGetDevicePointer((void**)&c->col_err_dev, c->col_err, 0));
     c->col_tries = env_int("CFD_SOLVE_TRIES", kWaitTries, 0, kWaitTries);
     ColMaps &a = c->colmap, &b = c->colmap_p;
     const int nu = d.nyu, nv = d.nyv, np = d.nyp;
@@ -1993,7 +1998,6 @@ int cfd_destroy(cfd_ctx* c) {
             if (c->xev[f][k]) cudaEventDestroy(c->xev[f][k]);
     if (c->xin) cudaStreamDestroy(c->xin);
     if (c->xout) cudaStreamDestroy(c->xout);
-    if (c->col_err) cudaFreeHost(c->col_err);
     if (c->ev_fork) cudaEventDestroy(c->ev_fork);
     if (c->ev_join) cudaEventDestroy(c->ev_join);
     if (c->side) cudaStreamDestroy(c->side);
@@ -2016,7 +2020,7 @@ int cfd_set_stream(cfd_ctx* c, void* stream) {
 int cfd_synchronize(cfd_ctx* c) {
     if (!c) return CFD_ERR_ARG;
     CK(cudaStreamSynchronize(c->stream));
-    return solves_complete(c);
+    return solves_complete(c, c->stream, true);
 }
 
 int cfd_field_shape(const cfd_ctx* c, int32_t field, int64_t* ncomplex, int32_t* j0, int32_t* nplanes, int32_t* ncolumns) {
@@ -2070,9 +2074,9 @@ int cfd_upload_field(cfd_ctx* c, int32_t field, const double* host, int32_t layo
     if (layout != CFD_LAYOUT_REF && layout != CFD_LAYOUT_PLANE) return fail(c, CFD_ERR_ARG, "bad layout %d", layout);
     CK(cudaSetDevice(c->device));
     if (field <= CFD_FIELD_U3) c->hx_valid = false;  // the nonlinear pass's transforms are stale
-    if (field <= CFD_FIELD_P && c->col_err && *(volatile int*)c->col_err) {  // a new state begins
-        CK(cudaStreamSynchronize(c->stream));
-        *c->col_err = 0;
+    if (field <= CFD_FIELD_P && c->col_bad) {  // a new state begins
+        CK(cudaMemsetAsync(c->scal + 3, 0, sizeof(double), c->stream));
+        c->col_bad = false;
     }
     const size_t n = (size_t)fi.nplanes * c->d.ncol;
     if (layout == CFD_LAYOUT_REF && field <= CFD_FIELD_P && !fi.single) {
@@ -2266,6 +2270,7 @@ int cfd_step(cfd_ctx* c, int32_t nsteps) {
     }
     for (int n = 0; n < nsteps; ++n) {
         CK(cudaGraphLaunch(c->gexec, c->stream));
+        c->col_new = c->colM > 0;
         c->launches += c->graph_launches;
     }
     return CFD_OK;
@@ -2279,6 +2284,8 @@ int cfd_get_scalars(cfd_ctx* c, double* mpgx, double* qx, double* dgx) {
     if (mpgx) *mpgx = h[0];
     if (qx) *qx = h[1];
     if (dgx) *dgx = h[2];
+    c->col_new = false;
+    c->col_bad = c->col_bad || h[3] != 0.0;
     if (int s = solves_complete(c)) return s;
     if (!std::isfinite(h[0]) || !std::isfinite(h[1]) || !std::isfinite(h[2]))
         return fail(c, CFD_ERR_NONFINITE, "non-finite mean-flow scalars (mpgx %g, Qx %g)", h[0], h[1]);
@@ -2304,7 +2311,7 @@ int cfd_divergence_max(cfd_ctx* c, double* errmax) {
         m = std::max(m, v);
     }
     *errmax = bad ? NAN : m;
-    if (int s2 = solves_complete(c)) return s2;
+    if (int s2 = solves_complete(c, c->stream, true)) return s2;
     if (bad) return fail(c, CFD_ERR_NONFINITE, "non-finite divergence");
     return CFD_OK;
 }
@@ -2410,7 +2417,7 @@ int cfd_spectra_read(cfd_ctx* c, double* spu, double* spv, double* spw, double* 
     auto& st = c->st;
     if (!st.on || !st.spu) return fail(c, CFD_ERR_STATE, "spectra not configured");
     CK(cudaStreamSynchronize(c->stream));
-    if (int e = solves_complete(c)) return e;
+    if (int e = solves_complete(c, c->stream, true)) return e;
     // device [plane][column] -> the reference's sp(j,column), j fastest
     std::vector<double> h;
     auto get = [&](double* out, const double* dev, int ny) -> int {
@@ -2437,7 +2444,7 @@ int cfd_stats_read(cfd_ctx* c, double* u_sums, double* v_sums, double* p_sums, d
     auto& st = c->st;
     if (!st.on) return fail(c, CFD_ERR_STATE, "statistics not configured");
     CK(cudaStreamSynchronize(c->stream));
-    if (int e = solves_complete(c)) return e;
+    if (int e = solves_complete(c, c->stream, true)) return e;
     if (u_sums) CK(cudaMemcpy(u_sums, st.su, sizeof(double) * 6 * d.nyu, cudaMemcpyDeviceToHost));
     if (v_sums) CK(cudaMemcpy(v_sums, st.sv, sizeof(double) * 5 * d.nyv, cudaMemcpyDeviceToHost));
     if (p_sums) CK(cudaMemcpy(p_sums, st.sp, sizeof(double) * 2 * d.nyp, cudaMemcpyDeviceToHost));
@@ -2575,7 +2582,10 @@ int cfd_ensemble_step(cfd_ensemble* e, int32_t nsteps) {
     for (int k = 0; k < nsteps; ++k) ECK(cudaGraphLaunch(e->gexec, e->master));
     // later work on a member's stream waits for the ensemble
     ECK(cudaEventRecord(e->done, e->master));
-    for (cfd_ctx* c : e->m) ECK(cudaStreamWaitEvent(c->stream, e->done, 0));
+    for (cfd_ctx* c : e->m) {
+        ECK(cudaStreamWaitEvent(c->stream, e->done, 0));
+        c->col_new = c->colM > 0;
+    }
     return CFD_OK;
 }
 
@@ -2583,7 +2593,7 @@ int cfd_ensemble_synchronize(cfd_ensemble* e) {
     if (!e) return CFD_ERR_ARG;
     ECK(cudaStreamSynchronize(e->master));
     for (size_t i = 0; i < e->m.size(); ++i)
-        if (int s = solves_complete(e->m[i])) return efail(e, s, "member %zu: %s", i, e->m[i]->err.c_str());
+        if (int s = solves_complete(e->m[i], e->master, true)) return efail(e, s, "member %zu: %s", i, e->m[i]->err.c_str());
     return CFD_OK;
 }
 
@@ -2640,7 +2650,7 @@ int cfd_cfl(cfd_ctx* c, double* dtc, double* terms) {
     if (s) return s;
     std::vector<double> h((size_t)3 * d.nyu);
     CK(cudaStreamSynchronize(c->stream));  // the pass runs on the (non-blocking) context stream
-    if ((s = solves_complete(c))) return s;
+    if ((s = solves_complete(c, c->stream, true))) return s;
     CK(cudaMemcpy(h.data(), c->st.mx, sizeof(double) * h.size(), cudaMemcpyDeviceToHost));
     double um = 0.0, wm = 0.0, vm = 1e-6;
     bool bad = false;

@@ -217,7 +217,7 @@ struct ColArgs {
     double dtirk;       // 1 / (dt (a+b))
     double dtrk;        // dt (a+b)
     double mean_diag;   // bottom row of D.G at kx = kz = 0
-    int* err;           // (host memory) set if a transfer did not arrive
+    double* err;        // set if a transfer did not arrive
     int tries;          // limit of the waits for one (kWaitTries)
     bool ahead;         // prefetch the next columns into L2 while these are solved
 };
@@ -470,10 +470,7 @@ __global__ void __launch_bounds__(32 * C * col_groups(M, C))
             }
         }
     }
-    if (!ok && lead) {
-        *A.err = 1;
-        __threadfence_system();
-    }
+    if (!ok && lead) *A.err = 1.0;
     if (lead) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
 }
 

@@ -176,9 +176,8 @@ int cfd_get_tuning(const cfd_ctx *ctx, cfd_tuning *tuning);
 
 /* Work on a caller-provided cudaStream_t (NULL = the context's own stream).
  * The column solves wait for their transfers with a limit.  If one ran out, the fields are
- * undefined: the calls that synchronise return CFD_ERR_CUDA from then on, as do stages, steps,
- * downloads and statistics issued after the host could see it, until cfd_upload_field begins a
- * new state. */
+ * undefined: the next call that synchronises returns CFD_ERR_CUDA, and from then on so do stages,
+ * steps, downloads and statistics, until cfd_upload_field begins a new state. */
 int cfd_set_stream(cfd_ctx *ctx, void *stream);
 int cfd_synchronize(cfd_ctx *ctx);
 
