@@ -1844,11 +1844,11 @@ int stats_pass_lines(cfd_ctx* c, bool acc) {
     auto& st = c->st;
     const auto *kz = line_kernels<double2>(d.ngal2), *kx = line_kernels<double2>(d.ngal1);
     const bool cond = acc && st.dnx > 0;
-    const int cp = cond ? st.lcpc : st.lcp, nlr = acc ? 4 : 2, rw = st_x_lines(kx->n1, kx->n2) / nlr;
-    const int nrow = (d.ngal2 + rw - 1) / rw, nf = acc ? 5 : 3;
-    const size_t smz = ((size_t)8 * ((kz->n1 * (kz->n2 + 1)) | 1) + d.ngal2) * sizeof(double2);
-    const size_t smx = ((size_t)nlr * rw * st_x_row(kx->n1, kx->n2) + d.ngal1) * sizeof(double2);
-    const int ntx = (nlr * rw * std::max(kx->n1, kx->n2) + 31) / 32 * 32;
+    const int cp = cond ? st.lcpc : st.lcp, ns = st_x_slots(acc), P = st_x_lines(kx->n1, kx->n2) / ns;
+    const int nrow = (d.ngal2 / 2 + P - 1) / P, nf = acc ? 5 : 3;
+    const size_t smz = z_lines_smem(kz->n1, kz->n2, 8, sizeof(double2));
+    const size_t smx = ((size_t)P * st_x_used(acc) * st_x_row(kx->n1, kx->n2) + d.ngal1) * sizeof(double2);
+    const int ntx = (ns * P * std::max(kx->n1, kx->n2) + 31) / 32 * 32;
     CK(smem_limit(kz->st_z, (int)smz));
     CK(smem_limit(kx->st_x[acc], (int)smx));
     for (int j0 = 0; j0 < d.nyu; j0 += cp) {
@@ -1859,7 +1859,7 @@ int stats_pass_lines(cfd_ctx* c, bool acc) {
             d, c->g, s, c->u1, c->u2, c->u3, c->p, st.hs, c->twz_d, 3);
         LK("k_st_z");
         prof_mark(c);
-        kx->st_x[acc]<<<dim3(nrow, n), ntx, smx, c->stream>>>(d, c->g, s, st.hs, c->twx_d, rw, ilog2(rw), st.lpart,
+        kx->st_x[acc]<<<dim3(nrow, n), ntx, smx, c->stream>>>(d, c->g, s, st.hs, c->twx_d, P, ilog2(P), st.lpart,
                                                              cond ? st.fold : nullptr, st.dnx, st.nbu, st.nbv, st.nbp);
         LK("k_st_x");
         const int nb = std::max(st.nbu, std::max(st.nbv, st.nbp));
@@ -1871,7 +1871,7 @@ int stats_pass_lines(cfd_ctx* c, bool acc) {
         }
     }
     prof_mark(c);
-    k_st_fin_lines<<<d.nyu, 256, 0, c->stream>>>(d, c->g, st.lpart, nrow, nlr, st.su, st.sv, st.sp, st.mx);
+    k_st_fin_lines<<<d.nyu, 256, 0, c->stream>>>(d, c->g, st.lpart, nrow, ns, st.su, st.sv, st.sp, st.mx);
     LK("k_st_fin_lines");
     return CFD_OK;
 }

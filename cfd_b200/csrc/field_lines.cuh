@@ -8,8 +8,8 @@
 // transforms them in x and reduces the physical values in registers: no physical plane is stored.
 // The planes go through in chunks whose transformed fields stay in L2.  The passes they replace
 // (planes built, transformed in place by radix-by-radix kernels and read again by the sums) moved 17
-// GB at 384 x 257(+90) x 384, 19.2 ms for a statistics call and a CFL query; here 3.8 ms, bound by the
-// FP64 transforms' latency at 12 warps an SM (k_st_x 86 us, k_st_z 27 us per 16 planes).  The plane
+// GB at 384 x 257(+90) x 384, 19.2 ms for a statistics call and a CFL query; here 3.7 ms, bound by the
+// FP64 transforms' latency at 12 warps an SM (k_st_x 85 us, k_st_z 27 us per 16 planes).  The plane
 // entry points (k_pl_cft, k_pl_rft_inv, k_pl_rft_fwd) take a line through shared memory once instead of
 // once a radix: 193 planes of 192 x 192, both ways, 264 -> 82 us.
 #pragma once
@@ -71,44 +71,45 @@ __device__ __forceinline__ unsigned long long mag_bits(double a) {
     return (unsigned long long)__double_as_longlong(a) & 0x7fffffffffffffffull;
 }
 
-// complex lines of a k_st_x CTA, and the pitch of a line's exchange
+// line slots of a k_st_x CTA, the pitch of a line's exchange, and for a pair of rows the lines
+// transformed and the slots they take (a power of two: adjacent lanes in the second step)
 __host__ __device__ constexpr int st_x_lines(int n1, int n2) { return (n1 > n2 ? n1 : n2) >= 16 ? 8 : 16; }
 __host__ __device__ constexpr int st_x_row(int n1, int n2) { return n1 * (n2 + 1) > n1 * n2 ? n1 * (n2 + 1) + 1 : n1 * n2 + 1; }
+__host__ __device__ constexpr int st_x_used(bool acc) { return acc ? 7 : 3; }
+__host__ __device__ constexpr int st_x_slots(bool acc) { return acc ? 8 : 4; }
 
-// A CTA: RW rows of plane index jr = j0 + blockIdx.y, NLR complex lines a row, each two real
-// signals:  ACC: u + i w, v(centre) + i p, v + i w(face), omega_x;  else: u + i w, v.
-// part[(jr*gridDim.x + blockIdx.x)*NLR*8 + l*8 + q]: of line l, the sums of a, a^2, c, c^2,
-// a * (a of the neighbour line), a*c and the maxima of |a| and |c| (a + i c the line's values;
-// omega_x over the first N1 x N2 points, stats.f90:53-60).  With pc, on the planes of a band (its
+// A CTA: P row pairs of plane index jr = j0 + blockIdx.y.  A complex line is one quantity on the two rows
+// of a pair (row z + i row z + 1), so that its rounding is relative to that quantity alone; lines 0.. of
+// a pair:  ACC: u, w, v(centre), p, v, w(face), omega_x;  else: u, w, v.
+// part[((jr*gridDim.x + blockIdx.x)*slots + l)*4 + q]: of line l, the sums of a, a^2 and a*o (o: w for
+// u, u for v(centre), w(face) for v) and the maximum of |a| over the points of the CTA's rows
+// (omega_x over the first N1 x N2 points, stats.f90:53-60).  With pc, on the planes of a band (its
 // nbu, nbv, nbp planes from either end): pc[((pl*ngal2 + z)*kStQ + q)*dnx + ti], row z folded
 // onto a tile of dnx points.
 template <int TN1, int TN2, bool ACC>
 __global__ void __launch_bounds__((st_x_lines(TN1, TN2) * (TN1 > TN2 ? TN1 : TN2) + 31) / 32 * 32, 2)
-    k_st_x(Dims d, Geo g, StChunk s, const double2* __restrict__ Hs, const double2* __restrict__ twx, int RW, int lrw,
+    k_st_x(Dims d, Geo g, StChunk s, const double2* __restrict__ Hs, const double2* __restrict__ twx, int P, int lp,
            double* __restrict__ part, double* __restrict__ pc, int dnx, int nbu, int nbv, int nbp) {
-    constexpr int N = TN1 * TN2, HX = N / 3, NK = HX + 1, NLR = ACC ? 4 : 2;
+    constexpr int N = TN1 * TN2, HX = N / 3, NK = HX + 1, NU = st_x_used(ACC), NL = st_x_slots(ACC);
     constexpr int LX = st_x_row(TN1, TN2);
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    __shared__ double red[16][NLR][8];
+    __shared__ double red[16][NL][4];
     double2* twt = reinterpret_cast<double2*>(smem_raw);
     double2* ex = twt + N;
     load_twiddles<double2, TN1, TN2>(twt, twx);
-    const int t = threadIdx.x, B = NLR * RW;
-    const int z0 = blockIdx.x * RW, jr = s.j0 + blockIdx.y;
+    const int t = threadIdx.x, z0 = blockIdx.x * 2 * P, jr = s.j0 + blockIdx.y;
     __syncthreads();
     // ---- inverse N1-point DFTs, thread (line b, column n2)
-    if (t < B * TN2) {
+    if (t < P * NU * TN2) {
         const int b = (unsigned)t / TN2, n2 = t - b * TN2;
-        const int l = b & (NLR - 1), z = min(z0 + b / NLR, d.ngal2 - 1);
-        auto P = [&](int f, int j) { return Hs + ((size_t)(s.off[f] + j - s.first[f]) * d.ngal2 + z) * NK; };
-        // a = a0 A0 + a1 A1 + a2 A2, c = c0 C0 + c1 C1
-        const double2* none = P(0, jr);
-        const double2 *A0 = none, *A1 = none, *A2 = none, *C0 = none, *C1 = none;
-        double a0 = 0, a1 = 0, a2 = 0, c0 = 0, c1 = 0;
-        if (l == 0) {
-            A0 = P(0, jr); a0 = 1.0;
-            C0 = P(1, jr); c0 = 1.0;
-        } else if (ACC && l == 1) {  // interp_v with its ghost centres (FOU3D.f90:285-308)
+        const int pr = b / NU, l = b - pr * NU, z = min(z0 + 2 * pr, d.ngal2 - 2);
+        auto F = [&](int f, int j) { return Hs + ((size_t)(s.off[f] + j - s.first[f]) * d.ngal2 + z) * NK; };
+        // a0 A0 + a1 A1 + a2 A2 of either row
+        const double2 *A0 = F(0, jr), *A1 = A0, *A2 = A0;
+        double a0 = 0, a1 = 0, a2 = 0;
+        if (l < 2) {
+            A0 = F(l, jr); a0 = 1.0;
+        } else if (ACC && l == 2) {  // interp_v with its ghost centres (FOU3D.f90:285-308)
             int j;
             if (jr == 0) {
                 j = 1; a0 = (1.0 - g.gwib) * g.vca[1]; a1 = g.gwib + (1.0 - g.gwib) * g.vcb[1];
@@ -117,25 +118,26 @@ __global__ void __launch_bounds__((st_x_lines(TN1, TN2) * (TN1 > TN2 ? TN1 : TN2
             } else {
                 j = jr; a0 = g.vca[jr]; a1 = g.vcb[jr];
             }
-            A0 = P(2, j); A1 = P(2, j - 1);
-            if (jr < d.nyp) { C0 = P(4, jr); c0 = 1.0; }
+            A0 = F(2, j); A1 = F(2, j - 1);
+        } else if (ACC && l == 3) {
+            if (jr < d.nyp) { A0 = F(4, jr); a0 = 1.0; }
         } else if (jr < d.nyv) {
-            if (!ACC || l == 2) {
-                A0 = P(2, jr); a0 = 1.0;
-                if (ACC) { C0 = P(1, jr + 1); c0 = g.ufa[jr]; C1 = P(1, jr); c1 = g.ufb[jr]; }
+            if (l == (ACC ? 4 : 2)) {
+                A0 = F(2, jr); a0 = 1.0;
+            } else if (l == 5) {  // w at the face
+                A0 = F(1, jr + 1); a0 = g.ufa[jr]; A1 = F(1, jr); a1 = g.ufb[jr];
             } else {  // omega_x = dw/dy - dv/dz at the face
-                A0 = P(1, jr + 1); a0 = g.dthdyv[jr];
-                A1 = P(1, jr); a1 = -a0;
-                A2 = P(3, jr); a2 = -1.0;
+                A0 = F(1, jr + 1); a0 = g.dthdyv[jr];
+                A1 = F(1, jr); a1 = -a0;
+                A2 = F(3, jr); a2 = -1.0;
             }
         }
-        const bool ta1 = a1 != 0.0, ta2 = a2 != 0.0, tc0 = c0 != 0.0, tc1 = c1 != 0.0;
-        auto fetch = [&](int k, double2& a, double2& c) {
-            a = dscl(a0, A0[k]);
+        const bool ta1 = a1 != 0.0, ta2 = a2 != 0.0;
+        auto fetch = [&](int k) {
+            double2 a = dscl(a0, A0[k]);
             if (ta1) a = dadd(a, dscl(a1, A1[k]));
             if (ta2) a = dadd(a, dscl(a2, A2[k]));
-            c = tc0 ? dscl(c0, C0[k]) : dc(0, 0);
-            if (tc1) c = dadd(c, dscl(c1, C1[k]));
+            return a;
         };
         double2 v[TN1];
 #pragma unroll
@@ -143,13 +145,13 @@ __global__ void __launch_bounds__((st_x_lines(TN1, TN2) * (TN1 > TN2 ? TN1 : TN2
             const int e0 = n1 * TN2, e = e0 + n2;
             const bool lo = (e0 + TN2 - 1 <= HX) || (e0 <= HX && e <= HX);
             const bool hi = (e0 >= N - HX) || (e0 + TN2 - 1 >= N - HX && e >= N - HX);
-            double2 val = dc(0, 0), a, c;
+            double2 val = dc(0, 0);
             if (lo) {  // the inverse real transform ignores Im of kx = 0
-                fetch(e, a, c);
+                double2 a = fetch(e), c = fetch(NK + e);
                 if (n1 == 0 && n2 == 0) { a.y = 0; c.y = 0; }
                 val = dc(a.x - c.y, a.y + c.x);
             } else if (hi) {
-                fetch(N - e, a, c);
+                const double2 a = fetch(N - e), c = fetch(NK + N - e);
                 val = dc(a.x + c.y, -a.y + c.x);
             }
             v[n1] = val;
@@ -160,54 +162,59 @@ __global__ void __launch_bounds__((st_x_lines(TN1, TN2) * (TN1 > TN2 ? TN1 : TN2
         for (int k1 = 0; k1 < TN1; ++k1) o[k1 * (TN2 + 1)] = k1 == 0 ? v[0] : cmulc(v[k1], twt[k1 * TN2 + n2]);
     }
     __syncthreads();
-    // ---- inverse N2-point DFTs -> x = k1 + N1 k2; the lines of a row in adjacent lanes
-    const bool act = t < B * TN1;
-    const int l = t & (NLR - 1), rest = t / NLR, rr = rest & (RW - 1), k1 = min(rest >> lrw, TN1 - 1);
-    const int b = rr * NLR + l, z = z0 + rr;
+    // ---- inverse N2-point DFTs -> x = k1 + N1 k2; the lines of a pair in adjacent lanes
+    const int l = t & (NL - 1), rest = t / NL, pr = rest & (P - 1), k1 = min(rest >> lp, TN1 - 1);
+    const bool act = t < P * NL * TN1 && l < NU;
+    const int b = pr * NU + min(l, NU - 1), z = z0 + 2 * pr;
+    // the lane of the line that this one is multiplied with
+    const int src = (t & 31 & ~(NL - 1)) | (l == 0 ? 1 : (l == 2 ? 0 : (l == 4 ? 5 : l)));
     double2 y[TN2];
-    double q[6] = {0, 0, 0, 0, 0, 0};
-    unsigned long long ma = 0, mc = 0;
-    if ((t & ~31) < B * TN1) {
+    double q[3] = {0, 0, 0};
+    unsigned long long ma = 0;
+    if ((t & ~31) < P * NL * TN1) {
         const double2* o = ex + (size_t)b * LX + k1 * (TN2 + 1);
 #pragma unroll
         for (int n2 = 0; n2 < TN2; ++n2) y[n2] = o[n2];
         rdft<TN2, +1>(y);
-        const bool in = act && z < d.ngal2;
+        // (omega_x: N2 is even, so both rows of a pair count or neither)
+        const bool wx = ACC && l == 6, in = act && z < (wx ? d.n2 : d.ngal2);
 #pragma unroll
         for (int k2 = 0; k2 < TN2; ++k2) {
             const double a = y[k2].x, c = y[k2].y;
-            const double o2 = ACC ? __shfl_xor_sync(0xffffffffu, a, 1) : 0.0;
-            const bool wx = ACC && l == 3;
-            if (in && (!wx || (k1 + TN1 * k2 < d.n1 && z < d.n2))) {
+            double oa = 0.0, oc = 0.0;
+            if (ACC) {
+                oa = __shfl_sync(0xffffffffu, a, src);
+                oc = __shfl_sync(0xffffffffu, c, src);
+            }
+            if (in && (!wx || k1 + TN1 * k2 < d.n1)) {
                 if (ACC) {
-                    q[0] += a; q[1] += a * a; q[2] += c; q[3] += c * c; q[4] += a * o2; q[5] += a * c;
+                    q[0] += a + c;
+                    q[1] += a * a + c * c;
+                    q[2] += a * oa + c * oc;
                 }
-                ma = max(ma, mag_bits(a));
-                mc = max(mc, mag_bits(c));
+                ma = max(ma, max(mag_bits(a), mag_bits(c)));
             }
         }
 #pragma unroll
-        for (int o2 = NLR; o2 < 32; o2 <<= 1) {
+        for (int o2 = NL; o2 < 32; o2 <<= 1) {
 #pragma unroll
-            for (int k = 0; k < 6; ++k)
+            for (int k = 0; k < 3; ++k)
                 if (ACC) q[k] += __shfl_xor_sync(0xffffffffu, q[k], o2);
             ma = max(ma, __shfl_xor_sync(0xffffffffu, ma, o2));
-            mc = max(mc, __shfl_xor_sync(0xffffffffu, mc, o2));
         }
     }
-    if ((t & 31) < NLR) {
+    if ((t & 31) < NL) {
         double* o = red[t >> 5][t & 31];
 #pragma unroll
-        for (int k = 0; k < 6; ++k) o[k] = q[k];
-        o[6] = __longlong_as_double((long long)ma);
-        o[7] = __longlong_as_double((long long)mc);
+        for (int k = 0; k < 3; ++k) o[k] = q[k];
+        o[3] = __longlong_as_double((long long)ma);
     }
     __syncthreads();
-    if (t < NLR * 8) {
-        const int lr = t >> 3, k = t & 7, nw = (blockDim.x + 31) >> 5;
+    if (t < NL * 4) {
+        const int lr = t >> 2, k = t & 3, nw = (blockDim.x + 31) >> 5;
         double v = red[0][lr][k];
-        for (int w = 1; w < nw; ++w) v = k < 6 ? v + red[w][lr][k] : nan_max(v, red[w][lr][k]);
-        part[((size_t)jr * gridDim.x + blockIdx.x) * NLR * 8 + t] = v;
+        for (int w = 1; w < nw; ++w) v = k < 3 ? v + red[w][lr][k] : nan_max(v, red[w][lr][k]);
+        part[((size_t)jr * gridDim.x + blockIdx.x) * NL * 4 + t] = v;
     }
     if constexpr (ACC) {
         auto band = [&](int ny, int nb) { return jr < ny && (jr < nb || ny - 1 - jr < nb); };
@@ -217,20 +224,21 @@ __global__ void __launch_bounds__((st_x_lines(TN1, TN2) * (TN1 > TN2 ? TN1 : TN2
             for (int k2 = 0; k2 < TN2; ++k2) ex[(size_t)b * LX + k1 + TN1 * k2] = y[k2];
         __syncthreads();
         const int ntx = N / dnx;
-        for (int it = t; it < RW * 3 * dnx; it += blockDim.x) {
+        for (int it = t; it < 2 * P * 3 * dnx; it += blockDim.x) {
             const int ti = it % dnx, gq = (it / dnx) % 3, row = it / (3 * dnx);
             if (z0 + row >= d.ngal2) break;
-            const double2* L0 = ex + (size_t)(row * 4 + (gq == 1 ? 2 : 0)) * LX + ti;
-            const double2* L1 = L0 + LX;
+            // point x of line r of the row's pair, at 2 x
+            auto line = [&](int r) { return reinterpret_cast<const double*>(ex + (size_t)((row >> 1) * NU + r) * LX + ti) + (row & 1); };
+            const double *L0 = line(gq == 0 ? 0 : (gq == 1 ? 4 : 3)), *L1 = line(gq == 0 ? 1 : (gq == 1 ? 6 : 3)),
+                         *L2 = line(gq == 0 ? 2 : (gq == 1 ? 5 : 3));
             double f[6] = {0, 0, 0, 0, 0, 0};
             for (int ix = 0; ix < ntx; ++ix) {
-                const double2 m = L0[ix * dnx], n = L1[ix * dnx];
-                if (gq == 0) {  // u + i w, v(centre) + i p
-                    f[0] += m.x; f[1] += m.x * m.x; f[2] += m.y; f[3] += m.y * m.y; f[4] += m.x * n.x; f[5] += m.x * m.y;
-                } else if (gq == 1) {  // v + i w(face), omega_x
-                    f[0] += m.x; f[1] += m.x * m.x; f[2] += n.x; f[3] += n.x * n.x; f[4] += m.x * m.y;
-                } else {
-                    f[0] += n.y; f[1] += n.y * n.y;
+                const double m = L0[2 * ix * dnx];
+                f[0] += m; f[1] += m * m;
+                if (gq < 2) {  // u, w, v(centre) or v, omega_x, w(face)
+                    const double n = L1[2 * ix * dnx];
+                    f[2] += n; f[3] += n * n; f[4] += m * L2[2 * ix * dnx];
+                    if (gq == 0) f[5] += m * n;
                 }
             }
             double* o = pc + (((size_t)blockIdx.y * d.ngal2 + z0 + row) * kStQ + (gq == 0 ? 0 : (gq == 1 ? 6 : 11))) * dnx + ti;

@@ -254,34 +254,37 @@ __global__ void __launch_bounds__(256) k_st_cond_fin(const double* __restrict__ 
 
 // The partial sums of k_st_x added into the plane accumulators, CTA after CTA in eight interleaved
 // runs that are then added in order (deterministic), and the maxima of the CFL query.  One CTA of
-// 256 threads per plane; nlr lines a row (4: sums and maxima, 2: maxima).
-__global__ void __launch_bounds__(256) k_st_fin_lines(Dims d, Geo g, const double* __restrict__ part, int nrow, int nlr,
+// 256 threads per plane; ns line slots a row pair (8: sums and maxima, 4: maxima).
+__global__ void __launch_bounds__(256) k_st_fin_lines(Dims d, Geo g, const double* __restrict__ part, int nrow, int ns,
                                                       double* __restrict__ su, double* __restrict__ sv,
                                                       double* __restrict__ sp, double* __restrict__ mx) {
     __shared__ double red[8][32];
-    const int jr = blockIdx.x, w = nlr * 8;
-    const int c = threadIdx.x & 31, s = threadIdx.x >> 5, k = c & 7;
+    const int jr = blockIdx.x, w = ns * 4;
+    const int c = threadIdx.x & 31, s = threadIdx.x >> 5, k = c & 3;
     if (c < w) {
         double v = 0.0;
         for (int r = s; r < nrow; r += 8) {
             const double x = part[((size_t)jr * nrow + r) * w + c];
-            v = k < 6 ? v + x : nan_max(v, x);
+            v = k < 3 ? v + x : nan_max(v, x);
         }
         red[s][c] = v;
     }
     __syncthreads();
     if (threadIdx.x >= w) return;
     double v = red[0][c];
-    for (int i = 1; i < 8; ++i) v = k < 6 ? v + red[i][c] : nan_max(v, red[i][c]);
-    const int l = c >> 3, lv = nlr == 4 ? 2 : 1;  // the line of v
-    if (k >= 6) {
-        if (l == 0) mx[(k == 6 ? 0 : d.nyu) + jr] = v;
-        else if (l == lv && k == 6 && jr < d.nyv) mx[2 * d.nyu + jr] = jr > 0 && jr < d.nyv - 1 ? v * g.dthdyv[jr] : 0.0;
-    } else if (nlr == 4) {
-        if (l == 0) su[(size_t)k * d.nyu + jr] += v;
-        else if (l == 1 && (k == 2 || k == 3) && jr < d.nyp) sp[(size_t)(k - 2) * d.nyp + jr] += v;
-        else if (l == 2 && (k < 2 || k == 5) && jr < d.nyv) sv[(size_t)(k == 5 ? 4 : k) * d.nyv + jr] += v;
-        else if (l == 3 && k < 2 && jr < d.nyv) sv[(size_t)(2 + k) * d.nyv + jr] += v;
+    for (int i = 1; i < 8; ++i) v = k < 3 ? v + red[i][c] : nan_max(v, red[i][c]);
+    const int l = c >> 2, lv = ns == 8 ? 4 : 2;  // the line of v
+    if (k == 3) {
+        if (l < 2) mx[l * d.nyu + jr] = v;
+        else if (l == lv && jr < d.nyv) mx[2 * d.nyu + jr] = jr > 0 && jr < d.nyv - 1 ? v * g.dthdyv[jr] : 0.0;
+    } else if (ns == 8) {
+        // lines u, w, v(centre), p, v, w(face), omega_x: sum, sum of squares, product
+        if (l == 0) su[(size_t)(k == 2 ? 5 : k) * d.nyu + jr] += v;
+        else if (l == 1 && k < 2) su[(size_t)(2 + k) * d.nyu + jr] += v;
+        else if (l == 2 && k == 2) su[(size_t)4 * d.nyu + jr] += v;
+        else if (l == 3 && k < 2 && jr < d.nyp) sp[(size_t)k * d.nyp + jr] += v;
+        else if (l == 4 && jr < d.nyv) sv[(size_t)(k == 2 ? 4 : k) * d.nyv + jr] += v;
+        else if (l == 6 && k < 2 && jr < d.nyv) sv[(size_t)(2 + k) * d.nyv + jr] += v;
     }
 }
 
