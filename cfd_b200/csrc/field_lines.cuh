@@ -2,9 +2,9 @@
 // entry points (sm_100a).
 //
 // Statistics (stats.f90:1-253) and dtc_calc (FOU3D.f90:516-544) reduce physical planes of u, v, w,
-// the y-interpolated v and w, omega_x and p.  Interpolation and dw/dy are linear in y and commute
-// with the transforms, so each field is transformed in z once on its own planes (k_st_z; dv/dz
-// takes its i kz there), and k_st_x forms the sources of a row from the transformed planes,
+// the y-interpolated v and w, omega_x and p.  Interpolation in y is linear and commutes with the
+// transforms, so each field is transformed in z once on its own planes (k_st_z; omega_x as a field of
+// its own), and k_st_x forms the sources of a row from the transformed planes,
 // transforms them in x and reduces the physical values in registers: no physical plane is stored.
 // The planes go through in chunks whose transformed fields stay in L2.  The passes they replace
 // (planes built, transformed in place by radix-by-radix kernels and read again by the sums) moved 17
@@ -19,7 +19,7 @@
 namespace cfd {
 
 // One chunk: u planes j0..j0+cp-1, v and p planes of the same index, and the neighbours their
-// interpolations read.  Field f (u, w, v, dv/dz, p) holds planes first[f]..first[f]+n[f]-1 of its
+// interpolations read.  Field f (u, w, v, omega_x, p) holds planes first[f]..first[f]+n[f]-1 of its
 // grid (those that exist) from slot off[f] on.
 struct StChunk {
     int j0, cp;
@@ -47,20 +47,31 @@ __global__ void __launch_bounds__(8 * (TN1 > TN2 ? TN1 : TN2), (TN1 > TN2 ? TN1 
     const int ny = f < 2 ? d.nyu : (f < 4 ? d.nyv : d.nyp);
     const int j = s.first[f] + pl;
     const bool live = line0 + b < nlines && j >= 0 && j < ny;
-    const double2* src = (f == 0 ? u1 : (f == 1 ? u3 : (f < 4 ? u2 : p))) + (size_t)min(max(j, 0), ny - 1) * d.ncol + i;
+    const int jc = min(max(j, 0), ny - 1);
+    const double2* src = (f == 0 ? u1 : (f == 1 ? u3 : (f < 4 ? u2 : p))) + (size_t)jc * d.ncol + i;
     double2* H = Hs + ((size_t)s.off[f] + pl) * N * d.nkx + i;
     const int r = threadIdx.x >> lb;
-    const bool dz = f == 3;
     __syncthreads();
-    auto load = [&](int e, int) -> double2 {
-        const int q = zrow_q<N, TN2>(e, r);
-        if (q < 0) return dc(0, 0);
-        const double2 v = src[(size_t)q * d.nkx];
-        // the kz = -N2/2 mode of a z derivative is zero (der_z, FOU3D.f90:388-412)
-        return dz ? (q == d.n2 / 2 ? dc(0, 0) : dik(g.kz[q], v)) : v;
-    };
     auto store = [&](int z, int, double2 v) {
         if (live) H[(size_t)z * d.nkx] = v;
+    };
+    if (f == 3) {  // omega_x = dw/dy - dv/dz at the face: w is differenced before its rounding by a transform
+        const double2* w = u3 + (size_t)jc * d.ncol + i;
+        const double dth = g.dthdyv[jc];
+        auto load = [&](int e, int) -> double2 {
+            const int q = zrow_q<N, TN2>(e, r);
+            if (q < 0) return dc(0, 0);
+            const size_t o = (size_t)q * d.nkx;
+            const double2 a = dscl(dth, dsub(w[o + d.ncol], w[o]));
+            // the kz = -N2/2 mode of a z derivative is zero (der_z, FOU3D.f90:388-412)
+            return q == d.n2 / 2 ? a : dsub(a, dik(g.kz[q], src[o]));
+        };
+        two_step_lines<double2, TN1, TN2, +1>(lb, ex, twt, load, store);
+        return;
+    }
+    auto load = [&](int e, int) -> double2 {
+        const int q = zrow_q<N, TN2>(e, r);
+        return q < 0 ? dc(0, 0) : src[(size_t)q * d.nkx];
     };
     two_step_lines<double2, TN1, TN2, +1>(lb, ex, twt, load, store);
 }
@@ -104,9 +115,9 @@ __global__ void __launch_bounds__((st_x_lines(TN1, TN2) * (TN1 > TN2 ? TN1 : TN2
         const int b = (unsigned)t / TN2, n2 = t - b * TN2;
         const int pr = b / NU, l = b - pr * NU, z = min(z0 + 2 * pr, d.ngal2 - 2);
         auto F = [&](int f, int j) { return Hs + ((size_t)(s.off[f] + j - s.first[f]) * d.ngal2 + z) * NK; };
-        // a0 A0 + a1 A1 + a2 A2 of either row
-        const double2 *A0 = F(0, jr), *A1 = A0, *A2 = A0;
-        double a0 = 0, a1 = 0, a2 = 0;
+        // a0 A0 + a1 A1 of either row
+        const double2 *A0 = F(0, jr), *A1 = A0;
+        double a0 = 0, a1 = 0;
         if (l < 2) {
             A0 = F(l, jr); a0 = 1.0;
         } else if (ACC && l == 2) {  // interp_v with its ghost centres (FOU3D.f90:285-308)
@@ -126,18 +137,14 @@ __global__ void __launch_bounds__((st_x_lines(TN1, TN2) * (TN1 > TN2 ? TN1 : TN2
                 A0 = F(2, jr); a0 = 1.0;
             } else if (l == 5) {  // w at the face
                 A0 = F(1, jr + 1); a0 = g.ufa[jr]; A1 = F(1, jr); a1 = g.ufb[jr];
-            } else {  // omega_x = dw/dy - dv/dz at the face
-                A0 = F(1, jr + 1); a0 = g.dthdyv[jr];
-                A1 = F(1, jr); a1 = -a0;
-                A2 = F(3, jr); a2 = -1.0;
+            } else {  // omega_x
+                A0 = F(3, jr); a0 = 1.0;
             }
         }
-        const bool ta1 = a1 != 0.0, ta2 = a2 != 0.0;
+        const bool two = a1 != 0.0;
         auto fetch = [&](int k) {
-            double2 a = dscl(a0, A0[k]);
-            if (ta1) a = dadd(a, dscl(a1, A1[k]));
-            if (ta2) a = dadd(a, dscl(a2, A2[k]));
-            return a;
+            const double2 a = dscl(a0, A0[k]);
+            return two ? dadd(a, dscl(a1, A1[k])) : a;
         };
         double2 v[TN1];
 #pragma unroll
