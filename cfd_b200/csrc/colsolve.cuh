@@ -38,7 +38,7 @@
 
 namespace cfd {
 
-// couplings of the reduced system that cannot change a double (2^-60)
+// couplings of the reduced system whose products cannot change a diagonal (2^-60)
 constexpr double kDecoupled = 8.67e-19;
 constexpr int kColTabs = 8;  // doubles per row of the coefficient table
 
@@ -124,34 +124,50 @@ __device__ __forceinline__ void warp_tridiag(double2 (&y)[NR][M], Coef coef) {
     }
     constexpr int L = M > 1 ? M - 2 : 0;
     coef(M - 1, a, c, s);
+    // (a sum takes its couplings together first, here and below: they are the smaller part, so one
+    // rounding of the full size is left instead of two)
     double2 f[NR];
 #pragma unroll
-    for (int k = 0; k < NR; ++k) f[k] = y[k][M - 1];
+    for (int k = 0; k < NR; ++k) {
+        const double2 n = dscl(c, shfl_down2(A[k], 1));
+        f[k] = dadd(y[k][M - 1], M > 1 ? dadds(n, a, y[k][L]) : n);
+    }
     double al = a;
     if (M > 1) {
         al = a * l[L];
         s += a * e;
-#pragma unroll
-        for (int k = 0; k < NR; ++k) f[k] = dadds(f[k], a, y[k][L]);
     }
     double ga = c * __shfl_down_sync(0xffffffffu, C, 1);
     s += c * __shfl_down_sync(0xffffffffu, E, 1);
-#pragma unroll
-    for (int k = 0; k < NR; ++k) f[k] = dadds(f[k], c, shfl_down2(A[k], 1));
-    // (al + ga + s) X(s) - al X(s-d) - ga X(s+d) = f, until the couplings are below rounding (at
-    // once for the Helmholtz rows of a small time step: they fall by about beta/dy^2 a row)
+    // (al + ga + s) X(s) - al X(s-d) - ga X(s+d) = f.  The rows are not scaled on the way, so f is
+    // rounded once a step, until the couplings are so small that their products cannot change the
+    // diagonals (at once for the Helmholtz rows of a small time step: they fall by about beta/dy^2 a
+    // row).  What they still carry from row to row counts where a right-hand side is zero or small:
+    // the steps left take it along, on rows scaled to a diagonal of 1.
+    int d = 1;
 #pragma unroll 1
-    for (int d = 1;; d <<= 1) {
+    for (;; d <<= 1) {
         const double r = pivot_rcp(s + (al + ga));
-        al *= r;
-        ga *= r;
-        s *= r;
+        if (d == 32 || __all_sync(0xffffffffu, fmax(fabs(al), fabs(ga)) * r < kDecoupled)) {
+            al *= r;
+            ga *= r;
 #pragma unroll
-        for (int k = 0; k < NR; ++k) f[k] = dscl(r, f[k]);
-        if (d == 32 || __all_sync(0xffffffffu, fmax(fabs(al), fabs(ga)) < kDecoupled)) break;
+            for (int k = 0; k < NR; ++k) f[k] = dscl(r, f[k]);
+            break;
+        }
+        const double alm = __shfl_up_sync(0xffffffffu, al, d), gap = __shfl_down_sync(0xffffffffu, ga, d);
+        al *= __shfl_up_sync(0xffffffffu, r, d);
+        ga *= __shfl_down_sync(0xffffffffu, r, d);
+#pragma unroll
+        for (int k = 0; k < NR; ++k) f[k] = dadd(f[k], dadds(dscl(al, shfl_up2(f[k], d)), ga, shfl_down2(f[k], d)));
+        s += al * __shfl_up_sync(0xffffffffu, s, d) + ga * __shfl_down_sync(0xffffffffu, s, d);
+        al *= alm;
+        ga *= gap;
+    }
+#pragma unroll 1
+    for (; d < 32; d <<= 1) {
 #pragma unroll
         for (int k = 0; k < NR; ++k) f[k] = dadds(dadds(f[k], al, shfl_up2(f[k], d)), ga, shfl_down2(f[k], d));
-        s += al * __shfl_up_sync(0xffffffffu, s, d) + ga * __shfl_down_sync(0xffffffffu, s, d);
         al *= __shfl_up_sync(0xffffffffu, al, d);
         ga *= __shfl_down_sync(0xffffffffu, ga, d);
     }
@@ -160,7 +176,7 @@ __device__ __forceinline__ void warp_tridiag(double2 (&y)[NR][M], Coef coef) {
         const double2 X = shfl_up2(f[k], 1);
         y[k][M - 1] = f[k];
 #pragma unroll
-        for (int i = M - 2; i >= 0; --i) y[k][i] = dadds(dadds(y[k][i], l[i], X), cs[i], y[k][i + 1]);
+        for (int i = M - 2; i >= 0; --i) y[k][i] = dadd(y[k][i], dadds(dscl(cs[i], y[k][i + 1]), l[i], X));
     }
 }
 
