@@ -1488,6 +1488,21 @@ int create_impl(const cfd_config* cfg, const cfd_ib_list* ibu, const cfd_ib_list
         }
     }
     if (c->LZ2 < 0) c->RW2 = 0;  // the two-step x-line kernels read the output of k_zinv2s
+    // k_zinv2, the z pass where no x-line kernel interpolates, takes as many lines as its registers let a
+    // CTA have (FP64: 136 to 174 a thread at the 27- and 32-point steps, so not 16 lines of them)
+    if (c->LZ2 >= 0 && (c->mb || !c->RW2 || (mixed && !named2)))
+        for (int n : {d.ngal2, c->mb ? c->dM.ngal2 : 0}) {
+            int n1s = 0, n2s = 0;
+            line_split(n, n1s, n2s);
+            if (!n1s) continue;
+            cudaFuncAttributes a;
+            CK(mixed ? cudaFuncGetAttributes(&a, line_kernels<float2>(n)->zinv2)
+                     : cudaFuncGetAttributes(&a, line_kernels<double2>(n)->zinv2));
+            while (c->LZ2 > 0 && (std::max(n1s, n2s) << c->LZ2) > a.maxThreadsPerBlock) --c->LZ2;
+            line_split(d.ngal2, n1s, n2s);
+            c->NTZ2 = (1 << c->LZ2) * std::max(n1s, n2s);
+            c->SMZ2 = z_lines_smem(n1s, n2s, 1 << c->LZ2, esz);
+        }
     if (c->mb) {
         // Three bands: a z pass that interpolates (k_zinv2), the x-line pass on interpolated planes
         // (k_xline2b, or k_xline for x lengths without a two-step split) and k_zfwd2, one launch a
