@@ -353,7 +353,7 @@ bool band_length(int n) { return n == 64 || n == 96 || n == 128 || n == 192 || n
 //   CFD_SOLVE_GROUP  columns of a group of the warp-per-column solves (4 or 8)
 //   CFD_SOLVE_TRIES  limit of their waits for a transfer (0: every wait runs out at once, and the
 //                    call that synchronises next reports it)
-//   CFD_RHS_CHUNK    y-planes per thread of the right-hand-side kernel (2..64)
+//   CFD_RHS_CHUNK    y-planes per thread of the right-hand-side kernel (1..64)
 int env_int(const char* name, int dflt, int lo, int hi) {
     const char* v = std::getenv(name);
     if (!v || !*v) return dflt;
@@ -1631,7 +1631,7 @@ int create_impl(const cfd_config* cfg, const cfd_ib_list* ibu, const cfd_ib_list
     // one plane a thread: 7.1 -> 3.1 us)
     c->JC = 4;
     while (c->JC > 1 && (long long)((d.ncol + 255) / 256) * ((d.nyu + c->JC - 1) / c->JC) < 2LL * c->nsm) c->JC /= 2;
-    c->JC = tune_int(&cfd_tuning::rhs_chunk, "CFD_RHS_CHUNK", c->JC, 2, 64);
+    c->JC = tune_int(&cfd_tuning::rhs_chunk, "CFD_RHS_CHUNK", c->JC, 1, 64);
     c->SNT = 1 << ilog2(tune_int(&cfd_tuning::solve_cols, "CFD_SOLVE_THREADS", 64, 32, 256));
     c->nch = (d.nyu - 2 + c->JC - 1) / c->JC;
     AL(c->scal, double, 4);

@@ -158,7 +158,7 @@ const char *cfd_last_error(const cfd_ctx *ctx);
  *   solve_kind   1 (the only kind; other values fall back to it): a warp per column on chip up
  *                to 736 planes, thread-per-column Thomas sweeps above
  *   solve_cols   threads (columns) per CTA of those sweeps: 32, 64, 128 or 256
- *   rhs_chunk    y-planes per thread of the right-hand-side kernel: 2 .. 64 (by default 4, fewer on
+ *   rhs_chunk    y-planes per thread of the right-hand-side kernel: 1 .. 64 (by default 4, fewer on
  *                grids whose CTAs would leave SMs without work)
  *   xsplit       radix order of the x-line transforms (x-line paths 1, 5): 1 = the split
  *                N = N1*N2 of the named lengths 64 = 8*8, 96 = 8*12, 128 = 8*16, 192 = 16*12, 384 = 16*24,
