@@ -37,9 +37,24 @@ def keeps_precision(setup, tuning) -> bool:
     return setup is None or tuning.get("xline_path") != 6 or (setup.cfg.ngal1 in NAMED and setup.cfg.ngal2 in NAMED)
 
 
-# knobs that only act with another setting (the library reports them as 0 or 1 otherwise)
-RELEVANT = {"xline_rows": lambda t: t.get("xline_path") != 2,
-            "zsplit": lambda t: t.get("xline_path") in (1, 5, 6)}
+# planes above which the implicit solves run as the column sweeps that solve_cols shapes
+SWEEP_PLANES = 736
+
+
+def relevant(knob, tuning, setup, precision) -> bool:
+    """Whether a knob acts at all: not on x-line path 2, whose kernel has no rows or z split of its own, nor
+    in FP64 at the lengths that march by two rows whatever is asked for, nor, for the sweeps, on columns
+    that the on-chip solves take.  (setup None: any grid.)"""
+    path = tuning.get("xline_path")
+    if knob == "xline_rows":
+        march = setup is not None and precision == "fp64" and path == 1 and tuning.get("xsplit") != 2 and \
+            tuning.get("xline_rows") == 2 and setup.cfg.ngal1 in (256, 288, 384, 432, 512)
+        return path != 2 and not march
+    if knob == "zsplit":
+        return path in (1, 5, 6)
+    if knob == "solve_cols":
+        return setup is None or setup.grid.nyu > SWEEP_PLANES
+    return True
 
 
 def _cache_path() -> str:
@@ -49,7 +64,7 @@ def _cache_path() -> str:
 
 def _key(setup, precision: str, gpu: str) -> str:
     c, g = setup.cfg, setup.grid
-    return f"v9|{gpu}|{c.ngal1}x{g.nyu}x{c.ngal2}|{precision}|ib{setup.ibu.n > 0}"
+    return f"v10|{gpu}|{c.ngal1}x{g.nyu}x{c.ngal2}|{precision}|ib{setup.ibu.n > 0}"
 
 
 def time_step(setup, precision, device, tuning, steps=5, warmup=2):
@@ -79,7 +94,7 @@ def autotune(setup, precision: str, device: int = 0, steps: int = 5, log=None):
     tried = {json.dumps(best, sort_keys=True)}
     for name, values in KNOBS:
         for v in values:
-            if name in RELEVANT and not RELEVANT[name](best):
+            if not isinstance(name, tuple) and not relevant(name, best, setup, precision):
                 continue
             cand = dict(best, **(dict(zip(name, v)) if isinstance(name, tuple) else {name: v}))
             if precision == "fp64" and cand.get("xline_path") in MIXED_ONLY_XLINE:
@@ -99,7 +114,7 @@ def autotune(setup, precision: str, device: int = 0, steps: int = 5, log=None):
             tried.add(json.dumps(eff, sort_keys=True))
             if log:
                 log(f"{eff} {t * 1e3:.3f} ms/step")
-            if t < best_t:
+            if t < best_t and eff != best:  # (equal shapes are the same program, timed again)
                 best_t, best = t, eff
     return best, best_t
 

@@ -1989,7 +1989,7 @@ int cfd_create_tuned(const cfd_config* cfg, const cfd_ib_list* ibu, const cfd_ib
 int cfd_get_tuning(const cfd_ctx* c, cfd_tuning* t) {
     if (!c || !t) return CFD_ERR_ARG;
     t->xline_path = c->RWD ? 1 : c->RW2 ? (c->XMRW && c->precision == CFD_PREC_MIXED ? 6 : (c->RW4 ? 4 : (c->XL3 ? 3 : (c->XR64 ? 5 : 1)))) : 2;
-    t->xline_rows = c->XMRW && c->precision == CFD_PREC_MIXED ? c->XMRW : (c->RW4 ? c->RW4 : (c->RWD ? c->RWD : c->RW2));
+    t->xline_rows = c->XMRW ? c->XMRW : (c->RW4 ? c->RW4 : (c->RWD ? c->RWD : c->RW2));
     t->zlines = c->LZ2 >= 0 ? (1 << c->LZ2) : 0;
     t->solve_kind = 1;
     t->solve_cols = c->SNT;
