@@ -462,8 +462,6 @@ int set_smem_attrs(cfd_ctx* c) {
         size_t smb = 0;  // (equal lengths share a kernel)
         for (int m = 0; m < 2; ++m)
             if (const auto* kb = line_kernels<T2>(nx[m])) {
-                c->RWB[m] = 4;
-                while (c->RWB[m] > 1 && xline2_smem(kb->n1, kb->n2, c->RWB[m], esz) > 110 * 1024) c->RWB[m] /= 2;
                 smb = std::max(nx[0] == nx[1] ? smb : 0, xline2_smem(kb->n1, kb->n2, c->RWB[m], esz));
                 set(kb->xline2b, smb);
             }
@@ -1123,20 +1121,21 @@ int setup_ib(cfd_ctx* c, const cfd_ib_list* l, int j0, int j1, IBDev& ib, IBPlan
     const int ng1 = c->d.ngal1, ng2 = c->d.ngal2;
     pl = ib_planes(l);
     // (of a plane that repeats another, the first point stands for the rest)
-    for (size_t q = 0; q < pl.as.size(); ++q)
-    for (int p = pl.begin[q], e = pl.as[q] == (int)q ? pl.begin[q + 1] : p + 1; p < e; ++p) {
-        const int32_t* id = l->idx + 9 * (size_t)p;
-        for (int t = 0; t < 3; ++t) {
-            const int i = id[3 * t], k = id[3 * t + 1], j = id[3 * t + 2];
-            if (i < 1 || i > ng1 || k < 1 || k > ng2)
-                return fail(c, CFD_ERR_ARG, "%s: point %d has (i,k)=(%d,%d) outside 1..%d x 1..%d", name, p, i, k, ng1, ng2);
-            if (j < j0 || j > j1 || slot[j - j0] < 0)
-                return fail(c, CFD_ERR_ARG, "%s: point %d references plane %d outside the round-trip ranges", name, p, j);
-        }
-        if (p > 0) {
-            const int32_t* pv = id - 9;
-            const long a = ((long)pv[2] * ng2 + pv[1]) * ng1 + pv[0], b = ((long)id[2] * ng2 + id[1]) * ng1 + id[0];
-            if (b < a) return fail(c, CFD_ERR_ARG, "%s: points must be sorted by (j,k,i) (point %d)", name, p);
+    for (size_t q = 0; q < pl.as.size(); ++q) {
+        for (int p = pl.begin[q], e = pl.as[q] == (int)q ? pl.begin[q + 1] : p + 1; p < e; ++p) {
+            const int32_t* id = l->idx + 9 * (size_t)p;
+            for (int t = 0; t < 3; ++t) {
+                const int i = id[3 * t], k = id[3 * t + 1], j = id[3 * t + 2];
+                if (i < 1 || i > ng1 || k < 1 || k > ng2)
+                    return fail(c, CFD_ERR_ARG, "%s: point %d has (i,k)=(%d,%d) outside 1..%d x 1..%d", name, p, i, k, ng1, ng2);
+                if (j < j0 || j > j1 || slot[j - j0] < 0)
+                    return fail(c, CFD_ERR_ARG, "%s: point %d references plane %d outside the round-trip ranges", name, p, j);
+            }
+            if (p > 0) {
+                const int32_t* pv = id - 9;
+                const long a = ((long)pv[2] * ng2 + pv[1]) * ng1 + pv[0], b = ((long)id[2] * ng2 + id[1]) * ng1 + id[0];
+                if (b < a) return fail(c, CFD_ERR_ARG, "%s: points must be sorted by (j,k,i) (point %d)", name, p);
+            }
         }
     }
     ib.n = l->n;
@@ -1422,25 +1421,18 @@ int create_impl(const cfd_config* cfg, const cfd_ib_list* ibu, const cfd_ib_list
     // field and slot instead of one per plane, 144 x 108 x 131 a step of 302 -> 312 us.
     const bool named2 = line_kernels_named<float2>(d.ngal1) && line_kernels_named<float2>(d.ngal2);
     const bool march_asked = line_march_f32(d.ngal1) && std::getenv("CFD_XMARCH_STEPS");
+    const LineDefaults dx = line_defaults(d.ngal1, mixed), dz = line_defaults(d.ngal2, mixed);
     const int xpath = g_tuning && g_tuning->xline_path
                           ? g_tuning->xline_path
-                          : env_int("CFD_XLINE_PATH", !mixed ? 1 : (named2 ? (d.ngal1 == 384 ? 6 : (d.ngal1 == 192 ? 5 : 1))
-                                                                          : (march_asked ? 6 : 1)), 1, 6);
+                          : env_int("CFD_XLINE_PATH", mixed && !named2 ? (march_asked ? 6 : 1) : dx.xpath, 1, 6);
     // (the tuning variants exist for the six named lengths; the others run path 1)
     const bool named = line_kernels_named<float2>(d.ngal1) != nullptr;
-    // (at 768 points the transposed splits are the default: FP32 x lines 24 * 32 in 8 rows 736 us
-    // against 818 for 32 * 24 in 4, z lines 166 + 298 against 200 + 331 FP32, 326 + 627 in 4 lines
-    // against 361 + 811 FP64, at
-    // 768 x 65 x 768; at 192 points too: a step of 192 x 193(+90) x 192 2.36 -> 2.24 ms FP64, of 192 x
-    // 161(+76) x 192 1.34 -> 1.25 ms FP32 with the 64-register x-line)
-    const bool x768 = d.ngal1 == 768 && mixed, z768 = d.ngal2 == 768;
-    const bool xalt = named && (xpath == 1 || xpath == 5) &&
-                      tune_int(&cfd_tuning::xsplit, "CFD_XSPLIT", x768 || d.ngal1 == 192 ? 2 : 1, 1, 2) == 2;
+    const bool xalt = named && (xpath == 1 || xpath == 5) && tune_int(&cfd_tuning::xsplit, "CFD_XSPLIT", dx.xsplit, 1, 2) == 2;
     {
         int n1s = 0, n2s = 0;
         line_split(d.ngal1, n1s, n2s, xalt);
         if (n1s) {
-            int rw = tune_int(&cfd_tuning::xline_rows, "CFD_XLINE_ROWS", x768 ? 8 : 4, 2, 8);
+            int rw = tune_int(&cfd_tuning::xline_rows, "CFD_XLINE_ROWS", dx.xrows, 2, 8);
             rw = 1 << (31 - __builtin_clz(rw));  // a power of two
             while (rw >= 2 && ((named && d.ngal2 % rw) || xline2_smem(n1s, n2s, rw, esz) > budget)) rw /= 2;
             if (rw >= 2) {
@@ -1481,7 +1473,7 @@ int create_impl(const cfd_config* cfg, const cfd_ib_list* ibu, const cfd_ib_list
         line_split(d.ngal2, n1s, n2s);
         if (n1s) {
             const int zl = g_tuning && (g_tuning->zlines == 4 || g_tuning->zlines == 8 || g_tuning->zlines == 16) ? g_tuning->zlines : 0;
-            const int lb = zl ? ilog2(zl) : env_int("CFD_ZLINES_LOG2", z768 ? (mixed ? 3 : 2) : (mixed ? 4 : 3), 2, 4);
+            const int lb = zl ? ilog2(zl) : env_int("CFD_ZLINES_LOG2", ilog2(dz.zlines), 2, 4);
             c->LZ2 = lb;
             c->NTZ2 = (1 << lb) * std::max(n1s, n2s);
             c->SMZ2 = z_lines_smem(n1s, n2s, 1 << lb, esz);
@@ -1517,6 +1509,11 @@ int create_impl(const cfd_config* cfg, const cfd_ib_list* ibu, const cfd_ib_list
         c->NTZm = (1 << c->LZ2) * std::max(n1s, n2s);
         c->SMZm = z_lines_smem(n1s, n2s, 1 << c->LZ2, esz);
         while (c->RWx > 1 && (cfg->ngal2_mid % c->RWx)) c->RWx /= 2;
+        for (int m = 0; m < 2; ++m) {
+            line_split(m ? cfg->ngal1_mid : d.ngal1, n1s, n2s);
+            if (n1s) c->RWB[m] = 4;
+            while (c->RWB[m] > 1 && xline2_smem(n1s, n2s, c->RWB[m], esz) > budget) c->RWB[m] /= 2;
+        }
     }
     // the x-line pass marching in y (one band).  FP32-mixed: x-line path 6, the default at 384 points
     // (microseconds a launch against the per-slot kernels, 384 x 257: 470 and 637; 128 x 129 62 and 46);
@@ -1549,7 +1546,7 @@ int create_impl(const cfd_config* cfg, const cfd_ib_list* ibu, const cfd_ib_list
                 const int nrb = d.ngal2 / rw, ns = d.nyu - 1;
                 int cs = 4;
                 for (int cand : {16, 12, 8, 6})
-                    if ((long long)nrb * ((ns + cand - 1) / cand) >= 20LL * 148) { cs = cand; break; }
+                    if ((long long)nrb * ((ns + cand - 1) / cand) >= 20LL * c->nsm) { cs = cand; break; }
                 c->XMC = env_int("CFD_XMARCH_STEPS", cs, 2, 1 << 20);
             }
         }
@@ -1569,8 +1566,7 @@ int create_impl(const cfd_config* cfg, const cfd_ib_list* ibu, const cfd_ib_list
     if (c->LZ2 >= 0) {
         int n1s = 0, n2s = 0;
         line_split(d.ngal2, n1s, n2s, true);
-        c->ZALT = n1s && c->RW2 &&
-                  tune_int(&cfd_tuning::zsplit, "CFD_ZSPLIT", z768 || d.ngal2 == 192 ? 2 : 1, 1, 2) == 2;
+        c->ZALT = n1s && c->RW2 && tune_int(&cfd_tuning::zsplit, "CFD_ZSPLIT", dz.zsplit, 1, 2) == 2;
         line_split(d.ngal2, n1s, n2s, c->ZALT);
         c->NTZN = (1 << c->LZ2) * std::max(n1s, n2s);
         c->SMZN = z_lines_smem(n1s, n2s, 1 << c->LZ2, esz);

@@ -56,6 +56,34 @@ struct LineKernels {
 // lengths (only zinv2s, zfwd2, xline2, their variants, ib_zin and ib_zout).
 template <typename T2> const LineKernels<T2>* line_kernels(int n, bool alt = false);
 
+// What a context runs where cfd_tuning does not say: x-line path, radix order and rows by its x length,
+// radix order and lines by its z length.  The transposed split is the default where both x and z lines
+// gain by it, and at 768 points in FP64 for z alone; microseconds a launch, plain | transposed (z inverse,
+// x-line, z forward; n x planes x n):
+//   64 x 97    FP64 3.8 12.4 5.3 | 5.4 23.8 8.0        FP32 3.7 10.0 4.2 | 3.9 16.9 5.9
+//   96 x 129   FP64 11.6 40.1 12.4 | 11.6 35.9 14.4    FP32 6.6 24.3 8.5 | 7.0 25.0 8.8
+//   128 x 129  FP64 17.6 78.4 22.1 | 18.4 78.2 28.2    FP32 14.9 42.0 13.1 | 15.5 52.3 15.2
+//   192 x 193  FP64 45.7 229 77.6 | 41.4 208 74.1      FP32 38.8 136 49.7 | 29.3 116 40.5
+//   384 x 129  FP64 117 574 226 | 128 612 224          FP32 72.1 325 114 | 79.0 340 127
+//   768 x 65   FP64 324 1730 715 | 322 1905 626        FP32 210 810 332 | 163 739 299
+// (the last in 2 and 8 x rows, 4 and 8 z lines; FP32 x lines in 4 rows 818 plain).  The 64-register x-line
+// (path 5) at 192 points: 119 | 109 us; the march (path 6) at 384: 470 us against 637 on 257 planes.
+struct LineDefaults {
+    int xpath = 1, xsplit = 1, xrows = 4, zsplit = 1, zlines = 8;
+};
+inline LineDefaults line_defaults(int n, bool f32) {
+    LineDefaults k;
+    if (f32) k.zlines = 16;
+    if (n == 192) { k.xsplit = k.zsplit = 2; if (f32) k.xpath = 5; }
+    if (n == 384 && f32) k.xpath = 6;
+    if (n == 768) {
+        k.zsplit = 2;
+        k.zlines = f32 ? 8 : 4;
+        if (f32) { k.xsplit = 2; k.xrows = 8; }
+    }
+    return k;
+}
+
 // what each unit holds (null for the lengths it does not)
 template <typename T2> const LineKernels<T2>* line_kernels_named(int n);
 template <typename T2> const LineKernels<T2>* line_kernels_alt(int n);
