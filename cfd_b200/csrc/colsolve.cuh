@@ -23,13 +23,13 @@
 // so that one group's transfers overlap another's elimination.  Where the planes lie far apart
 // (col_cols) a group owns eight columns, so that a row it touches brings 128 bytes.
 //
-// Measured on B200, microseconds per substep against the sweeps (k_solve_uvw + k_solve_p): 316
-// against 839 at 384 x 257(+90) x 384, 71 against 375 at 192 x 193(+90) x 192, 10 against 156 at
-// 64 x 97(+56) x 64, 2040 against 4527 at 768 x 385(+90) x 768.  At the first size that is 0.70
+// Measured on B200, microseconds per substep against the sweeps (k_solve_uvw + k_solve_p): 323
+// against 839 at 384 x 257(+90) x 384, 75 against 375 at 192 x 193(+90) x 192, 10 against 156 at
+// 64 x 97(+56) x 64, 2091 against 4527 at 768 x 385(+90) x 768.  At the first size that is 0.69
 // of the copy bandwidth on the 128 bytes; what is left is the latency of the elimination at the
-// 12 warps an SM holds (FP64 units 22 % busy, shared memory 36 %).  The same partition with
+// 12 warps an SM holds (FP64 units 22 % busy, shared memory 36 %).  An earlier form with
 // the columns brought in by cp.async, one thread a 16-byte row, took 507 (L1 tag lookups of the
-// 64-byte pieces), and 588 before the reduced system stopped at decoupled rows.
+// 64-byte pieces), and 588 before the reduced system's matrix stopped at decoupled rows.
 #pragma once
 
 #include <cuda.h>
@@ -85,6 +85,27 @@ __device__ __forceinline__ double pivot_rcp(double x) {
     asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
     r = fma(r, fma(-x, r, 1.0), r);
     return fma(r, fma(-x, r, 1.0), r);
+}
+
+// Whether couplings al, ga of at most 2^-60 cannot change any lane's f to a double, by the exponents of
+// the largest and the smallest of each component: then f + al f(s-d) + ga f(s+d) is f for every lane.
+// (Lanes without couplings, past the column's end, do not count.)
+template <int NR>
+__device__ __forceinline__ bool carries_nothing(double al, double ga, const double2 (&f)[NR]) {
+    auto ex = [](double a) { return ((unsigned)__double2hiint(a) & 0x7fffffffu) >> 20; };
+    const double c = fmax(fabs(al), fabs(ga));
+    const unsigned ec = __reduce_max_sync(0xffffffffu, ex(c));
+    bool ok = true;
+#pragma unroll
+    for (int k = 0; k < NR; ++k)
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            const double v = i ? f[k].y : f[k].x;
+            const unsigned hi = __reduce_max_sync(0xffffffffu, ex(v));
+            const unsigned lo = __reduce_min_sync(0xffffffffu, c == 0.0 ? 0x7ffu : ex(v));
+            ok = ok && (hi == 0 || (int)(ec + hi) - 1023 + 60 < (int)lo);
+        }
+    return ok;
 }
 
 // One system over the warp's column: y[k][i] holds the NR real-matrix complex right-hand sides of
@@ -143,7 +164,8 @@ __device__ __forceinline__ void warp_tridiag(double2 (&y)[NR][M], Coef coef) {
     // rounded once a step, until the couplings are so small that their products cannot change the
     // diagonals (at once for the Helmholtz rows of a small time step: they fall by about beta/dy^2 a
     // row).  What they still carry from row to row counts where a right-hand side is zero or small:
-    // the steps left take it along, on rows scaled to a diagonal of 1.
+    // the steps left take it along, on rows scaled to a diagonal of 1, unless no lane's f would change
+    // (384 x 257(+90) x 384: 335 us a substep without that test, 323 with it).
     int d = 1;
 #pragma unroll 1
     for (;; d <<= 1) {
@@ -164,6 +186,7 @@ __device__ __forceinline__ void warp_tridiag(double2 (&y)[NR][M], Coef coef) {
         al *= alm;
         ga *= gap;
     }
+    if (d < 32 && carries_nothing<NR>(al, ga, f)) d = 32;
 #pragma unroll 1
     for (; d < 32; d <<= 1) {
 #pragma unroll
