@@ -1418,7 +1418,7 @@ int create_impl(const cfd_config* cfg, const cfd_ib_list* ibu, const cfd_ib_list
     // FP32-mixed contexts interpolate in y in FP32, on transformed planes, only where both lengths are
     // named ones, or where the caller asks for the march.  Everywhere else the FP64 fields are interpolated
     // and rounded once (k_zinv2), and k_xline2b takes the planes (path 1): that costs a z transform per
-    // field and slot instead of one per plane, 144 x 108 x 131 a step of 302 -> 312 us.
+    // field and slot instead of one per plane, 144 x 131 x 108 a step of 302 -> 311 us.
     const bool named2 = line_kernels_named<float2>(d.ngal1) && line_kernels_named<float2>(d.ngal2);
     const bool march_asked = line_march_f32(d.ngal1) && std::getenv("CFD_XMARCH_STEPS");
     const LineDefaults dx = line_defaults(d.ngal1, mixed), dz = line_defaults(d.ngal2, mixed);

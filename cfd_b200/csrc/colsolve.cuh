@@ -24,7 +24,7 @@
 // (col_cols) a group owns eight columns, so that a row it touches brings 128 bytes.
 //
 // Measured on B200, microseconds per substep against the sweeps (k_solve_uvw + k_solve_p): 323
-// against 839 at 384 x 257(+90) x 384, 75 against 375 at 192 x 193(+90) x 192, 10 against 156 at
+// against 839 at 384 x 257(+90) x 384, 76 against 375 at 192 x 193(+90) x 192, 10 against 156 at
 // 64 x 97(+56) x 64, 2091 against 4527 at 768 x 385(+90) x 768.  At the first size that is 0.69
 // of the copy bandwidth on the 128 bytes; what is left is the latency of the elimination at the
 // 12 warps an SM holds (FP64 units 22 % busy, shared memory 36 %).  An earlier form with

@@ -4,10 +4,11 @@
 // 2^a 3^b from 12 to 768.  They are instantiated in lines_*.cu, a few lengths each, so that the
 // units compile side by side.  Against the radix-by-radix kernels that lengths other than the
 // named six (64, 96, 128, 192, 384, 768) ran before, microseconds a launch on B200 (z inverse, x,
-// z forward): 256 x 129 x 256 FP64 232, 602, 249 -> 46, 233, 85, FP32 177, 459, 152 -> 38, 147,
-// 49; 144 x 131 x 108 FP32 70, 146, 55 -> 8, 38, 13; 24 x 17(+6) x 18 FP64 4.1, 6.1, 3.9 -> 2.2,
-// 3.1, 2.3.  The shared-memory passes of those kernels, and a slot's z transform for each field
-// and slot instead of one a plane, were what they spent their time on.
+// z forward): 256 x 129 x 256 FP64 232, 602, 249 -> 46, 225, 86, FP32 177, 459, 152 -> 71, 118,
+// 50; 144 x 131 x 108 FP32 70, 146, 55 -> 16, 33, 13; 24 x 17(+6) x 18 FP64 4.1, 6.1, 3.9 -> 2.2,
+// 3.1, 2.3.  The shared-memory passes of those kernels, and in FP64 a slot's z transform for each
+// field and slot instead of one a plane, were what they spent their time on (FP32 keeps the latter at
+// these lengths, since it interpolates in FP64 before the transforms).
 #pragma once
 
 #include "field_lines.cuh"

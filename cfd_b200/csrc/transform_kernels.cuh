@@ -225,7 +225,7 @@ __global__ void __launch_bounds__(256) k_xline(Dims d, T2* __restrict__ H0, T2* 
 // elements of a subsequence are zero, direct or conjugated is resolved at compile time
 // except in the two blocks that straddle a boundary.
 // DIRECT (three bands; FP32-mixed at lengths that are not among the named six): u, w, v of every slot
-// of the launch lie interpolated in H0, H1, H2 already, and the products take their place (128-point rows of 128 x 97(+56) x 128 FP64: 36 -> 27 us a band
+// of the launch lie interpolated in H0, H1, H2 already, and the products take their place (128-point rows of 128 x 97(+56) x 128 FP64: 36 -> 28 us a band
 // against the radix-by-radix k_xline).
 template <typename T2, int N1, int N2, int TPAD = 1, bool DIRECT = false>
 __device__ __forceinline__ void xline2_body(Dims d, Geo g, const T2* __restrict__ Hx, T2* __restrict__ H0, T2* __restrict__ H1, T2* __restrict__ H2,

@@ -20,8 +20,8 @@
 // warp, lanes 30 and 31 idle) and pass u (A, B -> C) and the face value of w (C -> A, B)
 // with two shuffles, so every lane runs two forward lines, as one packed-pair transform
 // (fft_pair.cuh: each .f32x2 instruction serves both lines); in FP64 one line after the other, and the
-// forward exchange takes the place of the inverse one, so that three 96-thread CTAs at 224 registers
-// share an SM: 1534 -> 1290 us a launch at 384 x 257(+90) x 384 (4.5 instead of 7 complex lines a row and
+// forward exchange takes the place of the inverse one, so that three 96-thread CTAs at 168 registers
+// and 70 KB share an SM: 1534 -> 1261 us a launch at 384 x 257(+90) x 384 (4.5 instead of 7 complex lines a row and
 // plane pair, at 9 instead of 12 warps an SM).  The forward N1-point step holds
 // X[kb + N2 ka] in registers; the unpack of the two real spectra pairs X_k with X_N-k, which
 // lane N2 - kb of the same warp holds (N2 divides 32), so it needs no shared memory.
