@@ -1553,7 +1553,7 @@ int create_impl(const cfd_config* cfg, const cfd_ib_list* ibu, const cfd_ib_list
     }
     if (mixed && !named2 && c->RW2 && !c->XMRW) {
         const auto* k = line_kernels<float2>(d.ngal1);
-        c->RWD = 4;
+        c->RWD = 1 << (31 - __builtin_clz(tune_int(&cfd_tuning::xline_rows, "CFD_XLINE_ROWS", 4, 2, 8)));
         while (c->RWD > 1 && xline2_smem(k->n1, k->n2, c->RWD, esz) > budget) c->RWD /= 2;
         c->RW2 = 0; c->XL3 = false;
     }
